@@ -1,10 +1,9 @@
-// Correctly rounded FP64 division with few FP64 instructions, and the exact
+// Correctly rounded FP64 division without FP64 instructions, and the exact
 // shortcut of the limiters' 1e-30 + x.  GB300 issues FP64 at 1/64 of the FP32
 // rate, so the exact schemes are bound by their FP64 instruction count; a
-// quotient here costs four FP64 instructions (the product with a reciprocal
-// built in FP32, its Markstein correction and one residual for its proof), and
-// a lane whose result cannot be proven correctly rounded takes the division
-// instruction, so every function returns exactly the IEEE result.
+// quotient here is a long division on the integer pipe, and a lane outside its
+// range takes the division instruction, so every function returns exactly the
+// IEEE result.
 #pragma once
 #include <math.h>
 
@@ -28,145 +27,86 @@ DEVI double double_of(long long b) {
   return x;
 }
 
-// FP64 -> FP32 by truncation of the significand, on the integer pipe.  Below
-// the FP32 normal range the result is +-0, above it +-Inf (NaN too); only the
-// reciprocal seed uses it, and a seed from either is rejected downstream.
-DEVI float f32_trunc(double x) {
-  unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  unsigned sign = hi & 0x80000000u, mag = hi & 0x7fffffffu;
-  if (mag < (897u << 20)) return __uint_as_float(sign);
-  if (mag >= (1151u << 20)) return __uint_as_float(sign | 0x7f800000u);
-  return __uint_as_float(sign | ((mag - (896u << 20)) << 3) | (lo >> 29));
-}
-// hi + lo as a double, on the integer pipe, for normal FP32 values with
-// |lo| < 2^-20 |hi|: the significands are aligned on hi's exponent and added as
-// integers (exact when lo's lowest bit is not below hi's 53-bit grid, else lo
-// is truncated to it; one bit may be lost when the sum carries into the next
-// binade).  Other inputs give a finite or NaN value of no use, which the
-// division's proof then rejects.
-DEVI double join_f32(float hi, float lo) {
-  const unsigned bh = __float_as_uint(hi), bl = __float_as_uint(lo);
-  const int eh = (int)((bh >> 23) & 0xffu), el = (int)((bl >> 23) & 0xffu);
-  long long m = (long long)((bh & 0x7fffffu) | 0x800000u) << 29;  // hi's significand, bit 52 set
-  const long long ml = el ? (long long)((bl & 0x7fffffu) | 0x800000u) : 0;
-  const int sh = eh - el - 29;  // lo's significand is ml * 2^-sh units of m's lowest bit
-  long long al = 0;
-  if (sh >= 0 && sh < 40) al = ml >> sh;
-  else if (sh < 0 && sh > -30) al = ml << -sh;
-  m = ((bh ^ bl) & 0x80000000u) ? m - al : m + al;
-  int e = eh + 896;  // FP64 biased exponent of hi
-  if (m >= (1LL << 53)) {
-    m >>= 1;
-    ++e;
-  } else if (m < (1LL << 52)) {
-    m <<= 1;
-    --e;
-  }
-  return double_of(((long long)(bh & 0x80000000u) << 32) | ((long long)e << 52) | (m & 0x000fffffffffffffLL));
-}
-
-// Approximate reciprocal of b with no FP64 instruction.  b is split into FP32
-// terms bh + bl (its truncation to FP32 and the next 24 bits of the remaining
-// significand); y0 = rcp.approx(bh) (at most one FP32 ulp of error); the
-// residual e = 1 - bh*y0 - bl*y0 by two FP32 FMAs (rounding errors near 2^-46);
-// and y = y0 + y0*e joined into a double on the integer pipe, the first-order
-// Newton-Raphson correction carried in FP32.  |y*b - 1| is then about
-// (2^-22)^2 plus the FP32 roundings, below 2^-42, for 2^-103 <= |b| < 2^127
-// (other b give an unusable y, which the division's proof rejects).
-DEVI double recip_seed(double b) {
+// Quotients by long division on the integer pipe.  GB300 issues one FP64 warp
+// instruction per 19.4 SM cycles (measured; the number of active lanes does not
+// matter), an integer one per 0.3 to 0.5 (the 64-bit product and the high half
+// of a product per 1.1), so a division in integers leaves the FP64 pipe to the
+// additions and products: 26 SM cycles per warp and none of them on the FP64
+// pipe, against 76 for the Markstein correction of an FP32 reciprocal with its
+// FP64 proof (4 FP64 instructions) and 140 for the division instruction.  The
+// advection step of 10 tracers on 360x270x50 cells went from 7.34 to 5.42 ms
+// with it, that of 2 tracers on 120x80x30 from 0.143 to 0.102 ms.
+//
+// With significands A, B in [2^52, 2^53) three digits of 18 bits give
+// Q = floor(A 2^54 / B), in (2^53, 2^55).  A digit is the high half of the
+// remainder's top bits times Y, a 24-bit reciprocal of B rounded down, so it is
+// never above the true digit and at most one below it: Y is rcp.approx of B's
+// 24 leading bits (within 2^-23 of the reciprocal on [1, 2), that is two units
+// of 2^-24, and at most two more too large for the bits cut from B) less four
+// units, hence below 2^24 2^52/B by at most 2^-20.4 of it, and a digit is below
+// 2^19.  Every remainder is then in [0, 2B), so arithmetic modulo 2^64 is
+// exact, and the last one says whether one more belongs to Q.  A quotient of two 53-bit significands is never the
+// midpoint of two doubles, so Q's bits below the result's last one round it
+// correctly without a sticky bit.
+//
+// Normal operands with a normal result take this path, and a zero dividend
+// with a normal divisor; any other lane takes the division instruction, so
+// every function returns exactly the IEEE result.
+struct Divisor {
+  unsigned hi, nlo, nhi, y;  // high word of b; -B modulo 2^64; 24-bit reciprocal
+};
+DEVI Divisor divisor_of(double b) {
   const unsigned hi = (unsigned)__double2hiint(b), lo = (unsigned)__double2loint(b);
-  const unsigned sign = hi & 0x80000000u, E = (hi & 0x7fffffffu) >> 20;
-  const float bh = f32_trunc(b);
-  // remaining 29 significand bits: (lo & 0x1fffffff) * 2^-29 * 2^(E - 1046), sign of b
-  const float low = __uint2float_rz(lo & 0x1fffffffu) * 0x1p-29f;
-  const float scale = (E >= 920u && E <= 1150u) ? __uint_as_float((E - 919u) << 23) : 0.0f;
-  const float bl = __uint_as_float(__float_as_uint(low * scale) | sign);
-  float y0;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(bh));
-  float e = fmaf(-bh, y0, 1.0f);
-  e = fmaf(-bl, y0, e);
-  return join_f32(y0, y0 * e);
+  const unsigned m = (hi & 0xfffffu) | 0x100000u;
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffffu) | 0x3f800000u)));
+  unsigned yb = __float_as_uint(y);
+  yb = yb < 0x3f7fffffu ? yb : 0x3f7fffffu;  // rcp(1) = 1 would lose its leading bit
+  const unsigned long long nb = 0ULL - (((unsigned long long)m << 32) | lo);
+  return {hi, (unsigned)nb, (unsigned)(nb >> 32), ((yb & 0x7fffffu) | 0x800000u) - 4u};
 }
-
-// a / b from an approximate reciprocal y of b (Markstein's correction:
-// P. Markstein, IBM J. Res. Dev. 34(1), 1990; J.-M. Muller et al., Handbook of
-// Floating-Point Arithmetic, ch. 5): q = RN(a*y), r = RN(a - b*q) (one FMA),
-// q1 = RN(q + r*y).  For y within 2^-40 of 1/b (relative), q1 is within about
-// 2^-80 of a/b before its rounding.  It is then proven correctly rounded at run time: with
-// r1 = a - b*q1 from one more FMA (exact when q1 is within an ulp of a/b),
-// q1 = RN(a/b) when |r1| < |b|*ulp(q1)/2 and q1 is normal and not a power of
-// two, or when r1 is zero (q1 is the exact quotient).  A lane that cannot prove
-// it (a tie, a binade edge, extreme exponents, an unusable y) takes the
-// division instruction, so the result always equals a / b.
-DEVI double div_recip(double a, double b, double y) {
-  const long long kAbsMask = 0x7fffffffffffffffLL, kMant = 0x000fffffffffffffLL;
-  const long long ba = bits_of(a), bbits = bits_of(b);
-  long long ab = ba & kAbsMask, bb = bbits & kAbsMask;
-  int ea = (int)(ab >> 52), eb = (int)(bb >> 52);
-  double q1;
-  bool ok;
-  if (ab == 0) {  // 0 / b = +-0 for finite non-zero b
-    q1 = double_of((ba ^ bbits) & (long long)0x8000000000000000ULL);
-    ok = eb >= 1 && eb <= 2046;
-  } else {
-    double q = a * y;
-    double r = fma(-q, b, a);
-    q1 = fma(r, y, q);
-    double r1 = fma(-q1, b, a);
-    long long qb = bits_of(q1) & kAbsMask, rb = bits_of(r1) & kAbsMask;
-    int eq = (int)(qb >> 52);
-    int et = eb + eq - 1076;  // exponent of |b| * ulp(q1) / 2
-    ok = ea >= 64 && ea <= 1980 && eb >= 64 && eb <= 1980 && eq >= 64 && eq <= 1980 && et >= 1 && et <= 2046;
-    long long thr = (bb & kMant) | ((long long)et << 52);
-    ok = ok && ((qb & kMant) != 0 ? rb < thr : rb == 0);
-  }
+// The next 18-bit digit of r / B; r becomes the remainder.
+DEVI unsigned div_digit(unsigned long long& r, const Divisor& d) {
+  const unsigned q = __umulhi((unsigned)(r >> 26), d.y);
+  r = (r << 18) + (unsigned long long)q * d.nlo;
+  r += (unsigned long long)(q * d.nhi) << 32;
+  return q;
+}
+DEVI double div_by(double a, double b, const Divisor& d) {
+  const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
+  const unsigned ea = ah & 0x7ff00000u, eb = d.hi & 0x7ff00000u, sign = (ah ^ d.hi) & 0x80000000u;
+  unsigned long long r = ((unsigned long long)((ah & 0xfffffu) | 0x100000u) << 32) | al;
+  const unsigned q1 = div_digit(r, d), q2 = div_digit(r, d), q3 = div_digit(r, d);
+  unsigned long long q = (unsigned long long)q2 * (1u << 18) + q3 + ((unsigned long long)(q1 << 4) << 32);
+  // r + (-B) carries out of 64 bits where r >= B
+  q += r + (((unsigned long long)d.nhi << 32) | d.nlo) < r ? 1 : 0;
+  const unsigned sh = (unsigned)(q >> 32) >= (1u << 22) ? 2u : 1u;  // bits below the result's last
+  q = (q + sh) >> sh;                                               // half of the last place is sh
+  const unsigned rh = (unsigned)(q >> 32) + (ea - eb + ((1020u + sh) << 20));  // q's leading bit adds one to the field
+  const bool bn = eb - 0x100000u < 0x7fe00000u;
+  bool ok = bn && ea - 0x100000u < 0x7fe00000u && rh - 0x100000u < 0x7fe00000u;
+  unsigned lo = (unsigned)q, hi = rh | sign;
+  if (((ah & 0x7fffffffu) | al) == 0) lo = 0, hi = sign, ok = bn;  // 0 / b
+  double x = __hiloint2double((int)hi, (int)lo);
   if (!__all_sync(__activemask(), ok)) {
-    if (!ok) q1 = a / b;
+    if (!ok) x = a / b;
   }
-  return q1;
+  return x;
 }
 
 // a / b for a divisor used once.
-DEVI double div_seeded(double a, double b) { return div_recip(a, b, recip_seed(b)); }
+DEVI double div_seeded(double a, double b) { return div_by(a, b, divisor_of(b)); }
 
-// Two-term reciprocal yh + yl of b for a divisor shared by many quotients:
-// yh = recip_seed(b) and yl = yh*(1 - b*yh) (two FP64 instructions), so that
-// yh + yl is within about 2^-84 of 1/b (relative; the square of yh's error)
-// where recip_seed is usable, else unusable.
+// A divisor shared by many quotients, kept in two doubles' bits: yh holds its
+// reciprocal, yl the negated significand.
 DEVI void recip_pair(double b, double& yh, double& yl) {
-  yh = recip_seed(b);
-  yl = yh * fma(-b, yh, 1.0);
+  const Divisor d = divisor_of(b);
+  yh = __hiloint2double((int)d.hi, (int)d.y);
+  yl = __hiloint2double((int)d.nhi, (int)d.nlo);
 }
-
-// a / b from a two-term reciprocal (recip_pair): q1 = RN(a*yh + RN(a*yl))
-// (N. Brisebarre, J.-M. Muller, S. K. Raina, IEEE Trans. Computers 53(8),
-// 2004) is within about 2^-84 of a/b before its rounding; it is proven
-// correctly rounded as in div_recip, else the lane takes the division
-// instruction.  Three FP64 instructions.
 DEVI double div_pair(double a, double b, double yh, double yl) {
-  const long long kAbsMask = 0x7fffffffffffffffLL, kMant = 0x000fffffffffffffLL;
-  const long long ba = bits_of(a), bbits = bits_of(b);
-  long long ab = ba & kAbsMask, bb = bbits & kAbsMask;
-  int ea = (int)(ab >> 52), eb = (int)(bb >> 52);
-  double q1;
-  bool ok;
-  if (ab == 0) {
-    q1 = double_of((ba ^ bbits) & (long long)0x8000000000000000ULL);
-    ok = eb >= 1 && eb <= 2046;
-  } else {
-    q1 = fma(a, yh, a * yl);
-    double r1 = fma(-q1, b, a);
-    long long qb = bits_of(q1) & kAbsMask, rb = bits_of(r1) & kAbsMask;
-    int eq = (int)(qb >> 52);
-    int et = eb + eq - 1076;
-    ok = ea >= 64 && ea <= 1980 && eb >= 64 && eb <= 1980 && eq >= 64 && eq <= 1980 && et >= 1 && et <= 2046;
-    long long thr = (bb & kMant) | ((long long)et << 52);
-    ok = ok && ((qb & kMant) != 0 ? rb < thr : rb == 0);
-  }
-  if (!__all_sync(__activemask(), ok)) {
-    if (!ok) q1 = a / b;
-  }
-  return q1;
+  return div_by(a, b, {(unsigned)__double2hiint(yh), (unsigned)__double2loint(yl), (unsigned)__double2hiint(yl),
+                       (unsigned)__double2loint(yh)});
 }
 
 // RN(1e-30 + x) without an FP64 addition where that is exact by inspection:
