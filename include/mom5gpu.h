@@ -325,22 +325,17 @@ int mom5gpu_update_tracer(mom5gpu_domain* d, int n, int taum1, int taup1, double
  * halo update. */
 int mom5gpu_tracer_advection_step(mom5gpu_domain* d, int taum1, int tau, int taup1, double dtime);
 /* Time the candidate launch shapes of mom5gpu_tracer_advection_step on this
- * domain (precision form: tile height 16, 24, 32 or 64 rows, plain, with a
- * cp.async tracer prefetch, or TMA-staged; FP64: y-pass rows per thread 2..16)
+ * domain (precision form: tile height; FP64: y-pass rows per thread 2..16)
  * and keep the fastest.  The trials step taum1 = tau = 1 to
  * taup1 = 2: time level 2 of the tracers and th_tendency are overwritten.
  * A summary is written to report (may be NULL). */
 int mom5gpu_autotune(mom5gpu_domain* d, double dtime, char* report, size_t report_len);
 /* The launch shape autotune chose, or one to pin: precision-form tile height
- * (16, 24, 32 or 64 rows incl. halo); staging of the tile's operands: prefetch
- * 0 = plain loads, 1 = tracer levels prefetched by cp.async (height 16 only),
- * 2 = tiles staged by TMA with the tracer levels carried down the column in
- * registers (heights 16 and 24; domains of even ni, else the plain kernel),
- * 3 = the same with at most 5 tracers per block and two blocks per SM
- * (height 16);
- * FP64 y-pass rows per thread (0 = built-in choice, 2, 4, 8, 16).  Every shape
- * gives the same results bit for bit.  A TMA-staged launch whose bounded wait
- * gave up is reported by the next mom5gpu_synchronize as MOM5GPU_ETIMEDOUT. */
+ * (16 or 24 rows incl. halo; 32 or 64: 16 rows up to 4 tracers, else 20);
+ * prefetch 0, 1, 2 or 3, kept and reported (with 1 and 3 the height is 16,
+ * with 2 it is 16 or 24), the tiles are staged alike with all; FP64 y-pass rows
+ * per thread (0 = built-in choice, 2, 4, 8, 16).  Every shape gives the same
+ * results bit for bit. */
 int mom5gpu_set_tuning(mom5gpu_domain* d, int rows, int prefetch, int tj);
 /* Form of the exact B-grid barotropic subcycles (update_ocean_barotropic,
  * ocean_barotropic.F90:3344-3575): 0 (default) = momentum, and corrector with
@@ -481,20 +476,16 @@ int mom5gpu_batch_set_stream(mom5gpu_batch* b, void* stream);
  * every domain is stepped with parity[0], from a CUDA graph captured on the
  * first such call for that parity and replayed afterwards. */
 int mom5gpu_batch_step(mom5gpu_batch* b, const int* index, const int* parity, int count, double dtime);
-/* Time the candidate launch shapes (precision-form tile height and resident
- * blocks per SM; FP64 y-pass rows per thread) on the whole batch and keep the
+/* Time the candidate launch shapes (precision-form tile height; FP64 y-pass
+ * rows per thread) on the whole batch and keep the
  * fastest.  Each trial is a parity-0 step: time level 1 is read, level 2 is
  * overwritten.  A summary is written to report (may be NULL). */
 int mom5gpu_batch_autotune(mom5gpu_batch* b, double dtime, char* report, size_t report_len);
 /* Read or set the launch shape directly (e.g. to reuse one autotune result on
- * several batches): rows = precision-form tile height (16 or 32; 24 = the
- * TMA-staged tiles, 24 rows or 32 for at most 4 tracers, one block per SM, for
- * every domain with an even ni, and the plain 32-row tiles for the others), tj
- * = FP64 y-pass rows per thread (0 = automatic, else 2, 4, 8 or 16),
- * blocks_per_sm = resident blocks per SM of the persistent launch of the plain
- * tiles (1..4).  A TMA-staged tile whose bounded
- * wait gave up is reported by the next mom5gpu_synchronize of its domain as
- * MOM5GPU_ETIMEDOUT. */
+ * several batches): rows = precision-form tile height (16 or 24; 32: 16 rows up
+ * to 4 tracers, else 20), tj = FP64 y-pass rows per thread (0 = automatic, else
+ * 2, 4, 8 or 16), blocks_per_sm = most resident blocks per SM of the precision
+ * form's persistent launch (1..4). */
 int mom5gpu_batch_get_tuning(const mom5gpu_batch* b, int* rows, int* tj, int* blocks_per_sm);
 int mom5gpu_batch_set_tuning(mom5gpu_batch* b, int rows, int tj, int blocks_per_sm);
 /* Device milliseconds of the last batch step (CUDA events on the batch stream). */

@@ -356,9 +356,7 @@ int mom5gpu_synchronize(mom5gpu_domain* d) {
     if (e != cudaSuccess) return cuda_fail(d, e, "synchronize");
     if (v) {
       cudaMemset(d->wait_err, 0, sizeof(int));
-      if (v & 2)
-        return fail(d, MOM5GPU_ETIMEDOUT, "barotropic subcycles: a grid barrier wait gave up; the step's results are void");
-      return fail(d, MOM5GPU_ETIMEDOUT, "precision form: a tile's staged copy did not arrive; its results are void");
+      return fail(d, MOM5GPU_ETIMEDOUT, "barotropic subcycles: a grid barrier wait gave up; the step's results are void");
     }
   }
   return MOM5GPU_OK;
@@ -925,9 +923,7 @@ int mom5gpu_set_tuning(mom5gpu_domain* d, int rows, int prefetch, int tj) {
       (prefetch == 1 && rows != 16) || (prefetch == 2 && rows != 16 && rows != 24) || (prefetch == 3 && rows != 16) ||
       !(tj == 0 || tj == 2 || tj == 4 || tj == 8 || tj == 16))
     return fail(d, MOM5GPU_EINVAL,
-                "set_tuning: rows 16|24|32|64, prefetch 0, 1 (cp.async, rows 16), 2 (TMA, rows 16|24) or 3 "
-                "(TMA, 5 tracers per block, rows 16), "
-                "tj 0|2|4|8|16");
+                "set_tuning: rows 16|24|32|64, prefetch 0, 1 or 3 (rows 16) or 2 (rows 16|24), tj 0|2|4|8|16");
   d->tune_mixed_rows = rows;
   d->tune_mixed_pf = prefetch;
   d->tune_y_tj = tj;
@@ -946,11 +942,10 @@ int mom5gpu_autotune(mom5gpu_domain* d, double dtime, char* report, size_t repor
   if (!d) return MOM5GPU_EINVAL;
   if (!d->advect_ready) return fail(d, MOM5GPU_ESTATE, "autotune before mom5gpu_tracer_advect_init");
   bool mixed = d->opt.precision == MOM5GPU_PRECISION_MIXED;
-  // candidate launch shapes: precision-form tile height (and tracer prefetch); FP64 y-pass rows per thread
-  const int kRows[] = {32, 64, 24, 16, 16, 16, 24, 16};
-  const int kPf[] = {0, 0, 0, 0, 1, 2, 2, 3};
+  // candidate launch shapes: precision-form tile height (32: by the tracer count); FP64 y-pass rows per thread
+  const int kRows[] = {32, 16, 24};
   const int kTj[] = {2, 4, 8, 16};
-  int ncand = mixed ? (d->geo.ni % 2 == 0 ? 8 : 5) : 4;
+  int ncand = mixed ? 3 : 4;
   cudaEvent_t t0, t1;
   if (cudaEventCreate(&t0) != cudaSuccess) return fail(d, MOM5GPU_ECUDA, "autotune events");
   if (cudaEventCreate(&t1) != cudaSuccess) {
@@ -963,7 +958,7 @@ int mom5gpu_autotune(mom5gpu_domain* d, double dtime, char* report, size_t repor
   for (int c = 0; c < ncand && rc == MOM5GPU_OK; ++c) {
     if (mixed) {
       d->tune_mixed_rows = kRows[c];
-      d->tune_mixed_pf = kPf[c];
+      d->tune_mixed_pf = 0;
     } else {
       d->tune_y_tj = kTj[c];
     }
@@ -982,8 +977,7 @@ int mom5gpu_autotune(mom5gpu_domain* d, double dtime, char* report, size_t repor
     ms /= 3.f;
     char line[96];
     if (mixed)
-      snprintf(line, sizeof(line), "rows=%d%s: %.3f ms; ", kRows[c], kPf[c] == 3 ? "+tma5" : kPf[c] == 2 ? "+tma" : kPf[c] ? "+prefetch" : "",
-               ms);
+      snprintf(line, sizeof(line), "rows=%d: %.3f ms; ", kRows[c], ms);
     else snprintf(line, sizeof(line), "tj=%d: %.3f ms; ", kTj[c], ms);
     rep += line;
     if (ms < best) {
@@ -995,15 +989,13 @@ int mom5gpu_autotune(mom5gpu_domain* d, double dtime, char* report, size_t repor
   cudaEventDestroy(t1);
   if (mixed) {
     d->tune_mixed_rows = kRows[bestc];
-    d->tune_mixed_pf = kPf[bestc];
   } else {
     d->tune_y_tj = kTj[bestc];
   }
   if (rc) return rc;
   char line[64];
   if (mixed)
-    snprintf(line, sizeof(line), "chosen rows=%d%s", kRows[bestc],
-             kPf[bestc] == 3 ? "+tma5" : kPf[bestc] == 2 ? "+tma" : kPf[bestc] ? "+prefetch" : "");
+    snprintf(line, sizeof(line), "chosen rows=%d", kRows[bestc]);
   else snprintf(line, sizeof(line), "chosen tj=%d", kTj[bestc]);
   rep += line;
   if (report && report_len) {

@@ -106,9 +106,9 @@ struct mom5gpu_domain {
   long clock_calls[8] = {0};
   long launches = 0;
   // autotuned launch shapes (0 = built-in heuristic)
-  int tune_mixed_rows = 32;  // precision-form tile height incl. halo: 16, 24, 32 or 64
-  int tune_mixed_pf = 0;     // precision form: 1 tracer levels prefetched by cp.async (height 16), 2 TMA-staged tiles
-  int* wait_err = nullptr;   // set when a bounded device wait gave up: bit 0 a TMA-staged copy, bit 1 a grid barrier
+  int tune_mixed_rows = 32;  // precision-form tile height incl. halo: 16 or 24, else by the number of tracers
+  int tune_mixed_pf = 0;     // precision form: accepted and reported, every value runs the one staging there is
+  int* wait_err = nullptr;   // set when a bounded device wait gave up: bit 1 a grid barrier
   unsigned* bt_sync = nullptr;  // arrival counter of the cooperative barotropic subcycle's grid barriers
   int tune_y_tj = 0;         // FP64 y-pass rows per thread
   int bt_fused = 0;          // exact B-grid subcycles: 0 three launches each, 1 one launch each,
@@ -312,16 +312,17 @@ int ensure_mdfl_scratch(mom5gpu_domain* d, int ntr);
 // e; p*[e] is the first block of entry e in each pass (p*[count] = total).
 struct BatchWork {
   const int* entries;
-  const int *pz, *px, *py, *pu, *pb2, *pb1, *pm, *pt;
+  const int *pz, *px, *py, *pu, *pb2, *pb1, *pm;
   int count;
-  int tz, tx, ty, tu, tb2, tb1, tm, tt;  // total blocks of each pass
+  int tz, tx, ty, tu, tb2, tb1, tm;  // total blocks of each pass
+  int seg;                           // levels per item of the precision form
 };
-// blocks of one domain in each pass, for the work-list prefix sums; t: the
-// TMA-staged precision tiles (mixed_rows 24 on a domain that allows them)
+// blocks of one domain in each pass, for the work-list prefix sums; m: the
+// precision form's items, tiles of tile_rows rows by segments of seg levels
 struct BatchBlocks {
-  int z, x, y, u, b2, b1, m, t;
+  int z, x, y, u, b2, b1, m;
 };
-BatchBlocks batch_blocks(const Geo& g, int TJ, int mixed_rows, bool tma, int ntr);
+BatchBlocks batch_blocks(const Geo& g, int TJ, int tile_rows, int seg);
 // FP64: z/x/y MDFL passes and the explicit update for every entry
 void launch_batch_fp64_advection(const MdflArgs* mdfl, const UpdArgs* upd, const BatchWork& w, int ntr, bool sweby,
                                  int TJ, cudaStream_t s);
@@ -330,32 +331,27 @@ void launch_batch_fp64_advection(const MdflArgs* mdfl, const UpdArgs* upd, const
 void launch_batch_barotropic_loop(const BtArgs* bt, const BtExtra* x, const BatchWork& w, int nts, int stepB, bool fast,
                                   cudaStream_t s);
 // precision form: folded subcycle over the work list (k_batch.cu)
-// precision form, TMA-staged 24-row tiles over a batch's work list (k_mixed_tma.cu):
-// the bytes of one (domain, parity) entry of the device table, filling an entry
-// (MOM5GPU_EUNSUPPORTED when the domain cannot be described to TMA), the launch
-size_t batch_tma_bytes();
-int batch_tma_rows(int ntr);
-int fill_batch_tma(mom5gpu_domain* d, const MixArgs& a, void* host_entry);
-int launch_batch_mixed_tma(const MixArgs* mix, const void* tma, const BatchWork& w, int ntr, int blocks, int* counter,
-                           cudaStream_t s);
 void launch_batch_btf_prep(const BtArgs* bt, const BatchWork& w, cudaStream_t s);
 int launch_batch_btf_subcycle(const BtArgs* bt, const BatchWork& w, int itime, int nts, cudaStream_t s);
 void launch_batch_barotropic_post(const BtArgs* bt, const BtExtra* x, const BatchWork& w, int nts, int stepB, int phase,
                                   cudaStream_t s);
-// precision form: persistent kernel over (entry, tile) items
-// rows 16 or 32: the plain persistent tile kernel; rows 24: the TMA-staged tiles
-// (table tma, counter[1]) and the plain 32-row tiles for the other domains
-int launch_batch_mixed(const MixArgs* mix, const void* tma, const BatchWork& w, int ntr, int rows, int blocks,
-                       int sms, int* counter, cudaStream_t s);
-// sets the shared-memory attribute of every instantiation (before any graph capture)
+
+// ---- precision-form advection (k_mixed_stream.cu) ----
+// tile height of a tuning value (16, 24, or by the tracer count), a domain's tiles
+// of that height, and the levels per segment for a launch of so many tiles
+int stream_tile_rows(int tuned, int ntr);
+long stream_tiles(const Geo& g, int rows);
+int stream_levels(long tiles, int nk, int ntr, int rows);
+// the tracers of a (at most 10) of one domain, outputs numbered from n0
+int launch_mixed_stream(mom5gpu_domain* d, const MixArgs& a, int n0);
+// persistent kernel over a batch's items; the attributes are set before any graph capture
+int launch_batch_mixed(const MixArgs* mix, const BatchWork& w, int ntr, int tuned_rows, int blocks_per_sm, int sms,
+                       int* counter, cudaStream_t s);
 int prepare_batch_mixed();
-int prepare_batch_mixed_tma();
 
 // ---- precision form (k_mixed.cu) ----
 int launch_mdfl_mixed(mom5gpu_domain* d, int n_first, int ntr, int taum1, int tau, int taup1, double dtime,
                       bool fused_update);
-// TMA-staged variant of one launch (k_mixed_tma.cu); MOM5GPU_EUNSUPPORTED: use the plain kernel
 int ensure_wait_words(mom5gpu_domain* d);
-int launch_mixed_tma(mom5gpu_domain* d, const MixArgs& a, int n0, const double* Tall, int zt0, int ntr_all);
 
 }  // namespace mom5

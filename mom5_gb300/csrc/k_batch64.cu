@@ -134,7 +134,7 @@ void adv(const MdflArgs* m, const UpdArgs* u, const BatchWork& w, int TJ, cudaSt
 
 }  // namespace
 
-BatchBlocks batch_blocks(const Geo& g, int TJ, int mixed_rows, bool tma, int ntr) {
+BatchBlocks batch_blocks(const Geo& g, int TJ, int tile_rows, int seg) {
   BatchBlocks b;
   int nb = (g.ni + 127) / 128;
   b.z = nb * g.nj;
@@ -143,12 +143,7 @@ BatchBlocks batch_blocks(const Geo& g, int TJ, int mixed_rows, bool tma, int ntr
   b.u = nb * g.nj * g.nk;
   b.b2 = ((g.ni + 2 + 127) / 128) * (g.nj + 2);
   b.b1 = (int)((g.n2 + 255) / 256);
-  // rows 24: TMA-staged 24-row tiles where the domain allows them, else the plain 32-row tiles
-  const bool staged = mixed_rows == 24 && tma;
-  int tj = (mixed_rows == 24 ? 32 : mixed_rows) - 4;
-  b.m = staged ? 0 : ((g.ni + 27) / 28) * ((g.nj + tj - 1) / tj);
-  const int ttj = staged ? batch_tma_rows(ntr) - 4 : 1;
-  b.t = staged ? ((g.ni + 27) / 28) * ((g.nj + ttj - 1) / ttj) : 0;
+  b.m = (int)stream_tiles(g, tile_rows) * ((g.nk + seg - 1) / seg);
   return b;
 }
 

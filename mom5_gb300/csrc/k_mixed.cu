@@ -1,78 +1,9 @@
-// Precision form of MDFL Sweby: fluxes and limiters in FP32, tracer state in FP64.
-//
-// One fused kernel does the z, x and y passes of advect_tracer_mdfl_sweby
-// (ocean_tracer_advect.F90:3806-4066) for a tile of 28 columns by ZR-4 rows
-// (ZR = 16, 24 or 32, autotuned), marching down k, with the tile's 2-cell halo
-// recomputed instead of exchanged: the z pass runs on the 32 x ZR
-// tile-plus-halo, the x pass on ZR rows x 28 columns, the y pass on the
-// interior.  Face terms (mass flux, Courant number,
-// d0, d1, the limiter slope) are computed once per level and shared by every
-// tracer of the launch.
-//
-// The increment T_mdfl - T is carried as the sum of the three flux-divergence
-// increments; the divergence corrections the reference adds per pass and
-// removes at the end cancel exactly and are applied only to the intermediate
-// values the next pass limits on.  The state update
-// T(taup1) = (rho_dzt(taum1)*T + dtime*th)*rho_dztr (ocean_tracer.F90:2341-2350)
-// is evaluated as T + [(rho_dzt(taum1)*rho_dztr - 1)*T + rho_dzt(tau)*rho_dztr*dT]
-// with one FP64 add per tracer-cell.  FP64<->FP32 conversions are done with
-// integer operations: on GB300 a conversion issues at the FP64 rate.
-#include <math.h>
-
-
-#include "mixed_body.cuh"
+// Precision form: the barotropic subcycle kernels, and the arguments and launches
+// of the advection (mixed_stream.cuh, k_mixed_stream.cu).
+#include "internal.h"
 #include "bt_fast_body.cuh"
 
 namespace mom5 {
-
-using namespace mixed;
-
-namespace {
-
-// shared memory: the tile arrays, then (prefetch variant) the tracer buffers
-template <int ZR, bool PF>
-constexpr size_t mixed_smem() {
-  return ((sizeof(SmemT<ZR>) + 15) & ~(size_t)15) + (PF ? sizeof(PrefetchT<ZR>) : 0);
-}
-
-template <int NC, int ZR, bool PF>
-__global__ void __launch_bounds__(tile_threads(ZR), PF ? 2 : (ZR == 16 ? 4 : ZR == 24 ? 3 : ZR == 64 ? 1 : 2))
-    k_mdfl_mixed(MixArgs a, int n0) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  SmemT<ZR>& s = *reinterpret_cast<SmemT<ZR>*>(smem_raw);
-  PrefetchT<ZR>* pf =
-      PF ? reinterpret_cast<PrefetchT<ZR>*>(smem_raw + ((sizeof(SmemT<ZR>) + 15) & ~(size_t)15)) : nullptr;
-  mixed_tile<NC, ZR, PF, tile_threads(ZR)>(a, n0, blockIdx.x, blockIdx.y, s, pf);
-}
-
-template <int NC, int ZR, bool PF>
-int run_mixed_zr(mom5gpu_domain* d, MixArgs a, int n0) {
-  const Geo& g = d->geo;
-  constexpr size_t smem = mixed_smem<ZR, PF>();
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_mdfl_mixed<NC, ZR, PF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_fail(d, e, "mixed kernel attribute");
-    configured = true;
-  }
-  constexpr int TJ = ZR - 4;
-  dim3 grid((g.ni + TI - 1) / TI, (g.nj + TJ - 1) / TJ);
-  k_mdfl_mixed<NC, ZR, PF><<<grid, tile_threads(ZR), smem, d->stream>>>(a, n0);
-  count_launches(d, 1);
-  return MOM5GPU_OK;
-}
-
-template <int NC>
-int run_mixed(mom5gpu_domain* d, MixArgs a, int n0) {
-  if (d->tune_mixed_rows == 16 && d->tune_mixed_pf == 1) return run_mixed_zr<NC, 16, true>(d, a, n0);
-  if (d->tune_mixed_rows == 16) return run_mixed_zr<NC, 16, false>(d, a, n0);
-  if (d->tune_mixed_rows == 24) return run_mixed_zr<NC, 24, false>(d, a, n0);
-  if (d->tune_mixed_rows == 64) return run_mixed_zr<NC, 64, false>(d, a, n0);
-  return run_mixed_zr<NC, 32, false>(d, a, n0);
-}
-
-}  // namespace
 
 __global__ void __launch_bounds__(128) k_btf_prep(BtArgs a) { btfast::prep_body(a, blockIdx.x, blockIdx.y); }
 // The subcycle kernels are launched as programmatic dependents (launch_pdl).
@@ -199,16 +130,7 @@ int launch_mdfl_mixed(mom5gpu_domain* d, int n_first, int ntr, int taum1, int ta
       a.out = fptr(d, MOM5GPU_TH_TENDENCY, n_first + c0, 0);
     }
     if (!a.T || !a.out) return fail(d, MOM5GPU_ENOMEM, "precision form: tracer storage");
-    int n0 = fused_update ? n_first - 1 + c0 : 0;
-    if (d->tune_mixed_pf >= 2) {
-      rc = launch_mixed_tma(d, a, n0, fptr(d, MOM5GPU_TRACER, 1, taum1), n_first - 1 + c0,
-                            d->dims.num_prog_tracers);
-      if (rc != MOM5GPU_EUNSUPPORTED) continue;
-    }
-    if (cn <= 1) rc = run_mixed<1>(d, a, n0);
-    else if (cn <= 2) rc = run_mixed<2>(d, a, n0);
-    else if (cn <= 4) rc = run_mixed<4>(d, a, n0);
-    else rc = run_mixed<10>(d, a, n0);
+    rc = launch_mixed_stream(d, a, fused_update ? n_first - 1 + c0 : 0);
   }
   if (rc) return rc;
   cudaError_t e = cudaGetLastError();

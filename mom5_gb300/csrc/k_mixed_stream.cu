@@ -1,0 +1,163 @@
+// Precision form of MDFL Sweby: the kernels over the streaming tile
+// (mixed_stream.cuh), one domain per launch or a batch's work list, and the rules
+// for their launch shapes.
+#include "mixed_stream.cuh"
+
+namespace mom5 {
+
+using namespace mixed;
+
+namespace {
+
+// Rows of a tile (with its halo) and blocks per SM for NP tracer pairs.  Up to two
+// pairs, two blocks of 16 rows (64 registers) overlap each other's barriers:
+// 720x540x50 cells, 4 tracers, 895 us against 978 to 1033 with 12, 20, 24 or 32 rows; 2
+// tracers 674 against 734 to 871.  Three pairs and more do not fit twice; one block
+// of 20 rows (96 registers) is the largest without spills: 1440x1080x50, 10
+// tracers, 7.10 ms against 7.54 with 16 rows and 8.43 with 24.
+constexpr int stream_rows(int np) { return np <= 2 ? 16 : 20; }
+constexpr int stream_blocks(int np, int rows) { return np <= 2 && rows == 16 ? 2 : 1; }
+
+template <int NP, int ZR>
+__global__ void __launch_bounds__(32 * ZR, stream_blocks(NP, ZR)) k_mdfl_stream(MixArgs a, int n0, int L) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int k0 = blockIdx.z * L, k1 = k0 + L < a.g.nk ? k0 + L : a.g.nk;
+  stream_tile<NP, ZR>(a, n0, blockIdx.x, blockIdx.y, k0, k1, *reinterpret_cast<StreamSmem<NP, ZR>*>(smem_raw));
+}
+
+DEVI int find_entry_m(const int* prefix, int count, int b) {
+  int lo = 0, hi = count;
+  while (hi - lo > 1) {
+    int mid = (lo + hi) >> 1;
+    if (prefix[mid] <= b) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// Persistent: the resident blocks take (domain, tile, level segment) items from an
+// atomic counter, largest domains first.
+template <int NP, int ZR>
+__global__ void __launch_bounds__(32 * ZR, stream_blocks(NP, ZR))
+    kb_mdfl_stream(const MixArgs* __restrict__ d, BatchWork w, int* counter) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int item;
+  for (;;) {
+    if (threadIdx.x == 0) item = atomicAdd(counter, 1);
+    __syncthreads();
+    const int it = item;
+    __syncthreads();
+    if (it >= w.tm) return;
+    const int e = find_entry_m(w.pm, w.count, it);
+    const MixArgs& a = d[w.entries[e]];
+    const int local = it - w.pm[e];
+    const int ntx = (a.g.ni + TI - 1) / TI, nty = (a.g.nj + ZR - 5) / (ZR - 4);
+    const int k0 = local / (ntx * nty) * w.seg, k1 = k0 + w.seg < a.g.nk ? k0 + w.seg : a.g.nk;
+    stream_tile<NP, ZR>(a, 0, local % ntx, local / ntx % nty, k0, k1,
+                        *reinterpret_cast<StreamSmem<NP, ZR>*>(smem_raw));
+  }
+}
+
+long tiles_of(const Geo& g, int rows) { return (long)((g.ni + TI - 1) / TI) * ((g.nj + rows - 5) / (rows - 4)); }
+
+template <int NP, int ZR>
+int run(mom5gpu_domain* d, const MixArgs& a, int n0) {
+  const Geo& g = d->geo;
+  constexpr size_t smem = sizeof(StreamSmem<NP, ZR>);
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(k_mdfl_stream<NP, ZR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(d, e, "mixed kernel attribute");
+    configured = true;
+  }
+  const int L = stream_levels(tiles_of(g, ZR), g.nk, a.ntr, ZR);
+  dim3 grid((g.ni + TI - 1) / TI, (g.nj + ZR - 5) / (ZR - 4), (g.nk + L - 1) / L);
+  k_mdfl_stream<NP, ZR><<<grid, 32 * ZR, smem, d->stream>>>(a, n0, L);
+  count_launches(d, 1);
+  return MOM5GPU_OK;
+}
+
+template <int NP, int ZR>
+int run_batch(const MixArgs* m, const BatchWork& w, int bps, int sms, int* counter, cudaStream_t s) {
+  const int blocks = bps < stream_blocks(NP, ZR) ? bps : stream_blocks(NP, ZR);
+  cudaMemsetAsync(counter, 0, sizeof(int), s);
+  kb_mdfl_stream<NP, ZR><<<blocks * sms, 32 * ZR, sizeof(StreamSmem<NP, ZR>), s>>>(m, w, counter);
+  return MOM5GPU_OK;
+}
+
+template <int NP, int ZR>
+int configure_batch() {
+  return cudaFuncSetAttribute(kb_mdfl_stream<NP, ZR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(StreamSmem<NP, ZR>)) == cudaSuccess
+             ? 0
+             : 1;
+}
+
+template <int NP>
+int configure_batch_rows() {
+  return configure_batch<NP, 16>() | configure_batch<NP, stream_rows(NP)>() | configure_batch<NP, 24>();
+}
+
+// f<NP, ZR>() for ntr tracers (1..10) and a tile height of stream_tile_rows
+#define STREAM_DISPATCH_ROWS(NP, F, ...)                                    \
+  (rows == 24 ? F<NP, 24>(__VA_ARGS__) : rows == 16 ? F<NP, 16>(__VA_ARGS__) : F<NP, stream_rows(NP)>(__VA_ARGS__))
+#define STREAM_DISPATCH(F, ...)                                             \
+  (ntr <= 2   ? STREAM_DISPATCH_ROWS(1, F, __VA_ARGS__)                     \
+   : ntr <= 4 ? STREAM_DISPATCH_ROWS(2, F, __VA_ARGS__)                     \
+   : ntr <= 6 ? STREAM_DISPATCH_ROWS(3, F, __VA_ARGS__)                     \
+   : ntr <= 8 ? STREAM_DISPATCH_ROWS(4, F, __VA_ARGS__)                     \
+              : STREAM_DISPATCH_ROWS(5, F, __VA_ARGS__))
+
+}  // namespace
+
+int stream_tile_rows(int tuned, int ntr) {
+  return tuned == 16 || tuned == 24 ? tuned : stream_rows((ntr + 1) / 2);
+}
+
+long stream_tiles(const Geo& g, int rows) { return tiles_of(g, rows); }
+
+// Levels per segment of a launch of `tiles` tiles.  A domain with few tiles gives
+// the level march few blocks, each a long latency-bound chain; cutting it into
+// segments multiplies the blocks for about two levels more per segment (its
+// prologue and the z pass of the level above).  Of all cuts the cheapest by this
+// model, in level times of a block alone on its SM: each SM works through its
+// share of the blocks one after another, two that share the SM taking 1.55 of one
+// (measured).  255x181x40, 4 tracers: 131 us with segments of 14 levels against 174
+// for whole columns; 300x200x35: 120 (9 levels) against 173; 37x29x12, 2 tracers:
+// 12 (2 levels) against 34.
+int stream_levels(long tiles, int nk, int ntr, int rows) {
+  const bool two = stream_blocks((ntr + 1) / 2, rows) == 2;
+  int best = nk;
+  double cost = 0.0;
+  for (int want = 1; want == 1 || want <= nk / 2; ++want) {
+    const int L = (nk + want - 1) / want, n = (nk + L - 1) / L;
+    const long b = (tiles * n + 151) / 152;
+    const double c = (two ? 1.55 * (b / 2) + b % 2 : (double)b) * (L + (n > 1 ? 2.0 : 1.0));
+    if (want == 1 || c < cost) {
+      cost = c;
+      best = L;
+    }
+  }
+  return best;
+}
+
+int launch_mixed_stream(mom5gpu_domain* d, const MixArgs& a, int n0) {
+  const int ntr = a.ntr, rows = stream_tile_rows(d->tune_mixed_rows, ntr);
+  return STREAM_DISPATCH(run, d, a, n0);
+}
+
+int prepare_batch_mixed() {
+  return configure_batch_rows<1>() | configure_batch_rows<2>() | configure_batch_rows<3>() |
+                 configure_batch_rows<4>() | configure_batch_rows<5>()
+             ? MOM5GPU_ECUDA
+             : MOM5GPU_OK;
+}
+
+int launch_batch_mixed(const MixArgs* mix, const BatchWork& w, int ntr, int tuned_rows, int blocks_per_sm, int sms,
+                       int* counter, cudaStream_t s) {
+  if (w.tm <= 0) return MOM5GPU_OK;
+  const int rows = stream_tile_rows(tuned_rows, ntr);
+  return STREAM_DISPATCH(run_batch, mix, w, blocks_per_sm, sms, counter, s);
+}
+
+}  // namespace mom5
