@@ -7,6 +7,7 @@
 
 #include "internal.h"
 #include "fp64_div.cuh"
+#include "fp64_mul.cuh"
 
 namespace mom5 {
 namespace fp64 {
@@ -20,16 +21,6 @@ DEVI long IM(const Geo& g, int i, int j, int k) { return ((long)k * (g.nj + 4) +
 
 constexpr double kOneSixth = 1.0 / 6.0;  // ocean_parameters.F90:92
 
-// max(0, x) and min(a, b) on the integer pipe (ordered-integer comparison of
-// the bit patterns; equal to the FP comparison for all non-NaN operands).  The
-// bit patterns are taken through bits_of so that the compiler keeps the tests
-// integer.
-DEVI long long ordbits(double x) {
-  long long b = bits_of(x);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
-}
-DEVI double dmin(double a, double b) { return ordbits(a) <= ordbits(b) ? a : b; }
-DEVI double dmax0(double x) { return bits_of(x) > 0 ? x : 0.0; }
 DEVI bool dpos(double x) {  // x > 0 (false for NaN)
   long long b = bits_of(x);
   return b > 0 && b <= 0x7ff0000000000000LL;
@@ -42,8 +33,9 @@ DEVI bool is_one(double m) { return bits_of(m) == 0x3ff0000000000000LL; }
 DEVI bool is_zero(double m) { return (bits_of(m) << 1) == 0; }
 // x*m for a mask value m: 1 -> x (x*1 == x), +-0 -> 0.0 as the callers' selects do
 DEVI double mask_mul(double x, double m) {
-  if (is_one(m)) return x;
-  return x * m;
+  double r = x;
+  rare_lanes(!is_one(m), [&] { r = x * m; });
+  return r;
 }
 // x + 0.0: the same value except that -0 becomes +0
 DEVI double plus_zero(double x) { return bits_of(x) == (long long)0x8000000000000000ULL ? 0.0 : x; }
@@ -53,38 +45,49 @@ DEVI double neg_if(double x, bool flip) {
 }
 // 0.5*x: for a normal x whose exponent field is at least 2 the product is the
 // exponent lowered by one; +-0 is unchanged.  Subnormals, the smallest normals,
-// Inf and NaN take the multiply (decided per warp, so the common case issues no
-// FP64 instruction).
+// Inf and NaN take the multiply.
 DEVI double half_exact(double x) {
   long long b = bits_of(x);
   unsigned e = (unsigned)((unsigned long long)b >> 52) & 0x7ffu;
   bool normal = e - 2u < 0x7fdu;  // 2 <= e <= 0x7fe
-  bool fast = normal || (b << 1) == 0;
-  long long r = normal ? b - (1LL << 52) : b;
-  if (__all_sync(__activemask(), fast)) return double_of(r);
-  return fast ? double_of(r) : 0.5 * x;
+  double r = double_of(normal ? b - (1LL << 52) : b);
+  rare_lanes(!(normal || (b << 1) == 0), [&] { r = 0.5 * x; });
+  return r;
 }
 
-// Arithmetic policy of the MDFL bodies: the FP64 instructions.  (Integer-pipe
-// emulation of the FP64 additions and products was measured on C2 and was
-// 13-90% slower than the FP64 pipe at this occupancy, so none is used.)
-struct HwArith {
+// Arithmetic of an MDFL pass: sums on the FP64 pipe, the products whose bit is set
+// in MASK on the integer pipe.  The four of a face (d1*theta, c*theta, psi*Rj, the
+// mass flux) go there; with one more of the update's the passes took 0 to 3%
+// longer, with none 17 to 41% (z 1.71 -> 1.21 ms, x 1.67 -> 1.39, y 2.08 -> 1.77 for
+// 10 tracers on 360x270x50): by then the FP64 pipe is 65 to 76% busy, the adder and
+// logic pipe 50 to 57%, and the rest is latency at 20 to 31 warps per SM.
+template <unsigned MASK>
+struct Arith {
   static DEVI double add(double a, double b) { return a + b; }
   static DEVI double sub(double a, double b) { return a - b; }
   static DEVI double mul(double a, double b) { return a * b; }
+  // product B of a face: theta, psi and Rj are often zero
+  template <int B>
+  static DEVI double face_mul(double a, double b) {
+    if constexpr ((MASK >> B) & 1) return mul_int<B == 2, B <= 2>(a, b);
+    return a * b;
+  }
 };
-using MdflFaceArith = HwArith;
-using MdflUpdArith = HwArith;
+using FaceArith = Arith<15>;
 
 // Sweby limiter psi (ocean_tracer_advect.F90:3868-3878).  With the limiter on
 // the reference forms psi*(1-1) + max(...)*1, with it off psi*1 + max(...)*0;
 // for finite psi both reduce to the selected term exactly.
 template <bool SWEBY, class Ar>
 DEVI double limiter(double theta, double d0, double d1, double c) {
-  double lin = Ar::add(d0, Ar::mul(d1, theta));
+  double lin = Ar::add(d0, Ar::template face_mul<0>(d1, theta));
   if (!SWEBY) return lin;
-  double a = dmin(1.0, lin);
-  return dmax0(dmin(a, Ar::mul(c, theta)));
+  // max(0, min(1, lin, c*theta)) on the bit patterns as integers: they order
+  // non-negative values, and whichever of two negative ones is taken, 0 results
+  long long m = bits_of(lin), ct = bits_of(Ar::template face_mul<1>(c, theta));
+  m = m < ct ? m : ct;
+  m = m < 0x3ff0000000000000LL ? m : 0x3ff0000000000000LL;
+  return double_of(m > 0 ? m : 0);
 }
 
 // Flux of one face given the upwind-side data.  Reference form
@@ -103,8 +106,8 @@ DEVI double face_flux(double mf, double Rjm, double Rj, double Rjp, double Tp, d
   bool neg = b < 0 && b != (long long)0x8000000000000000ULL;        // mf < 0
   double theta = div_seeded(pos ? Rjm : Rjp, add_1em30(Rj));
   double psi = limiter<SWEBY, Ar>(theta, d0, d1, c);
-  double p = Ar::mul(psi, Rj);
-  double r = Ar::mul(mf, Ar::add(pos ? Tp : Tm, neg_if(p, !pos)));
+  double p = Ar::template face_mul<2>(psi, Rj);
+  double r = Ar::template face_mul<3>(mf, Ar::add(pos ? Tp : Tm, neg_if(p, !pos)));
   return (pos || neg) ? r : 0.0;
 }
 
@@ -143,8 +146,9 @@ DEVI double z_rdiff(const MdflArgs& a, const Geo& g, const double* T, int i, int
 // from the surface would carry into level k0 -- the flux through its top face
 // (the bottom face of level k0-1) and R(k0-1), R(k0) -- with the same
 // operations, so every segment length gives the same bits.
-template <bool ALL, bool SWEBY, int MAXN, class Ar = MdflFaceArith, class Au = MdflUpdArith, bool SEG = false>
+template <bool ALL, bool SWEBY, int MAXN, bool SEG = false>
 DEVI void mdfl_z_body(MdflArgs a, int bx, int by, int k0 = 0, int k1 = -1) {
+  using Ar = FaceArith;
   // ftp: flux through the top face; Rp, Rc: the masked differences R(k-1), R(k),
   // R(k) = (m(k) && m(k1)) ? T(k) - T(k1) : 0 with k1 = min(k+1, nk-1).  The
   // reference's Rjp at level k is R(k-1) (+0 at k = 0) and its Rjm is R(k+1), so
@@ -218,12 +222,12 @@ DEVI void mdfl_z_body(MdflArgs a, int bx, int by, int k0 = 0, int k1 = -1) {
       Rp[n][t] = Rj;
       Rc[n][t] = Rjm;
       double fbt = fm ? face_flux<SWEBY, Ar>(massflux, Rjm, Rj, Rjp, Tkp1, Tk, d0, d1, c) : 0.0;
-      double div = Au::add(Au::mul(datr, Au::sub(fbt, ftp[n][t])), Au::mul(Tk, wdiff));
+      double div = Ar::add(Ar::mul(datr, Ar::sub(fbt, ftp[n][t])), Ar::mul(Tk, wdiff));
       double tm;
       if (!ALL) {
-        tm = Au::add(Tk, Au::mul(dtr, div));
+        tm = Ar::add(Tk, Ar::mul(dtr, div));
       } else {
-        tm = Au::add(Tk, div_seeded(Au::mul(div, a.dtime), rdz));
+        tm = Ar::add(Tk, div_seeded(Ar::mul(div, a.dtime), rdz));
       }
       a.tz[n * g.n3 + p] = tm;
       ftp[n][t] = fbt;
@@ -298,8 +302,9 @@ DEVI void x_face(const MdflArgs& a, int i, int j, int k, double (*sm)[kTX + 1], 
   }
 }
 
-template <bool ALL, bool SWEBY, int MAXN, class Ar = MdflFaceArith, class Au = MdflUpdArith>
+template <bool ALL, bool SWEBY, int MAXN>
 DEVI void mdfl_x_body(MdflArgs a, int bx, int by, int bz) {
+  using Ar = FaceArith;
   __shared__ double sm[MAXN][kTX + 1], Rs[MAXN][kTX + 3];
   const Geo& g = a.g;
   int i0 = bx * kTX + 1;
@@ -333,12 +338,12 @@ DEVI void mdfl_x_body(MdflArgs a, int bx, int by, int bz) {
   for (int n = 0; n < a.ntr; ++n) {
     double Tk = a.T[n * a.tstride + p];
     double tm = a.tz[n * g.n3 + p];
-    double s = Au::add(Au::sub(sm[n][t], sm[n][t + 1]), Au::mul(Tk, divx));
+    double s = Ar::add(Ar::sub(sm[n][t], sm[n][t + 1]), Ar::mul(Tk, divx));
     if (!ALL) {
-      tm = Au::add(tm, Au::mul(coef, s));
+      tm = Ar::add(tm, Ar::mul(coef, s));
     } else {
-      double w1 = mk ? Au::mul(datr, s) : 0.0;
-      tm = Au::add(tm, div_seeded(Au::mul(w1, a.dtime), rdz));
+      double w1 = mk ? Ar::mul(datr, s) : 0.0;
+      tm = Ar::add(tm, div_seeded(Ar::mul(w1, a.dtime), rdz));
     }
     a.tx[n * g.n3 + p] = tm;
   }
@@ -388,8 +393,9 @@ DEVI double y_flux(const MdflArgs& a, const YFace& f, int i, int j, int k, int n
 // flux of the row's north face in a register, the south face's from the
 // previous row in shared memory), so the per-tracer shared state is fprev, Ra
 // and Rb only.
-template <bool ALL, bool SWEBY, int MAXN, class Ar = MdflFaceArith, class Au = MdflUpdArith>
+template <bool ALL, bool SWEBY, int MAXN>
 DEVI void mdfl_y_body(MdflArgs a, int TJ, int bx, int by, int bz) {
+  using Ar = FaceArith;
   __shared__ double fprev[MAXN][kMdflThreads];
   __shared__ double Ra[MAXN][kMdflThreads], Rb[MAXN][kMdflThreads];
   const Geo& g = a.g;
@@ -438,15 +444,15 @@ DEVI void mdfl_y_body(MdflArgs a, int TJ, int bx, int by, int bz) {
       double fp = fprev[n][t];
       double out;
       if (!ALL) {
-        tm = Au::add(tm, Au::mul(coef, Au::sub(fp, fc)));
-        tm = Au::add(tm, Au::mul(div_pair(Au::mul(a.dtime, Tk), rdz, rr_h, rr_l), corr));
+        tm = Ar::add(tm, Ar::mul(coef, Ar::sub(fp, fc)));
+        tm = Ar::add(tm, Ar::mul(div_pair(Ar::mul(a.dtime, Tk), rdz, rr_h, rr_l), corr));
       } else {
-        double w1 = Au::add(mk ? Au::mul(datr, Au::sub(fp, fc)) : 0.0, Au::mul(Tk, corr));
-        tm = Au::add(tm, div_pair(Au::mul(w1, a.dtime), rdz, rr_h, rr_l));
+        double w1 = Ar::add(mk ? Ar::mul(datr, Ar::sub(fp, fc)) : 0.0, Ar::mul(Tk, corr));
+        tm = Ar::add(tm, div_pair(Ar::mul(w1, a.dtime), rdz, rr_h, rr_l));
       }
-      out = mk ? div_pair(Au::mul(rdz, Au::sub(tm, Tk)), a.dtime, rdt_h, rdt_l) : 0.0;
+      out = mk ? div_pair(Ar::mul(rdz, Ar::sub(tm, Tk)), a.dtime, rdt_h, rdt_l) : 0.0;
       double* th = a.th + n * g.n3;
-      th[p] = a.th_fresh ? plus_zero(out) : Au::add(th[p], out);  // +0 + out == plus_zero(out)
+      th[p] = a.th_fresh ? plus_zero(out) : Ar::add(th[p], out);  // +0 + out == plus_zero(out)
       fprev[n][t] = fc;
     }
   }

@@ -27,6 +27,18 @@ DEVI double double_of(long long b) {
   return x;
 }
 
+// f() for the lanes with `rare` set, in a loop that runs once: the assembler turns
+// a branch around a few instructions into predicated ones, and an FP64
+// instruction takes its 19.4 cycles of the pipe with every lane switched off too
+// (measured: a product on the integer pipe whose fallback was a branch left the
+// FP64 pipe's instruction count as it was).
+template <class F>
+DEVI void rare_lanes(bool rare, F&& f) {
+  const unsigned act = __activemask();
+  for (unsigned m = __ballot_sync(act, rare); m; m &= ~act)
+    if (rare) f();
+}
+
 // Quotients by long division on the integer pipe.  GB300 issues one FP64 warp
 // instruction per 19.4 SM cycles (measured; the number of active lanes does not
 // matter), an integer one per 0.3 to 0.5 (the 64-bit product and the high half
@@ -49,11 +61,15 @@ DEVI double double_of(long long b) {
 // midpoint of two doubles, so Q's bits below the result's last one round it
 // correctly without a sticky bit.
 //
-// Normal operands with a normal result take this path, and a zero dividend
-// with a normal divisor; any other lane takes the division instruction, so
+// Operands of an exponent within 2^-510 .. 2^512 take this path, and a zero
+// dividend with such a divisor; any other lane takes the division instruction, so
 // every function returns exactly the IEEE result.
+//
+// Shifts are written as products where that lets the multiply-add pipe do them:
+// with the products of the schemes on the integer pipe too, the adder and logic
+// pipe is what bounds the rest.
 struct Divisor {
-  unsigned hi, nlo, nhi, y;  // high word of b; -B modulo 2^64; 24-bit reciprocal
+  unsigned ex, nlo, nhi, y;  // sign and exponent of b (its high word less the significand's); -B modulo 2^64; 24-bit reciprocal
 };
 DEVI Divisor divisor_of(double b) {
   const unsigned hi = (unsigned)__double2hiint(b), lo = (unsigned)__double2loint(b);
@@ -63,34 +79,39 @@ DEVI Divisor divisor_of(double b) {
   unsigned yb = __float_as_uint(y);
   yb = yb < 0x3f7fffffu ? yb : 0x3f7fffffu;  // rcp(1) = 1 would lose its leading bit
   const unsigned long long nb = 0ULL - (((unsigned long long)m << 32) | lo);
-  return {hi, (unsigned)nb, (unsigned)(nb >> 32), ((yb & 0x7fffffu) | 0x800000u) - 4u};
+  return {hi - m, (unsigned)nb, (unsigned)(nb >> 32), ((yb & 0x7fffffu) | 0x800000u) - 4u};
 }
 // The next 18-bit digit of r / B; r becomes the remainder.
 DEVI unsigned div_digit(unsigned long long& r, const Divisor& d) {
-  const unsigned q = __umulhi((unsigned)(r >> 26), d.y);
-  r = (r << 18) + (unsigned long long)q * d.nlo;
-  r += (unsigned long long)(q * d.nhi) << 32;
+  const unsigned q = __umulhi((unsigned)(r >> 26), d.y), rh = (unsigned)(r >> 32);
+  r = (unsigned long long)(unsigned)r * (1u << 18) + (unsigned long long)q * d.nlo;
+  r += (unsigned long long)(q * d.nhi + rh * (1u << 18)) << 32;
   return q;
 }
 DEVI double div_by(double a, double b, const Divisor& d) {
   const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
-  const unsigned ea = ah & 0x7ff00000u, eb = d.hi & 0x7ff00000u, sign = (ah ^ d.hi) & 0x80000000u;
-  unsigned long long r = ((unsigned long long)((ah & 0xfffffu) | 0x100000u) << 32) | al;
+  const unsigned am = (ah & 0xfffffu) | 0x100000u;
+  unsigned long long r = ((unsigned long long)am << 32) | al;
   const unsigned q1 = div_digit(r, d), q2 = div_digit(r, d), q3 = div_digit(r, d);
-  unsigned long long q = (unsigned long long)q2 * (1u << 18) + q3 + ((unsigned long long)(q1 << 4) << 32);
+  const unsigned long long q = (unsigned long long)q2 * (1u << 18) + q3;
+  unsigned ql, qh;
   // r + (-B) carries out of 64 bits where r >= B
-  q += r + (((unsigned long long)d.nhi << 32) | d.nlo) < r ? 1 : 0;
-  const unsigned sh = (unsigned)(q >> 32) >= (1u << 22) ? 2u : 1u;  // bits below the result's last
-  q = (q + sh) >> sh;                                               // half of the last place is sh
-  const unsigned rh = (unsigned)(q >> 32) + (ea - eb + ((1020u + sh) << 20));  // q's leading bit adds one to the field
-  const bool bn = eb - 0x100000u < 0x7fe00000u;
-  bool ok = bn && ea - 0x100000u < 0x7fe00000u && rh - 0x100000u < 0x7fe00000u;
-  unsigned lo = (unsigned)q, hi = rh | sign;
-  if (((ah & 0x7fffffffu) | al) == 0) lo = 0, hi = sign, ok = bn;  // 0 / b
+  asm("{\n .reg .u32 t;\n add.cc.u32 t, %2, %4;\n addc.cc.u32 t, %3, %5;\n addc.cc.u32 %0, %6, 0;\n addc.u32 %1, %7, 0;\n}"
+      : "=r"(ql), "=r"(qh)
+      : "r"((unsigned)r), "r"((unsigned)(r >> 32)), "r"(d.nlo), "r"(d.nhi), "r"((unsigned)q),
+        "r"((unsigned)(q >> 32) + q1 * 16u));
+  // one or two bits lie below the result's last: Q 2^31 or 2^30 plus half of 2^32, over 2^32
+  const unsigned top = qh >> 22, m = 0x80000000u >> top;
+  const unsigned long long w0 = (unsigned long long)ql * m + 0x80000000u;
+  const unsigned long long w = (unsigned long long)qh * m + (w0 >> 32);
+  // the signs' sum and the exponents' difference; w's leading bit adds one to the field
+  unsigned lo = (unsigned)w, hi = (unsigned)(w >> 32) + (ah - am - d.ex) + 0x3fd00000u + top * 0x100000u;
+  const unsigned eb = (d.ex + 0x100000u) * 2u - 0x40000000u;
+  const bool bn = (int)eb >= 0, zero = ((ah << 1) | al) == 0;
+  const bool ok = bn && (zero || ah * 2u - 0x40400000u < 0x7fc00000u);
+  if (zero) lo = 0, hi = (ah ^ d.ex) & 0x80000000u;
   double x = __hiloint2double((int)hi, (int)lo);
-  if (!__all_sync(__activemask(), ok)) {
-    if (!ok) x = a / b;
-  }
+  rare_lanes(!ok, [&] { x = a / b; });
   return x;
 }
 
@@ -101,7 +122,7 @@ DEVI double div_seeded(double a, double b) { return div_by(a, b, divisor_of(b));
 // reciprocal, yl the negated significand.
 DEVI void recip_pair(double b, double& yh, double& yl) {
   const Divisor d = divisor_of(b);
-  yh = __hiloint2double((int)d.hi, (int)d.y);
+  yh = __hiloint2double((int)d.ex, (int)d.y);
   yl = __hiloint2double((int)d.nhi, (int)d.nlo);
 }
 DEVI double div_pair(double a, double b, double yh, double yl) {
@@ -113,17 +134,14 @@ DEVI double div_pair(double a, double b, double yh, double yl) {
 // +-0 gives the constant 1e-30, and for |x| >= 2^-45 (biased exponent >= 978)
 // the sum rounds back to x (1e-30 is below half an ulp of x, also of the
 // binade under x when x is a negative power of two).  Tiny non-zero x, Inf and
-// NaN take the addition (decided per warp; the addition is volatile so that it
-// is not hoisted above the vote and issued for every lane).
+// NaN take the addition.
 DEVI double add_1em30(double x) {
   long long b = bits_of(x);
   unsigned e = (unsigned)((unsigned long long)b >> 52) & 0x7ffu;
   bool zero = (b << 1) == 0;
   bool keep = e >= 978u && e <= 2046u;
-  bool fast = zero || keep;
   double r = zero ? 1.0e-30 : x;
-  if (__all_sync(__activemask(), fast)) return r;
-  if (!fast) asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(1.0e-30), "d"(x));
+  rare_lanes(!(zero || keep), [&] { r = 1.0e-30 + x; });
   return r;
 }
 

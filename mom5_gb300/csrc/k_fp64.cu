@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(128) k_mdfl_z(MdflArgs a) {
 template <bool ALL, bool SWEBY, int MAXN>
 __global__ void __launch_bounds__(128) k_mdfl_z_seg(MdflArgs a, int L) {
   const int k0 = blockIdx.z * L;
-  mdfl_z_body<ALL, SWEBY, MAXN, MdflFaceArith, MdflUpdArith, true>(a, blockIdx.x, blockIdx.y, k0, k0 + L);
+  mdfl_z_body<ALL, SWEBY, MAXN, true>(a, blockIdx.x, blockIdx.y, k0, k0 + L);
 }
 
 // Levels per z-pass segment.  A domain with few columns gives the column march
