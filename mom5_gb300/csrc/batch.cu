@@ -20,7 +20,6 @@ struct mom5gpu_batch {
   std::string err;
   // descriptor tables, entry 2*d + parity (parity 0: tau 1 -> 2, parity 1: 2 -> 1)
   MdflArgs* d_mdfl = nullptr;
-  UpdArgs* d_upd = nullptr;
   BtArgs* d_bt = nullptr;
   BtExtra* d_btx = nullptr;
   MixArgs* d_mix = nullptr;
@@ -64,9 +63,7 @@ int default_tj(const mom5gpu_batch* b) {
   for (auto* d : b->doms) cols += (long)d->geo.ni * d->geo.nk;
   long nj = 0;
   for (auto* d : b->doms) nj = std::max<long>(nj, d->geo.nj);
-  int TJ = 16;
-  while (TJ > 2 && cols * ((nj + TJ - 1) / TJ) < 152L * 32 * 16) TJ /= 2;
-  return TJ;
+  return y_strip_rows(cols, nj);
 }
 
 int tj_of(const mom5gpu_batch* b) { return b->tj > 0 ? b->tj : default_tj(b); }
@@ -74,7 +71,6 @@ int tj_of(const mom5gpu_batch* b) { return b->tj > 0 ? b->tj : default_tj(b); }
 int build_descriptors(mom5gpu_batch* b, double dtime) {
   int n = (int)b->doms.size();
   std::vector<MdflArgs> m(2 * n);
-  std::vector<UpdArgs> u(2 * n);
   std::vector<BtArgs> bt(2 * n);
   std::vector<BtExtra> bx(2 * n);
   std::vector<MixArgs> mx(2 * n);
@@ -85,9 +81,8 @@ int build_descriptors(mom5gpu_batch* b, double dtime) {
       int rc = MOM5GPU_OK;
       if (b->prec == MOM5GPU_PRECISION_FP64) {
         if ((rc = make_mdfl_args(d, 1, b->ntr, taum1, tau, dtime, &m[2 * i + p])) ||
-            (rc = make_upd_args(d, taum1, taup1, dtime, &u[2 * i + p])))
+            (rc = add_step_args(d, 1, taum1, taup1, &m[2 * i + p])))
           return bfail(b, rc, "domain %d: %s", i, d->err.c_str());
-        m[2 * i + p].th_fresh = 1;  // the step zeroes only the halo ring of th_tendency
       } else if ((rc = make_mix_args(d, taum1, tau, taup1, dtime, &mx[2 * i + p]))) {
         return bfail(b, rc, "domain %d: %s", i, d->err.c_str());
       }
@@ -98,7 +93,6 @@ int build_descriptors(mom5gpu_batch* b, double dtime) {
   cudaError_t e = cudaSuccess;
   if (b->prec == MOM5GPU_PRECISION_FP64) {
     e = cudaMemcpyAsync(b->d_mdfl, m.data(), sizeof(MdflArgs) * 2 * n, cudaMemcpyHostToDevice, b->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_upd, u.data(), sizeof(UpdArgs) * 2 * n, cudaMemcpyHostToDevice, b->stream);
   } else {
     e = cudaMemcpyAsync(b->d_mix, mx.data(), sizeof(MixArgs) * 2 * n, cudaMemcpyHostToDevice, b->stream);
   }
@@ -112,7 +106,7 @@ int build_descriptors(mom5gpu_batch* b, double dtime) {
 }
 
 // Work list of (domain, parity) entries as ints: entries, then the prefix sums of
-// the passes z, x, y, update, 2-D barotropic, 1-D barotropic, precision form.
+// the passes z, x, y, 2-D barotropic, 1-D barotropic, precision form.
 void fill_work(const mom5gpu_batch* b, const std::vector<std::pair<int, int>>& list, std::vector<int>& h, BatchWork& w) {
   int c = (int)list.size();
   int TJ = tj_of(b);
@@ -121,10 +115,10 @@ void fill_work(const mom5gpu_batch* b, const std::vector<std::pair<int, int>>& l
   std::stable_sort(order.begin(), order.end(), [&](const std::pair<int, int>& a, const std::pair<int, int>& z) {
     return b->doms[a.first]->geo.n3 > b->doms[z.first]->geo.n3;
   });
-  h.assign((size_t)c + 7 * (size_t)(c + 1), 0);
+  h.assign((size_t)c + 6 * (size_t)(c + 1), 0);
   int* ent = h.data();
-  int* pr[7];
-  for (int k = 0; k < 7; ++k) pr[k] = ent + c + k * (c + 1);
+  int* pr[6];
+  for (int k = 0; k < 6; ++k) pr[k] = ent + c + k * (c + 1);
   // the precision form's tiles are cut into segments of one length, chosen for all of them together
   const int rows = stream_tile_rows(b->rows, b->ntr);
   long tiles = 0;
@@ -139,17 +133,16 @@ void fill_work(const mom5gpu_batch* b, const std::vector<std::pair<int, int>>& l
     const int dom = order[e].first;
     ent[e] = 2 * dom + order[e].second;
     BatchBlocks bb = batch_blocks(b->doms[dom]->geo, TJ, rows, w.seg);
-    int v[7] = {bb.z, bb.x, bb.y, bb.u, bb.b2, bb.b1, bb.m};
-    for (int k = 0; k < 7; ++k) pr[k][e + 1] = pr[k][e] + v[k];
+    int v[6] = {bb.z, bb.x, bb.y, bb.b2, bb.b1, bb.m};
+    for (int k = 0; k < 6; ++k) pr[k][e + 1] = pr[k][e] + v[k];
   }
   w.count = c;
   w.tz = pr[0][c];
   w.tx = pr[1][c];
   w.ty = pr[2][c];
-  w.tu = pr[3][c];
-  w.tb2 = pr[4][c];
-  w.tb1 = pr[5][c];
-  w.tm = pr[6][c];
+  w.tb2 = pr[3][c];
+  w.tb1 = pr[4][c];
+  w.tm = pr[5][c];
 }
 
 void bind_work(BatchWork& w, const int* d) {
@@ -159,10 +152,9 @@ void bind_work(BatchWork& w, const int* d) {
   w.pz = p;
   w.px = p + (c + 1);
   w.py = p + 2 * (c + 1);
-  w.pu = p + 3 * (c + 1);
-  w.pb2 = p + 4 * (c + 1);
-  w.pb1 = p + 5 * (c + 1);
-  w.pm = p + 6 * (c + 1);
+  w.pb2 = p + 3 * (c + 1);
+  w.pb1 = p + 4 * (c + 1);
+  w.pm = p + 5 * (c + 1);
 }
 
 // every kernel of one batched step, in stream order
@@ -172,21 +164,8 @@ int enqueue_step(mom5gpu_batch* b, const BatchWork& w, const std::vector<std::pa
   long launches = 0;
   if (b->ntr > 0) {
     if (b->prec == MOM5GPU_PRECISION_FP64) {
-      for (auto& it : list) {
-        mom5gpu_domain* d = b->doms[it.first];
-        double* th = fptr(d, MOM5GPU_TH_TENDENCY, 1, 0);
-        launch_zero_ring(d->geo, th, (long)b->ntr * d->geo.nk, s);
-        ++launches;
-      }
-      launch_batch_fp64_advection(b->d_mdfl, b->d_upd, w, b->ntr, true, tj_of(b), s);
-      launches += 4;
-      for (auto& it : list) {
-        mom5gpu_domain* d = b->doms[it.first];
-        if (!(d->geo.cx || d->geo.cy)) continue;
-        double* tp1 = fptr(d, MOM5GPU_TRACER, 1, 2 - it.second);
-        launch_halo_fill(d->geo, tp1, b->ntr * d->geo.nk, 3, s);  // every tracer's levels, one after another
-        launches += 1;
-      }
+      launch_batch_fp64_advection(b->d_mdfl, w, b->ntr, true, tj_of(b), s);
+      launches += 3;
     } else {
       rc = launch_batch_mixed(b->d_mix, w, b->ntr, b->rows, b->blocks_per_sm, b->sms, b->d_counter, s);
       if (rc) return bfail(b, rc, "precision-form batch launch");
@@ -353,7 +332,6 @@ int mom5gpu_batch_create(mom5gpu_domain* const* domains, int n, mom5gpu_batch** 
   if (e == cudaSuccess) e = cudaMalloc(&b->d_counter, sizeof(int));
   if (e == cudaSuccess && b->prec == MOM5GPU_PRECISION_FP64) {
     e = cudaMalloc(&b->d_mdfl, sizeof(MdflArgs) * nd);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_upd, sizeof(UpdArgs) * nd);
   } else if (e == cudaSuccess) {
     e = cudaMalloc(&b->d_mix, sizeof(MixArgs) * nd);
   }
@@ -388,7 +366,7 @@ void mom5gpu_batch_destroy(mom5gpu_batch* b) {
     if (b->gexec[p]) cudaGraphExecDestroy(b->gexec[p]);
     if (b->d_work_all[p]) cudaFree(b->d_work_all[p]);
   }
-  for (void* p : {(void*)b->d_mdfl, (void*)b->d_upd, (void*)b->d_bt, (void*)b->d_btx, (void*)b->d_mix, (void*)b->d_work,
+  for (void* p : {(void*)b->d_mdfl, (void*)b->d_bt, (void*)b->d_btx, (void*)b->d_mix, (void*)b->d_work,
                   (void*)b->d_counter})
     if (p) cudaFree(p);
   if (b->e0) cudaEventDestroy(b->e0);

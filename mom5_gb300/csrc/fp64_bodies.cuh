@@ -278,14 +278,18 @@ DEVI double tx_halo(const MdflArgs& a, int n, int i, int j, int k) {
   return tm_yhalo(g, a.tx + n * g.n3, i, j, k);
 }
 
-constexpr int kTX = 128;
+// An x block's threads form one face each, which closes one cell less: a 129th face
+// would cost a warp of its own, all of a face's FP64 instructions for one lane
+// (360x270x50, 10 tracers: 1.39 -> 1.12 ms).
+constexpr int kTX = 128, kXCells = kTX - 1;
+__host__ __device__ inline int x_blocks(const Geo& g) { return (g.ni + kXCells - 1) / kXCells; }
 
 // x-face i of row (j,k): fluxes of every tracer into sm[n][slot].  Rs[n][r-1..r+1]
 // hold the masked differences R of faces i-1, i, i+1 (the reference's Rjm, Rj,
 // Rjp), each formed once per block.
 template <bool SWEBY, int MAXN, class Ar>
-DEVI void x_face(const MdflArgs& a, int i, int j, int k, double (*sm)[kTX + 1], int slot,
-                 const double (*Rs)[kTX + 3], int r) {
+DEVI void x_face(const MdflArgs& a, int i, int j, int k, double (*sm)[kTX], int slot, const double (*Rs)[kTX + 2],
+                 int r) {
   const Geo& g = a.g;
   bool m1 = a.mask2[IM(g, i, j, k)], m2 = a.mask2[IM(g, i + 1, j, k)];
   double u = a.uh[I3(g, i, j, k)];
@@ -305,15 +309,15 @@ DEVI void x_face(const MdflArgs& a, int i, int j, int k, double (*sm)[kTX + 1], 
 template <bool ALL, bool SWEBY, int MAXN>
 DEVI void mdfl_x_body(MdflArgs a, int bx, int by, int bz) {
   using Ar = FaceArith;
-  __shared__ double sm[MAXN][kTX + 1], Rs[MAXN][kTX + 3];
+  __shared__ double sm[MAXN][kTX], Rs[MAXN][kTX + 2];
   const Geo& g = a.g;
-  int i0 = bx * kTX + 1;
+  int i0 = bx * kXCells + 1;
   int j = by + 1;
   int k = bz;
   int t = threadIdx.x;
-  int i = i0 + t;
-  // R(f) = (m(f) && m(f+1)) ? tz(f+1) - tz(f) : 0 for faces f = i0-2 .. i0+128 (slot f-i0+2)
-  for (int sl = t; sl < kTX + 3; sl += kTX) {
+  int i = i0 - 1 + t;  // this thread's face and, from thread 1 on, its cell
+  // R(f) = (m(f) && m(f+1)) ? tz(f+1) - tz(f) : 0 for faces f = i0-2 .. i0+127 (slot f-i0+2)
+  for (int sl = t; sl < kTX + 2; sl += kTX) {
     int f = i0 - 2 + sl;
     if (f > g.ni + 1) continue;
     bool ma = a.mask2[IM(g, f, j, k)], mb = a.mask2[IM(g, f + 1, j, k)];
@@ -323,10 +327,9 @@ DEVI void mdfl_x_body(MdflArgs a, int bx, int by, int bz) {
     }
   }
   __syncthreads();
-  if (i <= g.ni) x_face<SWEBY, MAXN, Ar>(a, i, j, k, sm, t + 1, Rs, t + 2);
-  if (t == 0) x_face<SWEBY, MAXN, Ar>(a, i0 - 1, j, k, sm, 0, Rs, 1);
+  if (i <= g.ni) x_face<SWEBY, MAXN, Ar>(a, i, j, k, sm, t, Rs, t + 1);
   __syncthreads();
-  if (i > g.ni) return;
+  if (t == 0 || i > g.ni) return;
   bool mk = a.mask2[IM(g, i, j, k)];
   double datr = a.datr[I2(g, i, j)];
   double rdz = a.rdz[I3(g, i, j, k)];
@@ -338,7 +341,7 @@ DEVI void mdfl_x_body(MdflArgs a, int bx, int by, int bz) {
   for (int n = 0; n < a.ntr; ++n) {
     double Tk = a.T[n * a.tstride + p];
     double tm = a.tz[n * g.n3 + p];
-    double s = Ar::add(Ar::sub(sm[n][t], sm[n][t + 1]), Ar::mul(Tk, divx));
+    double s = Ar::add(Ar::sub(sm[n][t - 1], sm[n][t]), Ar::mul(Tk, divx));
     if (!ALL) {
       tm = Ar::add(tm, Ar::mul(coef, s));
     } else {
@@ -389,6 +392,24 @@ DEVI double y_flux(const MdflArgs& a, const YFace& f, int i, int j, int k, int n
   return f.fm ? face_flux<SWEBY, Ar>(f.massflux, Rjm, Rj, Rjp, tB, tC, f.d0, f.d1, f.c) : 0.0;
 }
 
+// What a whole step leaves outside the compute domain, by the threads of its outer
+// cells: the periodic images of T(taup1) = tn (ocean_model.F90:1903-1911) and the
+// zeros of th_tendency's halo ring.
+// (Scalars: a reference to the kernel's arguments would move them to the stack.)
+static __device__ __noinline__ void step_edges(double* T1, double* th, double tn, int i, int j, int ni, int nj, bool cx,
+                                               bool cy) {
+  const long nxd = ni + 2;  // T1, th: the level's planes
+  for (int dj = -1; dj <= 1; ++dj)
+    for (int di = -1; di <= 1; ++di) {
+      if (di == 0 && dj == 0) continue;
+      const bool wx = di < 0 ? i == 1 : i == ni, wy = dj < 0 ? j == 1 : j == nj;
+      if ((di == 0 || wx) && (dj == 0 || wy)) th[(j + dj) * nxd + i + di] = 0.0;
+      const bool ex = di < 0 ? i == ni : i == 1, ey = dj < 0 ? j == nj : j == 1;
+      const int u = di == 0 ? i : di < 0 ? 0 : ni + 1, v = dj == 0 ? j : dj < 0 ? 0 : nj + 1;
+      if ((di == 0 || (cx && ex)) && (dj == 0 || (cy && ey))) T1[v * nxd + u] = tn;
+    }
+}
+
 // Each tracer's face flux is formed and used in the same iteration (the
 // flux of the row's north face in a register, the south face's from the
 // previous row in shared memory), so the per-tracer shared state is fprev, Ra
@@ -436,6 +457,8 @@ DEVI void mdfl_y_body(MdflArgs a, int TJ, int bx, int by, int bz) {
     double coef = ALL ? 0.0 : (mk ? div_seeded(a.dtime * datr, rdz) : 0.0);
     double rr_h, rr_l;  // two-term reciprocal of rho_dzt, shared by every tracer's divisions
     recip_pair(rdz, rr_h, rr_l);
+    const double rm1 = a.Tp1 ? a.rdz_m1[p] : 0.0, rdzr = a.Tp1 ? a.rdzr[p] : 0.0;
+    const bool edge = i == 1 || i == g.ni || j == 1 || j == g.nj;
 #pragma unroll 1
     for (int n = 0; n < a.ntr; ++n) {
       double tm;  // tracer_mdfl after the x pass at (i, j, k)
@@ -452,7 +475,14 @@ DEVI void mdfl_y_body(MdflArgs a, int TJ, int bx, int by, int bz) {
       }
       out = mk ? div_pair(Ar::mul(rdz, Ar::sub(tm, Tk)), a.dtime, rdt_h, rdt_l) : 0.0;
       double* th = a.th + n * g.n3;
-      th[p] = a.th_fresh ? plus_zero(out) : Ar::add(th[p], out);  // +0 + out == plus_zero(out)
+      out = a.th_fresh ? plus_zero(out) : Ar::add(th[p], out);  // +0 + out == plus_zero(out)
+      th[p] = out;
+      if (a.Tp1) {  // the explicit update (ocean_tracer.F90:2341-2350)
+        double* T1 = a.Tp1 + n * a.tstride;
+        const double tn = Ar::mul(Ar::add(mul_int<false, true>(rm1, Tk), a.dtime * out), rdzr);
+        T1[p] = tn;
+        if (edge) step_edges(T1 + (p - I2(g, i, j)), th + (p - I2(g, i, j)), tn, i, j, g.ni, g.nj, g.cx, g.cy);
+      }
       fprev[n][t] = fc;
     }
   }

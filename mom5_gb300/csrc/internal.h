@@ -167,6 +167,10 @@ struct MdflArgs {
   double* th;                 // th_tendency of tracer 0, tracer n at th + n*g.n3
   int tj = 0;                 // y-pass rows per thread (0 = choose from the domain size)
   int th_fresh = 0;           // th is +0 at every compute cell: the y pass writes out + 0.0 instead of th + out
+  // the whole step (th_fresh): the y pass also zeroes th's halo ring and writes the
+  // explicit update with its periodic images; nullptr Tp1: th_tendency only
+  const double *rdz_m1 = nullptr, *rdzr = nullptr;  // rho_dzt(taum1), rho_dztr
+  double* Tp1 = nullptr;                            // tracer 0 at taup1, tracer n at + n*tstride
   // decomposed domains: sides whose halo comes from a neighbouring subdomain
   // (bits 1 west, 2 east, 4 south, 8 north) and the strips its exchange filled:
   // tracer_mdfl after the z pass at i = -1, 0, ni+1, ni+2 (hz[((n*nk + k)*nj + j-1)*4 + slot])
@@ -248,7 +252,11 @@ int launch_barotropic_phase(mom5gpu_domain* d, int tau, int taup1, int phase, in
 void launch_halo_fill(const Geo& g, double* a, int nlev, int flags, cudaStream_t s);
 void launch_zero_ring(const Geo& g, double* a, long nlev, cudaStream_t s);
 int launch_mdfl(mom5gpu_domain* d, bool all, int n_first, int ntr, int taum1, int tau, double dtime,
-                double sweby_limiter, bool th_fresh = false);
+                double sweby_limiter);
+// the whole step of every tracer: th_tendency = its advection, T(taup1) by the explicit update
+int launch_mdfl_step(mom5gpu_domain* d, bool all, int taum1, int tau, int taup1, double dtime);
+int y_strip_rows(long cols, long nj);
+int add_step_args(mom5gpu_domain* d, int n_first, int taum1, int taup1, MdflArgs* a);
 int launch_upwind_horz(mom5gpu_domain* d, int n, int taum1);
 int launch_upwind_vert(mom5gpu_domain* d, int n, int taum1);
 int launch_quicker_horz(mom5gpu_domain* d, int n, int taum1, int tau);
@@ -312,20 +320,19 @@ int ensure_mdfl_scratch(mom5gpu_domain* d, int ntr);
 // e; p*[e] is the first block of entry e in each pass (p*[count] = total).
 struct BatchWork {
   const int* entries;
-  const int *pz, *px, *py, *pu, *pb2, *pb1, *pm;
+  const int *pz, *px, *py, *pb2, *pb1, *pm;
   int count;
-  int tz, tx, ty, tu, tb2, tb1, tm;  // total blocks of each pass
+  int tz, tx, ty, tb2, tb1, tm;      // total blocks of each pass
   int seg;                           // levels per item of the precision form
 };
 // blocks of one domain in each pass, for the work-list prefix sums; m: the
 // precision form's items, tiles of tile_rows rows by segments of seg levels
 struct BatchBlocks {
-  int z, x, y, u, b2, b1, m;
+  int z, x, y, b2, b1, m;
 };
 BatchBlocks batch_blocks(const Geo& g, int TJ, int tile_rows, int seg);
-// FP64: z/x/y MDFL passes and the explicit update for every entry
-void launch_batch_fp64_advection(const MdflArgs* mdfl, const UpdArgs* upd, const BatchWork& w, int ntr, bool sweby,
-                                 int TJ, cudaStream_t s);
+// FP64: z/x/y MDFL passes, the last with the explicit update, for every entry
+void launch_batch_fp64_advection(const MdflArgs* mdfl, const BatchWork& w, int ntr, bool sweby, int TJ, cudaStream_t s);
 // the barotropic step (init, nts x (pred, mom, corr), post) for every entry; halo fills of
 // cyclic domains are issued by the caller between the post phases
 void launch_batch_barotropic_loop(const BtArgs* bt, const BtExtra* x, const BatchWork& w, int nts, int stepB, bool fast,

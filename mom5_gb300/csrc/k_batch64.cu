@@ -1,5 +1,5 @@
-// Batched FP64 kernels: the MDFL passes, the explicit update and the barotropic
-// phases of many domains in one launch each.  A launch's blocks are a flat
+// Batched FP64 kernels: the MDFL passes (the last with the explicit update) and
+// the barotropic phases of many domains in one launch each.  A launch's blocks are a flat
 // work list; a block finds its (domain, block) from the per-pass prefix sums
 // and runs the same body as the one-domain kernel (fp64_bodies.cuh), so every
 // domain's result is identical to stepping it alone.  Built with --fmad=false.
@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(kTX) kb_mdfl_x(const MdflArgs* d, BatchWork w)
   int e = find_entry(w.px, w.count, blockIdx.x);
   const MdflArgs& a = d[w.entries[e]];
   int local = blockIdx.x - w.px[e];
-  int nb = (a.g.ni + kTX - 1) / kTX;
+  int nb = x_blocks(a.g);
   mdfl_x_body<false, SWEBY, MAXN>(a, local % nb, (local / nb) % a.g.nj, local / (nb * a.g.nj));
 }
 
@@ -51,19 +51,6 @@ __global__ void __launch_bounds__(128, 6) kb_mdfl_y(const MdflArgs* d, BatchWork
   mdfl_y_body<false, SWEBY, MAXN>(a, TJ, local % nb, (local / nb) % ns, local / (nb * ns));
 }
 
-__global__ void __launch_bounds__(128) kb_update(const UpdArgs* d, BatchWork w) {
-  int e = find_entry(w.pu, w.count, blockIdx.x);
-  const UpdArgs& u = d[w.entries[e]];
-  const Geo& g = u.g;
-  int local = blockIdx.x - w.pu[e];
-  int nb = (g.ni + 127) / 128;
-  int i = (local % nb) * 128 + threadIdx.x + 1;
-  int j = (local / nb) % g.nj + 1, k = local / (nb * g.nj);
-  if (i > g.ni) return;
-  long p = I3(g, i, j, k);
-  double a = u.rdz_m1[p], r = u.rdzr[p];
-  for (int n = 0; n < u.ntr; ++n) u.Tp1[n * u.tstride + p] = (a * u.Tm1[n * u.tstride + p] + u.dtime * u.th[n * g.n3 + p]) * r;
-}
 
 __global__ void __launch_bounds__(256) kb_bt_init(const BtArgs* d, const BtExtra* xs, BatchWork w) {
   int e = find_entry(w.pb1, w.count, blockIdx.x);
@@ -125,11 +112,10 @@ __global__ void __launch_bounds__(128) kb_bt_post3(const BtArgs* d, const BtExtr
 }
 
 template <bool SWEBY, int MAXN>
-void adv(const MdflArgs* m, const UpdArgs* u, const BatchWork& w, int TJ, cudaStream_t s) {
+void adv(const MdflArgs* m, const BatchWork& w, int TJ, cudaStream_t s) {
   if (w.tz > 0) kb_mdfl_z<SWEBY, MAXN><<<w.tz, 128, 0, s>>>(m, w);
   if (w.tx > 0) kb_mdfl_x<SWEBY, MAXN><<<w.tx, kTX, 0, s>>>(m, w);
   if (w.ty > 0) kb_mdfl_y<SWEBY, MAXN><<<w.ty, 128, 0, s>>>(m, w, TJ);
-  if (w.tu > 0) kb_update<<<w.tu, 128, 0, s>>>(u, w);
 }
 
 }  // namespace
@@ -138,27 +124,25 @@ BatchBlocks batch_blocks(const Geo& g, int TJ, int tile_rows, int seg) {
   BatchBlocks b;
   int nb = (g.ni + 127) / 128;
   b.z = nb * g.nj;
-  b.x = ((g.ni + kTX - 1) / kTX) * g.nj * g.nk;
+  b.x = x_blocks(g) * g.nj * g.nk;
   b.y = nb * ((g.nj + TJ - 1) / TJ) * g.nk;
-  b.u = nb * g.nj * g.nk;
   b.b2 = ((g.ni + 2 + 127) / 128) * (g.nj + 2);
   b.b1 = (int)((g.n2 + 255) / 256);
   b.m = (int)stream_tiles(g, tile_rows) * ((g.nk + seg - 1) / seg);
   return b;
 }
 
-void launch_batch_fp64_advection(const MdflArgs* m, const UpdArgs* u, const BatchWork& w, int ntr, bool sweby, int TJ,
-                                 cudaStream_t s) {
+void launch_batch_fp64_advection(const MdflArgs* m, const BatchWork& w, int ntr, bool sweby, int TJ, cudaStream_t s) {
   if (sweby) {
-    if (ntr <= 1) adv<true, 1>(m, u, w, TJ, s);
-    else if (ntr <= 2) adv<true, 2>(m, u, w, TJ, s);
-    else if (ntr <= 4) adv<true, 4>(m, u, w, TJ, s);
-    else adv<true, kMdflChunk>(m, u, w, TJ, s);
+    if (ntr <= 1) adv<true, 1>(m, w, TJ, s);
+    else if (ntr <= 2) adv<true, 2>(m, w, TJ, s);
+    else if (ntr <= 4) adv<true, 4>(m, w, TJ, s);
+    else adv<true, kMdflChunk>(m, w, TJ, s);
   } else {
-    if (ntr <= 1) adv<false, 1>(m, u, w, TJ, s);
-    else if (ntr <= 2) adv<false, 2>(m, u, w, TJ, s);
-    else if (ntr <= 4) adv<false, 4>(m, u, w, TJ, s);
-    else adv<false, kMdflChunk>(m, u, w, TJ, s);
+    if (ntr <= 1) adv<false, 1>(m, w, TJ, s);
+    else if (ntr <= 2) adv<false, 2>(m, w, TJ, s);
+    else if (ntr <= 4) adv<false, 4>(m, w, TJ, s);
+    else adv<false, kMdflChunk>(m, w, TJ, s);
   }
 }
 

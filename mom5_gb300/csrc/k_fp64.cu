@@ -86,15 +86,35 @@ void launch_zero_ring(const Geo& g, double* a, long nlev, cudaStream_t s) {
 // each face are computed once and reused for every tracer of the launch.
 // ---------------------------------------------------------------------------
 
+// The arguments of tracer n alone, for launches that give each tracer its own blocks.
+DEVI MdflArgs one_tracer(MdflArgs a, int n) {
+  a.ntr = 1;
+  a.T += n * a.tstride;
+  a.tz += n * a.g.n3;
+  a.tx += n * a.g.n3;
+  a.th += n * a.g.n3;
+  if (a.Tp1) a.Tp1 += n * a.tstride;
+  a.hz += (long)n * a.g.nk * a.g.nj * 4;
+  a.hx += (long)n * a.g.nk * a.g.ni * 4;
+  return a;
+}
+
+// The passes are launched as programmatic dependents (launch_pdl).  SPLIT: the
+// levels (z: segments) of tracer n are blocks n*nz .. n*nz + nz - 1 of the grid's z.
 template <bool ALL, bool SWEBY, int MAXN>
 __global__ void __launch_bounds__(128) k_mdfl_z(MdflArgs a) {
+  pdl_wait();
+  pdl_trigger();
   mdfl_z_body<ALL, SWEBY, MAXN>(a, blockIdx.x, blockIdx.y);
 }
 // blockIdx.z: the segment of L levels
-template <bool ALL, bool SWEBY, int MAXN>
+template <bool ALL, bool SWEBY, int MAXN, bool SPLIT>
 __global__ void __launch_bounds__(128) k_mdfl_z_seg(MdflArgs a, int L) {
-  const int k0 = blockIdx.z * L;
-  mdfl_z_body<ALL, SWEBY, MAXN, true>(a, blockIdx.x, blockIdx.y, k0, k0 + L);
+  pdl_wait();
+  pdl_trigger();
+  const int nz = SPLIT ? (a.g.nk + L - 1) / L : gridDim.z;
+  const int k0 = (SPLIT ? blockIdx.z % nz : blockIdx.z) * L;
+  mdfl_z_body<ALL, SWEBY, MAXN, true>(SPLIT ? one_tracer(a, blockIdx.z / nz) : a, blockIdx.x, blockIdx.y, k0, k0 + L);
 }
 
 // Levels per z-pass segment.  A domain with few columns gives the column march
@@ -110,97 +130,86 @@ static int z_segment_levels(const Geo& g) {
   int L = (g.nk + nseg - 1) / nseg;
   return L < 2 ? 2 : L;
 }
-template <bool ALL, bool SWEBY, int MAXN>
-static void launch_mdfl_z(const MdflArgs& a, cudaStream_t s) {
-  const Geo& g = a.g;
-  const int L = z_segment_levels(g);
-  if (L >= g.nk) {
-    k_mdfl_z<ALL, SWEBY, MAXN><<<dim3((g.ni + 127) / 128, g.nj), 128, 0, s>>>(a);
-  } else {
-    dim3 grid((g.ni + 127) / 128, g.nj, (g.nk + L - 1) / L);
-    k_mdfl_z_seg<ALL, SWEBY, MAXN><<<grid, 128, 0, s>>>(a, L);
-  }
-}
-
-template <bool ALL, bool SWEBY, int MAXN>
-__global__ void __launch_bounds__(kTX) k_mdfl_x(MdflArgs a) {
-  mdfl_x_body<ALL, SWEBY, MAXN>(a, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-template <bool ALL, bool SWEBY, int MAXN>
-__global__ void __launch_bounds__(128, 6) k_mdfl_y(MdflArgs a, int TJ) {
-  mdfl_y_body<ALL, SWEBY, MAXN>(a, TJ, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-template <bool ALL, bool SWEBY, int MAXN>
-static void run_mdfl(const MdflArgs& a, cudaStream_t s) {
-  const Geo& g = a.g;
-  launch_mdfl_z<ALL, SWEBY, MAXN>(a, s);
-  dim3 bx((g.ni + kTX - 1) / kTX, g.nj, g.nk);
-  k_mdfl_x<ALL, SWEBY, MAXN><<<bx, kTX, 0, s>>>(a);
-  // rows per thread: keep >= ~8 warps per SM of work where the domain allows
-  long cols = (long)g.ni * g.nk;
+// Rows per thread of the y pass for cols = columns*levels threads and nj rows: each
+// strip forms one face more than it has rows, so as long as the strips give every
+// SM 12 warps, longer ones are cheaper (120x80x30, 2 tracers: 104 us a step with 4
+// rows, 112 with 2, 121 with 8; 37x29x12: 25, 32 and 44 with 2, 4 and 8, 28 with 1).
+int y_strip_rows(long cols, long nj) {
   int TJ = 16;
-  while (TJ > 2 && cols * ((g.nj + TJ - 1) / TJ) < 152L * 32 * 16) TJ /= 2;
-  if (a.tj > 0) TJ = a.tj;
-  dim3 by((g.ni + 127) / 128, (g.nj + TJ - 1) / TJ, g.nk);
-  k_mdfl_y<ALL, SWEBY, MAXN><<<by, 128, 0, s>>>(a, TJ);
+  while (TJ > 2 && cols * ((nj + TJ - 1) / TJ) < 152L * 32 * 12) TJ /= 2;
+  return TJ;
 }
 
-template <bool ALL, bool SWEBY>
-static void run_mdfl_n(const MdflArgs& a, cudaStream_t s) {
-  if (a.ntr <= 1) run_mdfl<ALL, SWEBY, 1>(a, s);
-  else if (a.ntr <= 2) run_mdfl<ALL, SWEBY, 2>(a, s);
-  else if (a.ntr <= 4) run_mdfl<ALL, SWEBY, 4>(a, s);
-  else run_mdfl<ALL, SWEBY, kMdflChunk>(a, s);
+template <bool ALL, bool SWEBY, int MAXN, bool SPLIT>
+__global__ void __launch_bounds__(kTX) k_mdfl_x(MdflArgs a) {
+  pdl_wait();
+  pdl_trigger();
+  const int nk = a.g.nk;
+  mdfl_x_body<ALL, SWEBY, MAXN>(SPLIT ? one_tracer(a, blockIdx.z / nk) : a, blockIdx.x, blockIdx.y,
+                                SPLIT ? blockIdx.z % nk : blockIdx.z);
 }
 
-// one pass (1 z, 2 x, 3 y) of run_mdfl: a decomposed domain exchanges halos between them
-template <bool ALL, bool SWEBY, int MAXN>
-static void run_mdfl_one(const MdflArgs& a, int pass, cudaStream_t s) {
+template <bool ALL, bool SWEBY, int MAXN, bool SPLIT>
+__global__ void __launch_bounds__(128, 6) k_mdfl_y(MdflArgs a, int TJ) {
+  pdl_wait();
+  pdl_trigger();
+  const int nk = a.g.nk;
+  mdfl_y_body<ALL, SWEBY, MAXN>(SPLIT ? one_tracer(a, blockIdx.z / nk) : a, TJ, blockIdx.x, blockIdx.y,
+                                SPLIT ? blockIdx.z % nk : blockIdx.z);
+}
+
+// One pass (1 z, 2 x, 3 y), or all three (0), of every tracer; a decomposed domain
+// exchanges halos between them.
+template <bool ALL, bool SWEBY, int MAXN, bool SPLIT>
+static void run_mdfl(const MdflArgs& a, int pass, cudaStream_t s) {
   const Geo& g = a.g;
-  if (pass == 1) {
-    launch_mdfl_z<ALL, SWEBY, MAXN>(a, s);
-  } else if (pass == 2) {
-    dim3 bx((g.ni + kTX - 1) / kTX, g.nj, g.nk);
-    k_mdfl_x<ALL, SWEBY, MAXN><<<bx, kTX, 0, s>>>(a);
-  } else {
-    long cols = (long)g.ni * g.nk;
-    int TJ = 16;
-    while (TJ > 2 && cols * ((g.nj + TJ - 1) / TJ) < 152L * 32 * 16) TJ /= 2;
-    if (a.tj > 0) TJ = a.tj;
-    dim3 by((g.ni + 127) / 128, (g.nj + TJ - 1) / TJ, g.nk);
-    k_mdfl_y<ALL, SWEBY, MAXN><<<by, 128, 0, s>>>(a, TJ);
+  const unsigned nx = (g.ni + 127) / 128, nt = SPLIT ? a.ntr : 1;
+  // programmatic dependents hide a launch each, which domains of a few blocks per SM feel
+  // (37x29x12, 2 tracers: with SPLIT 24.6 us a step against 43.5); on larger ones the waiting
+  // blocks cost more than that (120x80x30 and 360x270x50: 3%)
+  const bool dep = (long)nx * g.nj * g.nk < 152L * 8;
+  auto launch = [&](auto k, dim3 grid, int threads, auto... args) {
+    if (dep) launch_pdl(k, grid, dim3(threads), s, args...);
+    else k<<<grid, threads, 0, s>>>(args...);
+  };
+  if (pass == 0 || pass == 1) {
+    const int L = z_segment_levels(g);
+    if (L >= g.nk && !SPLIT) launch(k_mdfl_z<ALL, SWEBY, MAXN>, dim3(nx, g.nj), 128, a);
+    else launch(k_mdfl_z_seg<ALL, SWEBY, MAXN, SPLIT>, dim3(nx, g.nj, nt * ((g.nk + L - 1) / L)), 128, a, L);
+  }
+  if (pass == 0 || pass == 2)
+    launch(k_mdfl_x<ALL, SWEBY, MAXN, SPLIT>, dim3(x_blocks(g), g.nj, nt * g.nk), kTX, a);
+  if (pass == 0 || pass == 3) {
+    const int TJ = a.tj > 0 ? a.tj : y_strip_rows((long)g.ni * g.nk, g.nj);
+    launch(k_mdfl_y<ALL, SWEBY, MAXN, SPLIT>, dim3(nx, (g.nj + TJ - 1) / TJ, nt * g.nk), 128, a, TJ);
   }
 }
 
+// Below 16 warps of cells per SM the passes are chains of latency on an idle chip,
+// and the terms a face's tracers share are cheaper formed again: each tracer gets
+// blocks of its own (37x29x12 cells, 2 tracers, with programmatic dependents: 24.6 us a
+// step against 43.5).
 template <bool ALL, bool SWEBY>
-static void run_mdfl_one_n(const MdflArgs& a, int pass, cudaStream_t s) {
-  if (a.ntr <= 1) run_mdfl_one<ALL, SWEBY, 1>(a, pass, s);
-  else if (a.ntr <= 2) run_mdfl_one<ALL, SWEBY, 2>(a, pass, s);
-  else if (a.ntr <= 4) run_mdfl_one<ALL, SWEBY, 4>(a, pass, s);
-  else run_mdfl_one<ALL, SWEBY, kMdflChunk>(a, pass, s);
+static void run_mdfl_n(const MdflArgs& a, int pass, cudaStream_t s) {
+  const Geo& g = a.g;
+  if (a.ntr <= 1) run_mdfl<ALL, SWEBY, 1, false>(a, pass, s);
+  else if ((long)((g.ni + 31) / 32) * g.nj * g.nk < 16L * 152) run_mdfl<ALL, SWEBY, 1, true>(a, pass, s);
+  else if (a.ntr <= 2) run_mdfl<ALL, SWEBY, 2, false>(a, pass, s);
+  else if (a.ntr <= 4) run_mdfl<ALL, SWEBY, 4, false>(a, pass, s);
+  else run_mdfl<ALL, SWEBY, kMdflChunk, false>(a, pass, s);
 }
 
 void run_mdfl_pass(const MdflArgs& a, bool all, bool sweby, int pass, cudaStream_t s) {
   if (all) {
-    if (sweby) run_mdfl_one_n<true, true>(a, pass, s);
-    else run_mdfl_one_n<true, false>(a, pass, s);
+    if (sweby) run_mdfl_n<true, true>(a, pass, s);
+    else run_mdfl_n<true, false>(a, pass, s);
   } else {
-    if (sweby) run_mdfl_one_n<false, true>(a, pass, s);
-    else run_mdfl_one_n<false, false>(a, pass, s);
+    if (sweby) run_mdfl_n<false, true>(a, pass, s);
+    else run_mdfl_n<false, false>(a, pass, s);
   }
 }
 
-void run_mdfl_kernels(const MdflArgs& a, bool all, bool sweby, cudaStream_t s) {
-  if (all) {
-    if (sweby) run_mdfl_n<true, true>(a, s);
-    else run_mdfl_n<true, false>(a, s);
-  } else {
-    if (sweby) run_mdfl_n<false, true>(a, s);
-    else run_mdfl_n<false, false>(a, s);
-  }
-}
+void run_mdfl_kernels(const MdflArgs& a, bool all, bool sweby, cudaStream_t s) { run_mdfl_pass(a, all, sweby, 0, s); }
 
 int ensure_mdfl_scratch(mom5gpu_domain* d, int ntr) {
   if ((int)d->mdfl_cap >= ntr) return MOM5GPU_OK;
@@ -254,8 +263,19 @@ int make_mdfl_args(mom5gpu_domain* d, int n_first, int ntr, int taum1, int tau, 
   return MOM5GPU_OK;
 }
 
-int launch_mdfl(mom5gpu_domain* d, bool all, int n_first, int ntr, int taum1, int tau, double dtime,
-                double sweby_limiter, bool th_fresh) {
+int add_step_args(mom5gpu_domain* d, int n_first, int taum1, int taup1, MdflArgs* a) {
+  a->th_fresh = 1;
+  a->rdz_m1 = fptr(d, MOM5GPU_RHO_DZT, 0, taum1);
+  a->rdzr = fptr(d, MOM5GPU_RHO_DZTR, 0, 0);
+  a->Tp1 = fptr(d, MOM5GPU_TRACER, n_first, taup1);
+  if (!a->rdz_m1 || !a->rdzr || !a->Tp1)
+    return fail(d, MOM5GPU_ESTATE, "update_tracer: a required field was never set");
+  return MOM5GPU_OK;
+}
+
+// taup1 0: the tendency only
+static int launch_mdfl_chunks(mom5gpu_domain* d, bool all, int n_first, int ntr, int taum1, int tau, int taup1,
+                              double dtime, double sweby_limiter) {
   // tracers per launch set: at most kMdflChunk, in chunks of equal size (the
   // tracer-independent face terms are computed once per chunk)
   int nchunks = (ntr + kMdflChunk - 1) / kMdflChunk;
@@ -267,13 +287,22 @@ int launch_mdfl(mom5gpu_domain* d, bool all, int n_first, int ntr, int taum1, in
     int cn = ntr - c0 < csize ? ntr - c0 : csize;
     MdflArgs a;
     rc = make_mdfl_args(d, n_first + c0, cn, taum1, tau, dtime, &a);
+    if (!rc && taup1) rc = add_step_args(d, n_first + c0, taum1, taup1, &a);
     if (rc) return rc;
-    a.th_fresh = th_fresh ? 1 : 0;
     count_launches(d, 3);
     run_mdfl_kernels(a, all, sweby_limiter != 0.0, d->stream);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MOM5GPU_OK : cuda_fail(d, e, "mdfl launch");
+}
+
+int launch_mdfl(mom5gpu_domain* d, bool all, int n_first, int ntr, int taum1, int tau, double dtime,
+                double sweby_limiter) {
+  return launch_mdfl_chunks(d, all, n_first, ntr, taum1, tau, 0, dtime, sweby_limiter);
+}
+
+int launch_mdfl_step(mom5gpu_domain* d, bool all, int taum1, int tau, int taup1, double dtime) {
+  return launch_mdfl_chunks(d, all, 1, d->dims.num_prog_tracers, taum1, tau, taup1, dtime, 1.0);
 }
 
 // ---------------------------------------------------------------------------
