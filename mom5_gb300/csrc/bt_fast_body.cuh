@@ -142,10 +142,10 @@ DEVI double corr_point(const BtArgs& a, int so, int sn, long q, float D) {
   return en;
 }
 
-DEVI void prep_body(const BtArgs& a, int bx, int by) {
+DEVI void prep_body(const BtArgs& a, int bx) {
   const Geo& g = a.g;
-  int i = bx * blockDim.x + threadIdx.x, j = by;
-  if (i > g.ni + 1) return;
+  int i, j;
+  if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j);
   double tmd = a.tmask1[q] * a.datr[q];
   plane(a, KG)[q] = (float)(-a.dtbt_gamma_rho0r * tmd * 0.5);
@@ -176,10 +176,10 @@ DEVI void prep_body(const BtArgs& a, int bx, int by) {
 }
 
 // with reuse, D of level so is the previous corrector's D of the same arrays
-DEVI void pred_body(const BtArgs& a, int so, int sn, int reuse, int bx, int by) {
+DEVI void pred_body(const BtArgs& a, int so, int sn, int reuse, int bx) {
   const Geo& g = a.g;
-  int i0 = bx * blockDim.x + threadIdx.x, j0 = by;
-  if (i0 > g.ni + 1) return;
+  int i0, j0;
+  if (!bt_point(g, bx, i0, j0)) return;
   double en;
   const float ps = pred_point(a, so, reuse, plane(a, DV), i0, j0, en);
   long q0 = I2(g, i0, j0);
@@ -187,10 +187,10 @@ DEVI void pred_body(const BtArgs& a, int so, int sn, int reuse, int bx, int by) 
   plane(a, PS)[q0] = ps;
 }
 
-DEVI void mom_body(const BtArgs& a, int so, int sn, double wgt, int bx, int by) {
+DEVI void mom_body(const BtArgs& a, int so, int sn, double wgt, int bx) {
   const Geo& g = a.g;
-  int i = bx * blockDim.x + threadIdx.x, j = by;
-  if (i > g.ni + 1) return;
+  int i, j;
+  if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j), n2 = g.n2;
   float px = 0.0f, py = 0.0f;
   if (i <= g.ni && j <= g.nj) {
@@ -206,10 +206,10 @@ DEVI void mom_body(const BtArgs& a, int so, int sn, double wgt, int bx, int by) 
   sum_point(a, wgt, q, un, vn);
 }
 
-DEVI void corr_body(const BtArgs& a, int so, int sn, int bx, int by) {
+DEVI void corr_body(const BtArgs& a, int so, int sn, int bx) {
   const Geo& g = a.g;
-  int i = bx * blockDim.x + threadIdx.x, j = by;
-  if (i > g.ni + 1) return;
+  int i, j;
+  if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j), n2 = g.n2;
   float D = div_num(g, a.uhb + sn * n2, a.vhb + sn * n2, i, j);
   plane(a, DV)[q] = D;
@@ -224,10 +224,10 @@ DEVI void corr_body(const BtArgs& a, int so, int sn, int bx, int by) {
 // it is.  The predicted eta is not stored (the next corrector overwrites it
 // unread), nor is the divergence.  Same arithmetic as corr_body then pred_body
 // with reuse, so the same bits.
-DEVI void corr_pred_body(const BtArgs& a, int so, int sn, int bx, int by) {
+DEVI void corr_pred_body(const BtArgs& a, int so, int sn, int bx) {
   const Geo& g = a.g;
-  int i = bx * blockDim.x + threadIdx.x, j = by;
-  if (i > g.ni + 1) return;
+  int i, j;
+  if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j), n2 = g.n2;
   const float D = div_num(g, a.uhb + sn * n2, a.vhb + sn * n2, i, j);
   double en = corr_point(a, so, sn, q, D);

@@ -490,6 +490,15 @@ DEVI void mdfl_y_body(MdflArgs a, int TJ, int bx, int by, int bz) {
 
 
 
+// Products of the exact B-grid subcycle: with INT those by dtbt, cori1, cori2, the
+// transports' lengths, datr, dtbt/rho0 and the time weight run on the integer pipe
+// (mul_int), 10 of 20 beside 28 sums (1440x1080, 60 subcycles: 9.8 -> 8.2 ms; with
+// all 20, 8.9); bt_int_products says where.
+template <bool INT, bool ZA = false>
+DEVI double bt_mul(double a, double b) {
+  if constexpr (INT) return mul_int<ZA, true>(a, b);
+  return a * b;
+}
 // DIV_UD at (i,j) (ocean_operators.F90:507-608), halo_in = halo_out = 1.
 DEVI double div_ud(const BtArgs& a, const double* u, const double* v, int i, int j) {
   const Geo& g = a.g;
@@ -518,6 +527,7 @@ DEVI double div_ud(const BtArgs& a, const double* u, const double* v, int i, int
 
 // B-grid DIV_UD from the stored products uh = u*dyu, vh = v*dxu: the same
 // operations as div_ud on the same values, without recomputing the products.
+template <bool INT = false>
 DEVI double div_ud_bh(const BtArgs& a, const double* uh, const double* vh, int i, int j) {
   const Geo& g = a.g;
   if (i < 1 || j < 1) return 0.0;
@@ -526,7 +536,7 @@ DEVI double div_ud_bh(const BtArgs& a, const double* uh, const double* vh, int i
   double vh_bax = half_exact(vh[q] + vh[qw]);
   double uhim_bay = half_exact(uh[qw] + uh[qsw]);
   double vhjm_bax = half_exact(vh[qs] + vh[qsw]);
-  return ((uh_bay - uhim_bay) + (vh_bax - vhjm_bax)) * a.datr[q];
+  return bt_mul<INT>(a.datr[q], (uh_bay - uhim_bay) + (vh_bax - vhjm_bax));
 }
 
 // image of a halo point under the single-PE full halo update; returns false
@@ -568,39 +578,46 @@ DEVI void bt_init_body(BtArgs a, const double* eta_bar_tau, const double* eta_ta
   a.steady[q] = a.tmask1[q] * (pme[q] + river[q] + source[q] - eta_smooth[q]);
 }
 
+// 0.25*x: the exponent lowered by two where that stays normal; +-0 is unchanged.
+DEVI double quarter_exact(double x) {
+  const long long b = bits_of(x);
+  const unsigned e = (unsigned)((unsigned long long)b >> 52) & 0x7ffu;
+  const bool normal = e - 3u < 0x7fcu;  // 3 <= e <= 0x7fe
+  double r = double_of(normal ? b - (2LL << 52) : b);
+  rare_lanes(!(normal || (b << 1) == 0), [&] { r = 0.25 * x; });
+  return r;
+}
+// C grid: the Coriolis acceleration of the transports u, v at (i, j) (:3707-3715)
+template <bool INT>
+DEVI void bt_coriolis_c(const BtArgs& a, const double* u, const double* v, int i, int j, double& c0, double& c1) {
+  const Geo& g = a.g;
+  const long q = I2(g, i, j), s = q - g.nxd, w = q - 1;
+  c0 = quarter_exact(bt_mul<INT>(a.f[q], v[q] + v[q + 1]) + bt_mul<INT>(a.f[s], v[s] + v[s + 1]));
+  c1 = neg_if(quarter_exact(bt_mul<INT>(a.f[q], u[q] + u[q + g.nxd]) + bt_mul<INT>(a.f[w], u[w] + u[w + g.nxd])), true);
+}
+
 // C-grid: initial Adams-Bashforth Coriolis history (:3707-3730)
 DEVI void bt_cgrid_init_body(BtArgs a, int bx, int by) {
   const Geo& g = a.g;
   int i = bx * blockDim.x + threadIdx.x + 1;
   int j = by + 1;
   if (i > g.ni) return;
-  const double abm0 = 23.0 / 12.0, abm1 = -16.0 / 12.0, abm2 = 5.0 / 12.0;
-  const int itime = 1;
-  int m2 = (itime + 0) % 3, m1 = (itime + 1) % 3, m0 = (itime + 2) % 3;
-  const double* u = a.ubt + g.n2;
-  const double* v = a.vbt + g.n2;
-  long n2 = g.n2;
-  long q = I2(g, i, j);
-  double c0 = 0.25 * (a.f[q] * (v[q] + v[I2(g, i + 1, j)]) + a.f[I2(g, i, j - 1)] * (v[I2(g, i, j - 1)] + v[I2(g, i + 1, j - 1)]));
-  a.cf[(m0 * 2 + 0) * n2 + q] = c0;
-  a.cf[(m1 * 2 + 0) * n2 + q] = c0;
-  a.cf[(m2 * 2 + 0) * n2 + q] = c0;
-  a.ca[q] = abm0 * c0 + abm1 * c0 + abm2 * c0;
-  double c1 = -0.25 * (a.f[q] * (u[q] + u[I2(g, i, j + 1)]) + a.f[I2(g, i - 1, j)] * (u[I2(g, i - 1, j)] + u[I2(g, i - 1, j + 1)]));
-  a.cf[(m0 * 2 + 1) * n2 + q] = c1;
-  a.cf[(m1 * 2 + 1) * n2 + q] = c1;
-  a.cf[(m2 * 2 + 1) * n2 + q] = c1;
-  a.ca[n2 + q] = abm0 * c1 + abm1 * c1 + abm2 * c1;
+  const long n2 = g.n2, q = I2(g, i, j);
+  double c0, c1;
+  bt_coriolis_c<false>(a, a.ubt + n2, a.vbt + n2, i, j, c0, c1);
+  for (int m = 0; m < 3; ++m) {
+    a.cf[(m * 2 + 0) * n2 + q] = c0;
+    a.cf[(m * 2 + 1) * n2 + q] = c1;
+  }
 }
 
 // predictor + ps (both grids).  With reuse the divergence of the transports at
 // level so is the one the previous subcycle's corrector formed from the same
 // arrays (its level sn), stored in dvs: the same values, read instead of formed.
-DEVI void bt_pred_body(BtArgs a, int so, int sn, int reuse, int bx, int by) {
+DEVI void bt_pred_body(BtArgs a, int so, int sn, int reuse, int bx) {
   const Geo& g = a.g;
-  int i0 = bx * blockDim.x + threadIdx.x;
-  int j0 = by;
-  if (i0 > g.ni + 1) return;
+  int i0, j0;
+  if (!bt_point(g, bx, i0, j0)) return;
   int i = i0, j = j0;
   // B-grid legacy halos: eta(fstaup1) is halo-updated right after the predictor,
   // so a halo point takes the value computed at its periodic image.
@@ -629,11 +646,11 @@ DEVI void bt_pred_body(BtArgs a, int so, int sn, int reuse, int bx, int by) {
 }
 
 // momentum update, B grid (:3466-3485)
-DEVI void bt_mom_b_body(BtArgs a, int so, int sn, int bx, int by) {
+template <bool INT = false>
+DEVI void bt_mom_b_body(BtArgs a, int so, int sn, int bx) {
   const Geo& g = a.g;
-  int i = bx * blockDim.x + threadIdx.x;
-  int j = by;
-  if (i > g.ni + 1) return;
+  int i, j;
+  if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j);
   double gx = 0.0, gy = 0.0;
   if (i <= g.ni && j <= g.nj) {
@@ -653,55 +670,95 @@ DEVI void bt_mom_b_body(BtArgs a, int so, int sn, int bx, int by) {
   double pf2 = -a.thicku[q] * gy;
   double uo = a.ubt[so * g.n2 + q], vo = a.vbt[so * g.n2 + q];
   double hf = half_exact(a.f[q]);  // 0.5*f; -0.5*f is its negation
-  double t1 = uo + a.dtbt * plus_zero(hf * vo + pf1 + a.forcing_u[q]);
-  double t2 = vo + a.dtbt * plus_zero((-hf) * uo + pf2 + a.forcing_v[q]);
-  double un = a.cori2[q] * (t1 + a.cori1[q] * t2);
-  double vn = a.cori2[q] * (t2 - a.cori1[q] * t1);
+  double t1 = uo + bt_mul<INT>(a.dtbt, plus_zero(hf * vo + pf1 + a.forcing_u[q]));
+  double t2 = vo + bt_mul<INT>(a.dtbt, plus_zero((-hf) * uo + pf2 + a.forcing_v[q]));
+  double un = bt_mul<INT>(a.cori2[q], t1 + bt_mul<INT>(a.cori1[q], t2));
+  double vn = bt_mul<INT>(a.cori2[q], t2 - bt_mul<INT>(a.cori1[q], t1));
   a.ubt[sn * g.n2 + q] = un;
   a.vbt[sn * g.n2 + q] = vn;
-  a.uhb[sn * g.n2 + q] = un * a.dyu[q];
-  a.vhb[sn * g.n2 + q] = vn * a.dxu[q];
+  a.uhb[sn * g.n2 + q] = bt_mul<INT>(a.dyu[q], un);
+  a.vhb[sn * g.n2 + q] = bt_mul<INT>(a.dxu[q], vn);
 }
 
-// C grid: Coriolis (compute domain) + gradient + momentum (:3780-3830)
-DEVI void bt_mom_c_body(BtArgs a, int so, int sn, int itime, int bx, int by) {
+// C grid: Coriolis (compute domain) + gradient + momentum (:3780-3830), and the
+// halo update of the transports: the thread of a halo point with a periodic image
+// forms the image's value.  The transports times their areas over their lengths,
+// which the divergence takes (ocean_operators.F90:507-608), are stored beside them.
+template <bool INT>
+DEVI void bt_mom_c_body(BtArgs a, int so, int sn, int itime, int bx) {
   const Geo& g = a.g;
-  int i = bx * blockDim.x + threadIdx.x;
-  int j = by;
-  if (i > g.ni + 1) return;
-  long n2 = g.n2;
-  long q = I2(g, i, j);
+  int i0, j0;
+  if (!bt_point(g, bx, i0, j0)) return;
+  int i = i0, j = j0;
+  if (!halo_image(g, i, j)) {
+    i = i0;
+    j = j0;
+  }
+  const long n2 = g.n2, q0 = I2(g, i0, j0), q = I2(g, i, j);
   const double abm0 = 23.0 / 12.0, abm1 = -16.0 / 12.0, abm2 = 5.0 / 12.0;
-  int m2 = (itime + 0) % 3, m1 = (itime + 1) % 3, m0 = (itime + 2) % 3;
+  const int m2 = (itime + 0) % 3, m1 = (itime + 1) % 3, m0 = (itime + 2) % 3;
   double ca0 = 0.0, ca1 = 0.0;
   if (i >= 1 && i <= g.ni && j >= 1 && j <= g.nj) {
-    const double* u = a.ubt + so * n2;
-    const double* v = a.vbt + so * n2;
-    double c0 = 0.25 * (a.f[q] * (v[q] + v[I2(g, i + 1, j)]) + a.f[I2(g, i, j - 1)] * (v[I2(g, i, j - 1)] + v[I2(g, i + 1, j - 1)]));
-    a.cf[(m0 * 2 + 0) * n2 + q] = c0;
-    ca0 = abm0 * c0 + abm1 * a.cf[(m1 * 2 + 0) * n2 + q] + abm2 * a.cf[(m2 * 2 + 0) * n2 + q];
-    double c1 = -0.25 * (a.f[q] * (u[q] + u[I2(g, i, j + 1)]) + a.f[I2(g, i - 1, j)] * (u[I2(g, i - 1, j)] + u[I2(g, i - 1, j + 1)]));
-    a.cf[(m0 * 2 + 1) * n2 + q] = c1;
-    ca1 = abm0 * c1 + abm1 * a.cf[(m1 * 2 + 1) * n2 + q] + abm2 * a.cf[(m2 * 2 + 1) * n2 + q];
+    double c0, c1;
+    bt_coriolis_c<INT>(a, a.ubt + so * n2, a.vbt + so * n2, i, j, c0, c1);
+    if (q == q0) {
+      a.cf[(m0 * 2 + 0) * n2 + q] = c0;
+      a.cf[(m0 * 2 + 1) * n2 + q] = c1;
+    }
+    ca0 = bt_mul<INT>(abm0, c0) + bt_mul<INT>(abm1, a.cf[(m1 * 2 + 0) * n2 + q]) + abm2 * a.cf[(m2 * 2 + 0) * n2 + q];
+    ca1 = bt_mul<INT>(abm0, c1) + bt_mul<INT>(abm1, a.cf[(m1 * 2 + 1) * n2 + q]) + abm2 * a.cf[(m2 * 2 + 1) * n2 + q];
   }
+  const double te = a.tmen_e[q], tn = a.tmen_n[q];
   double gx = 0.0, gy = 0.0;
   if (i <= g.ni && j <= g.nj) {
-    gx = (a.ps[I2(g, i + 1, j)] - a.ps[q]) * a.dxter[q] * a.tmen_e[q];
-    gy = (a.ps[I2(g, i, j + 1)] - a.ps[q]) * a.dytnr[q] * a.tmen_n[q];
+    const double p = a.ps[q];
+    gx = is_zero(te) ? 0.0 : mask_mul((a.ps[q + 1] - p) * a.dxter[q], te);
+    gy = is_zero(tn) ? 0.0 : mask_mul((a.ps[q + g.nxd] - p) * a.dytnr[q], tn);
   }
-  double pf1 = -a.thicken_e[q] * gx;
-  double pf2 = -a.thicken_n[q] * gy;
-  double uo = a.ubt[so * n2 + q], vo = a.vbt[so * n2 + q];
-  a.ubt[sn * n2 + q] = uo + a.dtbt * a.tmen_e[q] * (ca0 + pf1 + a.forcing_u[q] + 0.0);
-  a.vbt[sn * n2 + q] = vo + a.dtbt * a.tmen_n[q] * (ca1 + pf2 + a.forcing_v[q] + 0.0);
+  const double pf1 = bt_mul<INT, true>(-a.thicken_e[q], gx);
+  const double pf2 = bt_mul<INT, true>(-a.thicken_n[q], gy);
+  // dtbt*tmasken*(...): nothing is added where the mask is zero
+  const double su = ca0 + pf1 + a.forcing_u[q], sv = ca1 + pf2 + a.forcing_v[q];
+  double du = bt_mul<INT>(a.dtbt, su), dv = bt_mul<INT>(a.dtbt, sv);
+  rare_lanes(!(is_one(te) || is_zero(te)), [&] { du = a.dtbt * te * su; });
+  rare_lanes(!(is_one(tn) || is_zero(tn)), [&] { dv = a.dtbt * tn * sv; });
+  const double un = a.ubt[so * n2 + q] + (is_zero(te) ? 0.0 : du);
+  const double vn = a.vbt[so * n2 + q] + (is_zero(tn) ? 0.0 : dv);
+  a.ubt[sn * n2 + q0] = un;
+  a.vbt[sn * n2 + q0] = vn;
+  a.ca[q0] = bt_mul<INT>(un, a.dat[q0]) * a.dxter[q0];
+  a.ca[n2 + q0] = bt_mul<INT>(vn, a.dat[q0]) * a.dytnr[q0];
+}
+
+// C grid: the corrector of subcycle t and the predictor of subcycle t+1, which
+// reads only its own point's corrected eta and divergence (bt_corr_body's and
+// bt_pred_body's operations).
+template <bool INT>
+DEVI void bt_corr_pred_c_body(BtArgs a, int so, int sn, double wgt, int bx) {
+  const Geo& g = a.g;
+  int i, j;
+  if (!bt_point(g, bx, i, j)) return;
+  const long n2 = g.n2, q = I2(g, i, j);
+  double dv = 0.0;
+  if (i >= 1 && j >= 1)
+    dv = bt_mul<INT>(a.datr[q], (a.ca[q] - a.ca[q - 1]) + (a.ca[n2 + q] - a.ca[n2 + q - g.nxd]));
+  const double tm = a.tmask1[q];
+  const double st = (is_zero(tm) ? 0.0 : mask_mul(-dv, tm)) + a.steady[q];
+  const double en = a.eta_bt[so * n2 + q] + bt_mul<INT>(a.dtbt_rho0r, st);
+  a.eta_bt[sn * n2 + q] = en;
+  a.eta_bar[q] = a.eta_bar[q] + en;
+  const double un = a.ubt[sn * n2 + q], vn = a.vbt[sn * n2 + q];
+  a.udrho_u[q] = a.udrho_u[q] + (a.stepB ? bt_mul<INT>(wgt, un) : un);
+  a.udrho_v[q] = a.udrho_v[q] + (a.stepB ? bt_mul<INT>(wgt, vn) : vn);
+  const double ep = dpos(a.gamma) ? en + a.dtbt_gamma_rho0r * st : en;
+  a.ps[q] = a.rho_g[q] * ep + a.patm[q];
 }
 
 // corrector + accumulation
-DEVI void bt_corr_body(BtArgs a, int so, int sn, double wgt, int bx, int by) {
+DEVI void bt_corr_body(BtArgs a, int so, int sn, double wgt, int bx) {
   const Geo& g = a.g;
-  int i = bx * blockDim.x + threadIdx.x;
-  int j = by;
-  if (i > g.ni + 1) return;
+  int i, j;
+  if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j);
   double dv = a.cgrid ? div_ud(a, a.ubt + sn * g.n2, a.vbt + sn * g.n2, i, j)
                       : div_ud_bh(a, a.uhb + sn * g.n2, a.vhb + sn * g.n2, i, j);
@@ -729,24 +786,24 @@ DEVI void bt_corr_body(BtArgs a, int so, int sn, double wgt, int bx, int by) {
 // at the periodic halo points whose image it is.  The predicted eta is not
 // stored (the next corrector overwrites it unread), nor is the divergence.  The
 // operations are bt_corr_body's and bt_pred_body's, so the bits are theirs.
-DEVI void bt_corr_pred_body(BtArgs a, int so, int sn, double wgt, int bx, int by) {
+template <bool INT = false>
+DEVI void bt_corr_pred_body(BtArgs a, int so, int sn, double wgt, int bx) {
   const Geo& g = a.g;
-  int i = bx * blockDim.x + threadIdx.x;
-  int j = by;
-  if (i > g.ni + 1) return;
+  int i, j;
+  if (!bt_point(g, bx, i, j)) return;
   const long n2 = g.n2;
   long q = I2(g, i, j);
-  double dv = div_ud_bh(a, a.uhb + sn * n2, a.vhb + sn * n2, i, j);
+  double dv = div_ud_bh<INT>(a, a.uhb + sn * n2, a.vhb + sn * n2, i, j);
   double tm = a.tmask1[q];
   double tmp = is_zero(tm) ? 0.0 : mask_mul(-dv, tm);
   const double st = tmp + a.steady[q];
-  double en = a.eta_bt[so * n2 + q] + a.dtbt_rho0r * st;
+  double en = a.eta_bt[so * n2 + q] + bt_mul<INT>(a.dtbt_rho0r, st);
   a.eta_bt[sn * n2 + q] = en;
   a.eta_bar[q] = a.eta_bar[q] + en;
   double un = a.ubt[sn * n2 + q], vn = a.vbt[sn * n2 + q];
   if (a.stepB) {
-    a.udrho_u[q] = a.udrho_u[q] + wgt * un;
-    a.udrho_v[q] = a.udrho_v[q] + wgt * vn;
+    a.udrho_u[q] = a.udrho_u[q] + bt_mul<INT>(wgt, un);
+    a.udrho_v[q] = a.udrho_v[q] + bt_mul<INT>(wgt, vn);
   } else {
     a.udrho_u[q] = a.udrho_u[q] + un;
     a.udrho_v[q] = a.udrho_v[q] + vn;
@@ -901,11 +958,10 @@ DEVI void bt_fused_body(BtArgs a, int so, int sn, int reuse, double wgt, int bx,
   }
 }
 
-DEVI void bt_post2_body(BtArgs a, double* conv, double* eta_u, double* ps_out, int bx, int by) {
+DEVI void bt_post2_body(BtArgs a, double* conv, double* eta_u, double* ps_out, int bx) {
   const Geo& g = a.g;
-  int i = bx * blockDim.x + threadIdx.x;
-  int j = by;
-  if (i > g.ni + 1) return;
+  int i, j;
+  if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j);
   conv[q] = -div_ud(a, a.udrho_u, a.udrho_v, i, j);
   double r = 0.0;
@@ -920,11 +976,10 @@ DEVI void bt_post2_body(BtArgs a, double* conv, double* eta_u, double* ps_out, i
   ps_out[q] = a.rho_g[q] * a.eta_bar[q] + a.patm[q];
 }
 
-DEVI void bt_post3_body(BtArgs a, const double* ps, double* gxo, double* gyo, int bx, int by) {
+DEVI void bt_post3_body(BtArgs a, const double* ps, double* gxo, double* gyo, int bx) {
   const Geo& g = a.g;
-  int i = bx * blockDim.x + threadIdx.x;
-  int j = by;
-  if (i > g.ni + 1) return;
+  int i, j;
+  if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j);
   double gx = 0.0, gy = 0.0;
   if (i <= g.ni && j <= g.nj) {

@@ -274,6 +274,17 @@ int launch_eta_update(mom5gpu_domain* d, int taum1, int taup1, double dtime);
 // kernel still reads only completed results.  Launched the ordinary way, the
 // two instructions do nothing.
 #ifdef __CUDACC__
+// The data-domain point of this thread in a 2-D barotropic launch, its rows laid end
+// to end: with blocks of one row each the last of a row is part empty, and the SMs
+// that get more of the full ones set the time (270x200 columns, 80 subcycles: 1.18 ->
+// 0.81 ms; 300x260: 1.40 -> 0.99).
+__device__ __forceinline__ bool bt_point(const Geo& g, int block, int& i, int& j) {
+  const unsigned q = (unsigned)block * blockDim.x + threadIdx.x;
+  if (q >= (unsigned)g.n2) return false;
+  j = (int)(q / (unsigned)g.nxd);
+  i = (int)(q - (unsigned)j * (unsigned)g.nxd);
+  return true;
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
@@ -292,6 +303,16 @@ cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, A
   return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// Whether a launch over so many columns takes the subcycle's products on the integer
+// pipe (bt_mul).  On the FP64 pipe and on the integer pipe, 80 subcycles: 120x100
+// columns 0.65 and 0.74 ms, 300x260 0.99 and 1.14, 360x300 1.23 and 1.10; C grid, 48
+// subcycles, 361x243 0.68 and 0.60; 60 subcycles, 1440x1080 9.81 and 8.17.
+inline bool bt_int_products(long columns) { return columns >= 85000; }
+// Threads and blocks of a 2-D barotropic launch of one domain: small blocks while
+// they fit the SMs in one round (360x300: 1.10 ms with 64 threads, 1.12 with 128, 1.34
+// with 32, of which an SM holds too few).
+inline int bt_threads(const Geo& g) { return g.n2 < 152L * 2048 ? 64 : 128; }
+inline dim3 bt_grid(const Geo& g, int threads) { return dim3((unsigned)((g.n2 + threads - 1) / threads)); }
 // precision-form barotropic subcycle (k_mixed.cu, k_batch.cu)
 void launch_btf_prep(const BtArgs& a, cudaStream_t s);
 int launch_btf_subcycle(const BtArgs& a, int itime, int nts, bool fused, cudaStream_t s);

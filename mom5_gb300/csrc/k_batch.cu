@@ -20,37 +20,35 @@ DEVI int find_entry_m(const int* prefix, int count, int b) {
 #define BTF_ENTRY                                    \
   int e = find_entry_m(w.pb2, w.count, blockIdx.x);  \
   const BtArgs& a = d[w.entries[e]];                 \
-  int local = blockIdx.x - w.pb2[e];                 \
-  int nb = (a.g.ni + 2 + 127) / 128;                 \
-  int bx = local % nb, by = local / nb;
+  const int bx = blockIdx.x - w.pb2[e];
 
 __global__ void __launch_bounds__(128) kb_btf_prep(const BtArgs* d, BatchWork w) {
   BTF_ENTRY
-  btfast::prep_body(a, bx, by);
+  btfast::prep_body(a, bx);
 }
 __global__ void __launch_bounds__(128) kb_btf_pred(const BtArgs* d, BatchWork w, int so, int sn, int reuse) {
   pdl_wait();
   pdl_trigger();
   BTF_ENTRY
-  btfast::pred_body(a, so, sn, reuse, bx, by);
+  btfast::pred_body(a, so, sn, reuse, bx);
 }
 __global__ void __launch_bounds__(128) kb_btf_mom(const BtArgs* d, BatchWork w, int so, int sn, double wgt) {
   pdl_wait();
   pdl_trigger();
   BTF_ENTRY
-  btfast::mom_body(a, so, sn, wgt, bx, by);
+  btfast::mom_body(a, so, sn, wgt, bx);
 }
 __global__ void __launch_bounds__(128) kb_btf_corr(const BtArgs* d, BatchWork w, int so, int sn) {
   pdl_wait();
   pdl_trigger();
   BTF_ENTRY
-  btfast::corr_body(a, so, sn, bx, by);
+  btfast::corr_body(a, so, sn, bx);
 }
 __global__ void __launch_bounds__(128) kb_btf_corr_pred(const BtArgs* d, BatchWork w, int so, int sn) {
   pdl_wait();
   pdl_trigger();
   BTF_ENTRY
-  btfast::corr_pred_body(a, so, sn, bx, by);
+  btfast::corr_pred_body(a, so, sn, bx);
 }
 
 }  // namespace

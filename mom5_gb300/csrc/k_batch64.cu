@@ -63,33 +63,33 @@ __global__ void __launch_bounds__(256) kb_bt_init(const BtArgs* d, const BtExtra
 #define BT2D_ENTRY                                   \
   int e = find_entry(w.pb2, w.count, blockIdx.x);    \
   const BtArgs& a = d[w.entries[e]];                 \
-  int local = blockIdx.x - w.pb2[e];                 \
-  int nb = (a.g.ni + 2 + 127) / 128;                 \
-  int bx = local % nb, by = local / nb;
+  const int bx = blockIdx.x - w.pb2[e];
 
 __global__ void __launch_bounds__(128) kb_bt_pred(const BtArgs* d, BatchWork w, int so, int sn, int reuse) {
   pdl_wait();
   pdl_trigger();
   BT2D_ENTRY
-  bt_pred_body(a, so, sn, reuse, bx, by);
+  bt_pred_body(a, so, sn, reuse, bx);
 }
+template <bool INT>
 __global__ void __launch_bounds__(128) kb_bt_mom_b(const BtArgs* d, BatchWork w, int so, int sn) {
   pdl_wait();
   pdl_trigger();
   BT2D_ENTRY
-  bt_mom_b_body(a, so, sn, bx, by);
+  bt_mom_b_body<INT>(a, so, sn, bx);
 }
 __global__ void __launch_bounds__(128) kb_bt_corr(const BtArgs* d, BatchWork w, int so, int sn, double wgt) {
   pdl_wait();
   pdl_trigger();
   BT2D_ENTRY
-  bt_corr_body(a, so, sn, wgt, bx, by);
+  bt_corr_body(a, so, sn, wgt, bx);
 }
+template <bool INT>
 __global__ void __launch_bounds__(128) kb_bt_corr_pred(const BtArgs* d, BatchWork w, int so, int sn, double wgt) {
   pdl_wait();
   pdl_trigger();
   BT2D_ENTRY
-  bt_corr_pred_body(a, so, sn, wgt, bx, by);
+  bt_corr_pred_body<INT>(a, so, sn, wgt, bx);
 }
 __global__ void __launch_bounds__(256) kb_bt_post1(const BtArgs* d, BatchWork w, double rntsp1, double rnts) {
   int e = find_entry(w.pb1, w.count, blockIdx.x);
@@ -103,12 +103,12 @@ __global__ void __launch_bounds__(256) kb_bt_post1(const BtArgs* d, BatchWork w,
 __global__ void __launch_bounds__(128) kb_bt_post2(const BtArgs* d, const BtExtra* xs, BatchWork w) {
   BT2D_ENTRY
   const BtExtra& x = xs[w.entries[e]];
-  bt_post2_body(a, x.conv, x.eta_u, x.ps_out, bx, by);
+  bt_post2_body(a, x.conv, x.eta_u, x.ps_out, bx);
 }
 __global__ void __launch_bounds__(128) kb_bt_post3(const BtArgs* d, const BtExtra* xs, BatchWork w) {
   BT2D_ENTRY
   const BtExtra& x = xs[w.entries[e]];
-  bt_post3_body(a, x.ps_out, x.gxo, x.gyo, bx, by);
+  bt_post3_body(a, x.ps_out, x.gxo, x.gyo, bx);
 }
 
 template <bool SWEBY, int MAXN>
@@ -126,7 +126,7 @@ BatchBlocks batch_blocks(const Geo& g, int TJ, int tile_rows, int seg) {
   b.z = nb * g.nj;
   b.x = x_blocks(g) * g.nj * g.nk;
   b.y = nb * ((g.nj + TJ - 1) / TJ) * g.nk;
-  b.b2 = ((g.ni + 2 + 127) / 128) * (g.nj + 2);
+  b.b2 = (int)((g.n2 + 127) / 128);
   b.b1 = (int)((g.n2 + 255) / 256);
   b.m = (int)stream_tiles(g, tile_rows) * ((g.nk + seg - 1) / seg);
   return b;
@@ -161,8 +161,9 @@ void launch_batch_barotropic_loop(const BtArgs* bt, const BtExtra* x, const Batc
     const dim3 g2(w.tb2), b(128);
     const double wgt = (double)(nts - itime + 1);
     if (itime == 1) launch_pdl(kb_bt_pred, g2, b, s, bt, w, so, sn, 0);
-    launch_pdl(kb_bt_mom_b, g2, b, s, bt, w, so, sn);
-    if (itime < nts) launch_pdl(kb_bt_corr_pred, g2, b, s, bt, w, so, sn, wgt);
+    const bool bint = bt_int_products(128L * w.tb2);
+    launch_pdl(bint ? kb_bt_mom_b<true> : kb_bt_mom_b<false>, g2, b, s, bt, w, so, sn);
+    if (itime < nts) launch_pdl(bint ? kb_bt_corr_pred<true> : kb_bt_corr_pred<false>, g2, b, s, bt, w, so, sn, wgt);
     else launch_pdl(kb_bt_corr, g2, b, s, bt, w, so, sn, wgt);
   }
   (void)stepB;

@@ -1321,23 +1321,36 @@ __global__ void k_bt_cgrid_init(BtArgs a) { bt_cgrid_init_body(a, blockIdx.x, bl
 __global__ void k_bt_pred(BtArgs a, int so, int sn, int reuse) {
   pdl_wait();
   pdl_trigger();
-  bt_pred_body(a, so, sn, reuse, blockIdx.x, blockIdx.y);
+  bt_pred_body(a, so, sn, reuse, blockIdx.x);
 }
+template <bool INT>
 __global__ void k_bt_mom_b(BtArgs a, int so, int sn) {
   pdl_wait();
   pdl_trigger();
-  bt_mom_b_body(a, so, sn, blockIdx.x, blockIdx.y);
+  bt_mom_b_body<INT>(a, so, sn, blockIdx.x);
 }
-__global__ void k_bt_mom_c(BtArgs a, int so, int sn, int itime) { bt_mom_c_body(a, so, sn, itime, blockIdx.x, blockIdx.y); }
+template <bool INT>
+__global__ void k_bt_mom_c(BtArgs a, int so, int sn, int itime) {
+  pdl_wait();
+  pdl_trigger();
+  bt_mom_c_body<INT>(a, so, sn, itime, blockIdx.x);
+}
+template <bool INT>
+__global__ void k_bt_corr_pred_c(BtArgs a, int so, int sn, double wgt) {
+  pdl_wait();
+  pdl_trigger();
+  bt_corr_pred_c_body<INT>(a, so, sn, wgt, blockIdx.x);
+}
 __global__ void k_bt_corr(BtArgs a, int so, int sn, double wgt) {
   pdl_wait();
   pdl_trigger();
-  bt_corr_body(a, so, sn, wgt, blockIdx.x, blockIdx.y);
+  bt_corr_body(a, so, sn, wgt, blockIdx.x);
 }
+template <bool INT>
 __global__ void k_bt_corr_pred(BtArgs a, int so, int sn, double wgt) {
   pdl_wait();
   pdl_trigger();
-  bt_corr_pred_body(a, so, sn, wgt, blockIdx.x, blockIdx.y);
+  bt_corr_pred_body<INT>(a, so, sn, wgt, blockIdx.x);
 }
 // 32 x 8 tiles of 352 threads: one point per thread in each phase (the 34 x 10
 // pressure ring is the largest); 64 x 8 tiles of 256 threads, several points
@@ -1352,8 +1365,7 @@ __global__ void __launch_bounds__(kFusedThreads) k_bt_fused(BtArgs a, int so, in
 //
 // A persistent grid of 128-thread blocks, all resident (cooperative launch),
 // walks the blocks of the predictor, momentum and corrector launches (virtual
-// block vb = bx + nbx*by of their (ni+2)/128 x (nj+2) grid) with the same
-// bodies, and a grid barrier stands where a launch boundary stood, so the
+// block vb) with the same bodies, and a grid barrier stands where a launch boundary stood, so the
 // results are those of the three launches bit for bit.  A barrier is an
 // arrival counter: thread 0 of each block publishes the block's writes (fence),
 // adds one and waits until the counter reaches the barrier's target.  The wait
@@ -1402,17 +1414,17 @@ DEVI bool grid_barrier(unsigned* ctr, unsigned target, int* err, long long limit
 
 __global__ void __launch_bounds__(128) k_bt_coop(BtArgs a, unsigned* ctr, int* err) {
   const Geo& g = a.g;
-  const int nbx = (g.ni + 2 + 127) / 128, nvb = nbx * (g.nj + 2);
+  const int nvb = (int)((g.n2 + 127) / 128);
   const unsigned per = gridDim.x;
   unsigned target = 0;
   for (int itime = 1; itime <= a.nts; ++itime) {
     const int so = itime % 2, sn = (itime + 1) % 2;
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) bt_pred_body(a, so, sn, itime > 1, vb % nbx, vb / nbx);
+    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) bt_pred_body(a, so, sn, itime > 1, vb);
     if (!grid_barrier(ctr, target += per, err, kGridWaitCycles)) return;
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) bt_mom_b_body(a, so, sn, vb % nbx, vb / nbx);
+    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) bt_mom_b_body(a, so, sn, vb);
     if (!grid_barrier(ctr, target += per, err, kGridWaitCycles)) return;
     const double wgt = (double)(a.nts - itime + 1);
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) bt_corr_body(a, so, sn, wgt, vb % nbx, vb / nbx);
+    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) bt_corr_body(a, so, sn, wgt, vb);
     if (itime < a.nts && !grid_barrier(ctr, target += per, err, kGridWaitCycles)) return;
   }
 }
@@ -1518,8 +1530,8 @@ int grid_barrier_selftest(mom5gpu_domain* d, int rounds, int unreachable) {
   return MOM5GPU_OK;
 }
 
-__global__ void k_bt_post2(BtArgs a, double* conv, double* eta_u, double* ps_out) { bt_post2_body(a, conv, eta_u, ps_out, blockIdx.x, blockIdx.y); }
-__global__ void k_bt_post3(BtArgs a, const double* ps, double* gxo, double* gyo) { bt_post3_body(a, ps, gxo, gyo, blockIdx.x, blockIdx.y); }
+__global__ void k_bt_post2(BtArgs a, double* conv, double* eta_u, double* ps_out) { bt_post2_body(a, conv, eta_u, ps_out, blockIdx.x); }
+__global__ void k_bt_post3(BtArgs a, const double* ps, double* gxo, double* gyo) { bt_post3_body(a, ps, gxo, gyo, blockIdx.x); }
 
 int make_bt_args(mom5gpu_domain* d, int tau, int taup1, BtArgs* ap, BtExtra* xp) {
   const Geo& g = d->geo;
@@ -1660,14 +1672,14 @@ int launch_barotropic(mom5gpu_domain* d, int tau, int taup1) {
   const bool fused = form == 1;
   const long sub_launches = coop      ? 1
                             : fused   ? (long)a.nts
-                            : a.cgrid ? (long)a.nts * (3 + 2 * halo)
                                       : 1 + 2L * a.nts;
   count_launches(d, 1 + (a.cgrid ? 1 : 0) + (a.btf ? 1 : 0) + sub_launches + 4 + 5 * halo);
   k_bt_init<<<(unsigned)((n2 + 255) / 256), 256, 0, s>>>(a, eta_bar_tau, eta_tau, ud_tau, vd_tau, pme, river, src,
                                                           esm, d->opt.initsum_with_bar);
-  dim3 g2((g.ni + 2 + 127) / 128, g.nj + 2);
+  const int bt = bt_threads(g);
+  const dim3 g2 = bt_grid(g, bt);
+  const bool bint = bt_int_products(n2);
   if (a.cgrid) {
-    cudaMemsetAsync(a.cf, 0, sizeof(double) * 8 * n2, s);
     dim3 gc((g.ni + 127) / 128, g.nj);
     k_bt_cgrid_init<<<gc, 128, 0, s>>>(a);
   }
@@ -1686,21 +1698,19 @@ int launch_barotropic(mom5gpu_domain* d, int tau, int taup1) {
         launch_pdl(k_bt_fused, gf, dim3(kFusedThreads), st, a, so, sn, (int)(itime > 1), (double)(a.nts - itime + 1));
         continue;
       }
-      if (!a.cgrid) {
-        // B grid: the predictor as a launch of its own only in the first
-        // subcycle; every corrector but the last forms the next predictor
-        const double wgt = (double)(a.nts - itime + 1);
-        if (itime == 1) launch_pdl(k_bt_pred, g2, dim3(128), st, a, so, sn, 0);
-        launch_pdl(k_bt_mom_b, g2, dim3(128), st, a, so, sn);
-        if (itime < a.nts) launch_pdl(k_bt_corr_pred, g2, dim3(128), st, a, so, sn, wgt);
-        else launch_pdl(k_bt_corr, g2, dim3(128), st, a, so, sn, wgt);
+      // the predictor as a launch of its own only in the first subcycle; every
+      // corrector but the B grid's last forms the next predictor
+      const double wgt = (double)(a.nts - itime + 1);
+      if (itime == 1) launch_pdl(k_bt_pred, g2, dim3(bt), st, a, so, sn, 0);
+      if (a.cgrid) {
+        launch_pdl(bint ? k_bt_mom_c<true> : k_bt_mom_c<false>, g2, dim3(bt), st, a, so, sn, itime);
+        launch_pdl(bint ? k_bt_corr_pred_c<true> : k_bt_corr_pred_c<false>, g2, dim3(bt), st, a, so, sn, wgt);
         continue;
       }
-      k_bt_pred<<<g2, 128, 0, st>>>(a, so, sn, itime > 1);
-      k_bt_mom_c<<<g2, 128, 0, st>>>(a, so, sn, itime);
-      launch_halo_fill(g, a.ubt + sn * n2, 1, 3, st);
-      launch_halo_fill(g, a.vbt + sn * n2, 1, 3, st);
-      k_bt_corr<<<g2, 128, 0, st>>>(a, so, sn, (double)(a.nts - itime + 1));
+      launch_pdl(bint ? k_bt_mom_b<true> : k_bt_mom_b<false>, g2, dim3(bt), st, a, so, sn);
+      if (itime < a.nts)
+        launch_pdl(bint ? k_bt_corr_pred<true> : k_bt_corr_pred<false>, g2, dim3(bt), st, a, so, sn, wgt);
+      else launch_pdl(k_bt_corr, g2, dim3(bt), st, a, so, sn, wgt);
     }
   };
   int crc = coop ? launch_bt_coop(d, a, s) : MOM5GPU_EUNSUPPORTED;
@@ -1712,10 +1722,10 @@ int launch_barotropic(mom5gpu_domain* d, int tau, int taup1) {
   launch_halo_fill(g, a.eta_bar, 1, 3, s);
   launch_halo_fill(g, a.udrho_u, 1, 3, s);
   launch_halo_fill(g, a.udrho_v, 1, 3, s);
-  k_bt_post2<<<g2, 128, 0, s>>>(a, conv, eta_u, ps_out);
+  k_bt_post2<<<g2, bt, 0, s>>>(a, conv, eta_u, ps_out);
   launch_halo_fill(g, conv, 1, 3, s);
   launch_halo_fill(g, eta_u, 1, 3, s);
-  k_bt_post3<<<g2, 128, 0, s>>>(a, ps_out, gxo, gyo);
+  k_bt_post3<<<g2, bt, 0, s>>>(a, ps_out, gxo, gyo);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MOM5GPU_OK : cuda_fail(d, e, "barotropic");
 }
@@ -1735,7 +1745,7 @@ int launch_barotropic_phase(mom5gpu_domain* d, int tau, int taup1, int phase, in
     return fail(d, MOM5GPU_EINVAL, "barotropic subcycle %d (1..%d)", itime, a.nts);
   long n2 = g.n2;
   cudaStream_t s = d->stream;
-  dim3 g2((g.ni + 2 + 127) / 128, g.nj + 2);
+  const dim3 g2 = bt_grid(g, 128);
   int so = (itime + 0) % 2, sn = (itime + 1) % 2;
   switch (phase) {
     case 0:
@@ -1749,7 +1759,7 @@ int launch_barotropic_phase(mom5gpu_domain* d, int tau, int taup1, int phase, in
       count_launches(d, 1);
       break;
     case 2:
-      k_bt_mom_b<<<g2, 128, 0, s>>>(a, so, sn);
+      k_bt_mom_b<false><<<g2, 128, 0, s>>>(a, so, sn);
       k_bt_corr<<<g2, 128, 0, s>>>(a, so, sn, (double)(a.nts - itime + 1));
       count_launches(d, 2);
       break;

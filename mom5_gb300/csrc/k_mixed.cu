@@ -5,32 +5,31 @@
 
 namespace mom5 {
 
-__global__ void __launch_bounds__(128) k_btf_prep(BtArgs a) { btfast::prep_body(a, blockIdx.x, blockIdx.y); }
+__global__ void __launch_bounds__(128) k_btf_prep(BtArgs a) { btfast::prep_body(a, blockIdx.x); }
 // The subcycle kernels are launched as programmatic dependents (launch_pdl).
 __global__ void __launch_bounds__(128) k_btf_pred(BtArgs a, int so, int sn, int reuse) {
   pdl_wait();
   pdl_trigger();
-  btfast::pred_body(a, so, sn, reuse, blockIdx.x, blockIdx.y);
+  btfast::pred_body(a, so, sn, reuse, blockIdx.x);
 }
 __global__ void __launch_bounds__(128) k_btf_mom(BtArgs a, int so, int sn, double wgt) {
   pdl_wait();
   pdl_trigger();
-  btfast::mom_body(a, so, sn, wgt, blockIdx.x, blockIdx.y);
+  btfast::mom_body(a, so, sn, wgt, blockIdx.x);
 }
 __global__ void __launch_bounds__(128) k_btf_corr(BtArgs a, int so, int sn) {
   pdl_wait();
   pdl_trigger();
-  btfast::corr_body(a, so, sn, blockIdx.x, blockIdx.y);
+  btfast::corr_body(a, so, sn, blockIdx.x);
 }
 __global__ void __launch_bounds__(128) k_btf_corr_pred(BtArgs a, int so, int sn) {
   pdl_wait();
   pdl_trigger();
-  btfast::corr_pred_body(a, so, sn, blockIdx.x, blockIdx.y);
+  btfast::corr_pred_body(a, so, sn, blockIdx.x);
 }
 
 void launch_btf_prep(const BtArgs& a, cudaStream_t s) {
-  dim3 g2((a.g.ni + 2 + 127) / 128, a.g.nj + 2);
-  k_btf_prep<<<g2, 128, 0, s>>>(a);
+  k_btf_prep<<<bt_grid(a.g, 128), 128, 0, s>>>(a);
 }
 
 // One launch per subcycle (mom5gpu_set_barotropic_fusion mode 1): 32 x 8 tiles of
@@ -60,11 +59,11 @@ int launch_btf_subcycle(const BtArgs& a, int itime, int nts, bool fused, cudaStr
     launch_pdl(k_btf_fused, gf, dim3(kBtfThreads), s, a, so, sn, (int)(itime > 1), wgt);
     return 1;
   }
-  dim3 g2((a.g.ni + 2 + 127) / 128, a.g.nj + 2);
-  if (itime == 1) launch_pdl(k_btf_pred, g2, dim3(128), s, a, so, sn, 0);
-  launch_pdl(k_btf_mom, g2, dim3(128), s, a, so, sn, wgt);
-  if (itime < nts) launch_pdl(k_btf_corr_pred, g2, dim3(128), s, a, so, sn);
-  else launch_pdl(k_btf_corr, g2, dim3(128), s, a, so, sn);
+  const dim3 b(bt_threads(a.g)), g2 = bt_grid(a.g, b.x);
+  if (itime == 1) launch_pdl(k_btf_pred, g2, b, s, a, so, sn, 0);
+  launch_pdl(k_btf_mom, g2, b, s, a, so, sn, wgt);
+  if (itime < nts) launch_pdl(k_btf_corr_pred, g2, b, s, a, so, sn);
+  else launch_pdl(k_btf_corr, g2, b, s, a, so, sn);
   return itime == 1 ? 3 : 2;
 }
 
