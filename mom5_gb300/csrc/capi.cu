@@ -318,7 +318,7 @@ void mom5gpu_destroy(mom5gpu_domain* d) {
   QuickerWeights& q = d->qw;
   for (double* p : {q.quick_x, q.quick_y, q.curv_xp, q.curv_xn, q.curv_yp, q.curv_yn, q.quick_z, q.curv_zp, q.curv_zn})
     if (p) cudaFree(p);
-  for (double* p : {d->cori1, d->cori2, d->mdfl_a, d->mdfl_b, d->bt, d->red, d->ppm_scr, d->psom_scr})
+  for (double* p : {d->cori1, d->cori2, d->mdfl_a, d->mdfl_b, d->bt, d->red, d->psom_scr})
     if (p) cudaFree(p);
   if (d->mixed_scr) cudaFree(d->mixed_scr);
   if (d->flag) cudaFree(d->flag);

@@ -55,6 +55,17 @@ DEVI double half_exact(double x) {
   return r;
 }
 
+// 2*x: the exponent raised by one where both are normal; +-0 is unchanged, the rest
+// take the multiply.
+DEVI double twice(double x) {
+  const long long b = bits_of(x);
+  const unsigned e = (unsigned)((unsigned long long)b >> 52) & 0x7ffu;
+  const bool normal = e - 1u < 0x7fdu;  // 1 <= e <= 0x7fd
+  double r = double_of(normal ? b + (1LL << 52) : b);
+  rare_lanes(!(normal || (b << 1) == 0), [&] { r = 2.0 * x; });
+  return r;
+}
+
 // Arithmetic of an MDFL pass: sums on the FP64 pipe, the products whose bit is set
 // in MASK on the integer pipe.  The four of a face (d1*theta, c*theta, psi*Rj, the
 // mass flux) go there; with one more of the update's the passes took 0 to 3%

@@ -964,153 +964,130 @@ struct PpmArgs {
   int lim;
   double dtime;
   const double *tmask, *dat, *datr, *dxte, *dyte, *dxtn, *dytn, *uh, *vh, *w, *rdz, *T;
-  double *dak, *fz, *tz, *tx, *th;
+  double *tz, *tx, *th;
 };
 
-// vertical slope dak of every cell with the clamped neighbour levels and their
-// collapse factors real(kp1-k) ... (:6064-6099)
-__global__ void k_ppm_dak(PpmArgs a) {
-  const Geo& g = a.g;
-  int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1, k = blockIdx.z;
-  if (i > g.ni) return;
-  const int nk = g.nk, K = k + 1;
-  int km2 = K - 2 > 1 ? K - 2 : 1, km1 = K - 1 > 1 ? K - 1 : 1, kp1 = K + 1 < nk ? K + 1 : nk,
-      kp2 = K + 2 < nk ? K + 2 : nk;
-  auto at = [&](const double* f, int L) { return f[I3(g, i, j, L - 1)]; };
-  double S[5] = {at(a.T, km2), at(a.T, km1), at(a.T, K), at(a.T, kp1), at(a.T, kp2)};
-  double M[5] = {at(a.tmask, km2) * (double)(km1 - km2), at(a.tmask, km1) * (double)(K - km1), at(a.tmask, K),
-                 at(a.tmask, kp1) * (double)(kp1 - K), at(a.tmask, kp2) * (double)(kp2 - kp1)};
-  double t0, t1, t2, t3;
-  ppm::slope(S, M, a.dak[I3(g, i, j, k)], t0, t1, t2, t3);
+using ppm::Edges;
+using ppm::LineSmem;
+
+// Positions per segment of a line of n cells: each segment closes 8 cells fewer, so
+// of four lengths the one that covers the line with the fewest threads.  With 48
+// registers a thread some are spilled, but the FP64 pipe's latency wants the warps
+// (180x135x50 cells, 2 tracers: 753 us a step with the 62 to 72 registers of the
+// compiler's choice and 19 to 28 warps per SM, 635 with 40).
+static int ppm_length(int n, int l0, int l1, int l2, int l3) {
+  int best = l0;
+  for (int L : {l1, l2, l3})
+    if ((n + L - 9) / (L - 8) * L < (n + best - 9) / (best - 8) * best) best = L;
+  return best;
 }
 
-// edge values, limiter and the fluxes through the bottom (massflux <= 0) and top
-// (massflux > 0) faces of a cell (:6101-6170).  The reference's loop over the
-// levels carries nothing from one level to the next, and a face is written by
-// exactly one of its two cells (the same mask-product massflux, <= 0 from above,
-// > 0 from below), so every cell runs in its own thread.
-__global__ void k_ppm_zflux(PpmArgs a) {
+// z pass (:6064-6182), PPM_BY columns per block, segments of L - 8 levels: the
+// flux through a face comes from the level above it where the masked flow is
+// downward or nil (<= 0), else from the one below, at the Courant number of the
+// level above.
+constexpr int PPM_BY = 4, PPM_WARPS = 40;  // columns per block, resident warps per SM (48 registers; see ppm_length)
+
+template <int L>
+__global__ void __launch_bounds__(PPM_BY* L, 32 * PPM_WARPS / (PPM_BY * L)) k_ppm_z(PpmArgs a) {
+  __shared__ LineSmem<L, PPM_BY> sm;
   const Geo& g = a.g;
-  int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;
-  if (i > g.ni) return;
-  const int nk = g.nk;
-  const long q = I2(g, i, j);
-  auto at = [&](const double* f, int L) { return f[I3(g, i, j, L - 1)]; };
-  const double dat = a.dat[q];
-  {
-    const int K = blockIdx.z + 1;
-    int km2 = K - 2 > 1 ? K - 2 : 1, km1 = K - 1 > 1 ? K - 1 : 1, kp1 = K + 1 < nk ? K + 1 : nk,
-        kp2 = K + 2 < nk ? K + 2 : nk;
-    double mskp2 = at(a.tmask, kp2) * (double)(kp2 - kp1), mskp1 = at(a.tmask, kp1) * (double)(kp1 - K);
-    double msk0 = at(a.tmask, K), mskm1 = at(a.tmask, km1) * (double)(K - km1);
-    double mskm2 = at(a.tmask, km2) * (double)(km1 - km2);
-    double Sip2 = at(a.T, kp2), Sip1 = at(a.T, kp1), Si = at(a.T, K), Sim1 = at(a.T, km1), Sim2 = at(a.T, km2);
-    double d1m = (Si - Sim1) * mskm1, d1p = (Sip1 - Si) * mskp1;
-    double d1mm = (Sim1 - Sim2) * mskm1 * mskm2, d1pp = (Sip2 - Sip1) * mskp1 * mskp2;
-    Sim1 = Si - d1m;
-    Sip1 = Si + d1p;
-    double dk = at(a.dak, K);
-    double al = 0.5 * (Sim1 + Si) + ppm::kSixth * (at(a.dak, km1) - dk);
-    double ar = 0.5 * (Si + Sip1) + ppm::kSixth * (dk - at(a.dak, kp1));
-    ppm::limit(a.lim, Si, dk, d1m, d1p, d1mm, d1pp, al, ar);
-    double c6 = 6. * Si - 3. * (ar + al);
-    double wk = a.w[I3(g, i, j, K)];
-    double massflux = dat * wk * msk0 * mskp1;
-    if (!sel::gt0(massflux)) {
-      double cfl = fabs(div_seeded(wk * a.dtime, at(a.rdz, K)));
-      a.fz[I3(g, i, j, K - 1)] = massflux * (ar + 0.5 * cfl * ((al - ar) + (1. - ppm::kTwoThirds * cfl) * c6));
-    }
-    double wkm1 = a.w[I3(g, i, j, km1)];
-    massflux = dat * wkm1 * msk0 * mskm1;
-    if (sel::gt0(massflux)) {
-      double cfl = fabs(div_seeded(wkm1 * a.dtime, at(a.rdz, km1)));
-      a.fz[I3(g, i, j, km1 - 1)] = massflux * (al + 0.5 * cfl * ((ar - al) + (1. - ppm::kTwoThirds * cfl) * c6));
-    }
-  }
+  const int i = blockIdx.x * PPM_BY + threadIdx.x + 1, j = blockIdx.y + 1, nk = g.nk;
+  auto at = [&](const double* f, int K) { return f[I3(g, i, j, K - 1)]; };
+  auto S = [&](int K) { return at(a.T, K < 1 ? 1 : K > nk ? nk : K); };
+  auto M = [&](int K) { return K >= 1 && K <= nk && !fp64::is_zero(at(a.tmask, K)); };
+  auto face = [&](int K, const Edges& up, const Edges& lo) {
+    const double wk = a.w[I3(g, i, j, K)];
+    const double mf = mul_int<false, true>(a.dat[I2(g, i, j)], wk);
+    const double cfl = ppm::magnitude(div_seeded(mul_int<false, true>(a.dtime, wk), at(a.rdz, K)));
+    const bool below = sel::gt0(mf);
+    return ppm::upwind_flux(mf, cfl, below ? lo.L : up.R, below ? lo.R : up.L, below ? lo.six : up.six);
+  };
+  auto upd = [&](int K, double T, bool, double Ft, double Fb) {
+    const long p = I3(g, i, j, K - 1);
+    const double wtop = K > 1 ? a.w[p] : 0.0;
+    a.tz[p] = T + mul_int<false, true>(div_seeded(a.dtime, a.rdz[p]),
+                                       mul_int<false, true>(a.datr[I2(g, i, j)], Fb - Ft) +
+                                           mul_int<true, true>(T, wtop - a.w[p + g.n2]));
+  };
+  ppm::tile_line<L, PPM_BY, true>(nk, a.lim, (int)blockIdx.z * (L - 8) - 3, threadIdx.y, threadIdx.x,
+                                       i <= g.ni, sm, S, M, face, upd);
 }
 
-// vertical update of tracer_mdppm (:6173-6182)
-__global__ void k_ppm_zupd(PpmArgs a) {
-  const Geo& g = a.g;
-  int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1, k = blockIdx.z;
-  if (i > g.ni) return;
-  const int K = k + 1, km1 = K - 1 > 1 ? K - 1 : 1;
-  const double mskm1 = (double)(K - km1);
-  long p = I3(g, i, j, k), pm = I3(g, i, j, km1 - 1);
-  double T = a.T[p];
-  a.tz[p] = T + div_seeded(a.dtime, a.rdz[p]) *
-                    (a.datr[I2(g, i, j)] * (a.fz[p] - mskm1 * a.fz[pm]) +
-                     T * (mskm1 * a.w[I3(g, i, j, km1)] - a.w[I3(g, i, j, K)]));
+// A horizontal face of length len and cell distance dist at p and its neighbour pn:
+// mass flux len*u and Courant number (:6293-6305, :6470-6482)
+DEVI double ppm_hface(double u, double dt, double len, double dist, double rdz, double rdz_n, const Edges& lo,
+                      const Edges& hi) {
+  const double mf = mul_int<true, true>(len, u);
+  const bool pos = sel::ge0(mf);
+  const double cfl = div_seeded(twice(mul_int<false, true>(dt, u)), mul_int(rdz + rdz_n, dist));
+  return ppm::upwind_flux(mf, neg_if(cfl, !pos), pos ? lo.R : hi.L, pos ? lo.L : hi.R, pos ? lo.six : hi.six);
 }
 
 // x pass along the rows (:6193-6325): tracer_mdppm after the x halo update;
-// segments of PPM_LX - 8 cells, one thread per position
-constexpr int PPM_LX = 128, PPM_BY = 8, PPM_LY = 64;
-
-__global__ void __launch_bounds__(PPM_LX) k_ppm_x(PpmArgs a) {
-  __shared__ double sm[7][PPM_LX][1];
+// segments of L - 8 cells, one thread per position
+template <int L>
+__global__ void __launch_bounds__(L, 32 * PPM_WARPS / L) k_ppm_x(PpmArgs a) {
+  __shared__ LineSmem<L, 1> sm;
   const Geo& g = a.g;
   const int j = blockIdx.y + 1, k = blockIdx.z;
   const double dt = a.dtime;
   auto S = [&](int i) { return tq(g, a.tz, i, j, k); };
-  auto M = [&](int i) { return tq(g, a.tmask, i, j, k); };
-  auto face = [&](int i, double m0, double m1, double aL0, double aR0, double a60, double aL1, double aR1,
-                  double a61) {
-    double u = a.uh[I3(g, i, j, k)];
-    double massflux = a.dyte[I2(g, i, j)] * u;
-    double cfl = div_seeded(u * dt * 2.0, (a.rdz[I3(g, i, j, k)] + a.rdz[I3(g, i + 1, j, k)]) * a.dxte[I2(g, i, j)]);
-    return ppm::hflux(massflux, m0, m1, cfl, aL0, aR0, a60, aL1, aR1, a61);
+  auto M = [&](int i) { return !fp64::is_zero(tq(g, a.tmask, i, j, k)); };
+  auto face = [&](int i, const Edges& lo, const Edges& hi) {
+    return ppm_hface(a.uh[I3(g, i, j, k)], dt, a.dyte[I2(g, i, j)], a.dxte[I2(g, i, j)], a.rdz[I3(g, i, j, k)],
+                     a.rdz[I3(g, i + 1, j, k)], lo, hi);
   };
-  auto upd = [&](int i, double Sv, double m, double Fw, double Fe) {
-    long p = I3(g, i, j, k);
-    double div = a.dyte[I2(g, i, j)] * a.uh[p] - a.dyte[I2(g, i - 1, j)] * a.uh[I3(g, i - 1, j, k)];
-    a.tx[p] = Sv + div_seeded(dt * m * a.datr[I2(g, i, j)], a.rdz[p]) * (Fw - Fe + a.T[p] * div);
+  auto upd = [&](int i, double Sv, bool wet, double Fw, double Fe) {
+    const long p = I3(g, i, j, k), q = I2(g, i, j);
+    double t = Sv;
+    if (wet) {  // a dry cell's factor dtime*tmask*datr/rho_dzt is zero
+      const double div = mul_int<true, true>(a.dyte[q], a.uh[p]) - mul_int<true, true>(a.dyte[q - 1], a.uh[p - 1]);
+      t = Sv + mul_int<false, true>(div_seeded(mul_int(dt, a.datr[q]), a.rdz[p]),
+                                    Fw - Fe + mul_int<true, true>(a.T[p], div));
+    }
+    a.tx[p] = t;
   };
-  ppm::tile_line<PPM_LX, 1>(g.ni, a.lim, (int)blockIdx.x * (PPM_LX - 8) - 3, threadIdx.x, 0, true, sm, S, M, face,
-                            upd);
+  ppm::tile_line<L, 1, false>(g.ni, a.lim, (int)blockIdx.x * (L - 8) - 3, threadIdx.x, 0, true, sm, S, M,
+                                   face, upd);
 }
 
 // y pass along the columns (:6330-6502) and the tendency: th += -advect_tracer_mdppm;
-// PPM_BY columns per block, segments of PPM_LY - 8 cells
-__global__ void __launch_bounds__(PPM_BY* PPM_LY) k_ppm_y(PpmArgs a) {
-  __shared__ double sm[7][PPM_LY][PPM_BY];
+// PPM_BY columns per block, segments of L - 8 cells
+template <int L>
+__global__ void __launch_bounds__(PPM_BY* L, 32 * PPM_WARPS / (PPM_BY * L)) k_ppm_y(PpmArgs a) {
+  __shared__ LineSmem<L, PPM_BY> sm;
   const Geo& g = a.g;
   const int i = blockIdx.x * PPM_BY + threadIdx.x + 1, k = blockIdx.z;
   const double dt = a.dtime;
   auto S = [&](int j) { return tq(g, a.tx, i, j, k); };
-  auto M = [&](int j) { return tq(g, a.tmask, i, j, k); };
-  auto face = [&](int j, double m0, double m1, double aL0, double aR0, double a60, double aL1, double aR1,
-                  double a61) {
-    double v = a.vh[I3(g, i, j, k)];
-    double massflux = a.dxtn[I2(g, i, j)] * v;
-    double cfl = div_seeded(v * dt * 2.0, (a.rdz[I3(g, i, j, k)] + a.rdz[I3(g, i, j + 1, k)]) * a.dytn[I2(g, i, j)]);
-    return ppm::hflux(massflux, m0, m1, cfl, aL0, aR0, a60, aL1, aR1, a61);
+  auto M = [&](int j) { return !fp64::is_zero(tq(g, a.tmask, i, j, k)); };
+  auto face = [&](int j, const Edges& lo, const Edges& hi) {
+    return ppm_hface(a.vh[I3(g, i, j, k)], dt, a.dxtn[I2(g, i, j)], a.dytn[I2(g, i, j)], a.rdz[I3(g, i, j, k)],
+                     a.rdz[I3(g, i, j + 1, k)], lo, hi);
   };
-  auto upd = [&](int j, double Sv, double m, double Fs, double Fn) {
-    long p = I3(g, i, j, k);
-    double rdz = a.rdz[p], datr = a.datr[I2(g, i, j)], T = a.T[p];
-    double t = Sv + div_seeded(dt * a.tmask[p] * datr, rdz) * (Fs - Fn);
-    double wkm1 = k > 0 ? a.w[I3(g, i, j, k)] : 0.0;
-    t = t + div_seeded(dt * T, rdz) *
-                (a.w[I3(g, i, j, k + 1)] - wkm1 +
-                 datr * (a.dyte[I2(g, i - 1, j)] * a.uh[I3(g, i - 1, j, k)] - a.dyte[I2(g, i, j)] * a.uh[p]));
-    double advect = div_seeded(-rdz * (t - T), dt) * m;
+  auto upd = [&](int j, double Sv, bool wet, double Fs, double Fn) {
+    if (!wet) return;  // the tendency of a dry cell is multiplied by its mask
+    const long p = I3(g, i, j, k), q = I2(g, i, j);
+    const double rdz = a.rdz[p], datr = a.datr[q], T = a.T[p];
+    const fp64::Divisor d = fp64::divisor_of(rdz);
+    double t = Sv + mul_int<false, true>(fp64::div_by(mul_int(dt, datr), rdz, d), Fs - Fn);
+    const double wkm1 = k > 0 ? a.w[p] : 0.0;
+    t = t + mul_int<true, true>(fp64::div_by(mul_int<false, true>(dt, T), rdz, d),
+                                a.w[p + g.n2] - wkm1 +
+                                    mul_int<false, true>(datr, mul_int<true, true>(a.dyte[q - 1], a.uh[p - 1]) -
+                                                                   mul_int<true, true>(a.dyte[q], a.uh[p])));
+    const double advect = div_seeded(mul_int<false, true>(-rdz, t - T), dt);
     a.th[p] = a.th[p] + (-advect);
   };
-  ppm::tile_line<PPM_LY, PPM_BY>(g.nj, a.lim, (int)blockIdx.y * (PPM_LY - 8) - 3, threadIdx.y, threadIdx.x,
-                                 i <= g.ni, sm, S, M, face, upd);
+  ppm::tile_line<L, PPM_BY, false>(g.nj, a.lim, (int)blockIdx.y * (L - 8) - 3, threadIdx.y, threadIdx.x,
+                                        i <= g.ni, sm, S, M, face, upd);
 }
 
 int launch_mdppm(mom5gpu_domain* d, int n, int taum1, int tau, double dtime) {
   const Geo& g = d->geo;
   int rc = ensure_mdfl_scratch(d, 1);
   if (rc) return rc;
-  if (!d->ppm_scr) {
-    cudaError_t e = cudaMalloc(&d->ppm_scr, sizeof(double) * 2 * (size_t)g.n3);
-    if (e != cudaSuccess) return fail(d, MOM5GPU_ENOMEM, "mdppm scratch: %s", cudaGetErrorString(e));
-    d->bytes += sizeof(double) * 2 * (size_t)g.n3;
-    cudaMemsetAsync(d->ppm_scr, 0, sizeof(double) * 2 * (size_t)g.n3, d->stream);
-  }
   PpmArgs a;
   a.g = g;
   a.lim = d->scheme[n - 1].ppm_limiter;
@@ -1128,23 +1105,29 @@ int launch_mdppm(mom5gpu_domain* d, int n, int taum1, int tau, double dtime) {
   a.rdz = fptr(d, MOM5GPU_RHO_DZT, 0, tau);
   a.T = fptr(d, MOM5GPU_TRACER, n, taum1);
   a.th = fptr(d, MOM5GPU_TH_TENDENCY, n, 0);
-  a.dak = d->ppm_scr;
-  a.fz = d->ppm_scr + g.n3;
   a.tz = d->mdfl_a;
   a.tx = d->mdfl_b;
   const void* need[] = {a.tmask, a.dat, a.datr, a.dxte, a.dyte, a.dxtn, a.dytn, a.uh, a.vh, a.w, a.rdz, a.T, a.th};
   for (const void* p : need)
     if (!p) return fail(d, MOM5GPU_ESTATE, "mdppm: a required field was never set");
   ClockScope clk(d, SEC_MDFL);
-  count_launches(d, 5);
+  count_launches(d, 3);
   cudaStream_t s = d->stream;
-  dim3 g3((g.ni + 127) / 128, g.nj, g.nk);
-  k_ppm_dak<<<g3, 128, 0, s>>>(a);
-  k_ppm_zflux<<<g3, 128, 0, s>>>(a);
-  k_ppm_zupd<<<g3, 128, 0, s>>>(a);
-  k_ppm_x<<<dim3((g.ni + PPM_LX - 9) / (PPM_LX - 8), g.nj, g.nk), PPM_LX, 0, s>>>(a);
-  k_ppm_y<<<dim3((g.ni + PPM_BY - 1) / PPM_BY, (g.nj + PPM_LY - 9) / (PPM_LY - 8), g.nk), dim3(PPM_BY, PPM_LY), 0, s>>>(
-      a);
+  const int nb = (g.ni + PPM_BY - 1) / PPM_BY;
+  auto segments = [](int n, int L) { return (n + L - 9) / (L - 8); };
+#define PPM_Z(L) k_ppm_z<L><<<dim3(nb, g.nj, segments(g.nk, L)), dim3(PPM_BY, L), 0, s>>>(a)
+#define PPM_X(L) k_ppm_x<L><<<dim3(segments(g.ni, L), g.nj, g.nk), L, 0, s>>>(a)
+#define PPM_Y(L) k_ppm_y<L><<<dim3(nb, segments(g.nj, L), g.nk), dim3(PPM_BY, L), 0, s>>>(a)
+#define PPM_LENGTHS(K, n, l0, l1, l2, l3)            \
+  switch (ppm_length(n, l0, l1, l2, l3)) {           \
+    case l0: K(l0); break;                           \
+    case l1: K(l1); break;                           \
+    case l2: K(l2); break;                           \
+    default: K(l3);                                  \
+  }
+  PPM_LENGTHS(PPM_Z, g.nk, 64, 24, 40, 80)
+  PPM_LENGTHS(PPM_X, g.ni, 128, 64, 96, 192)
+  PPM_LENGTHS(PPM_Y, g.nj, 64, 32, 48, 80)
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MOM5GPU_OK : cuda_fail(d, e, "mdppm");
 }
