@@ -112,26 +112,29 @@ DEVI void ps_diff(float p00, float p10, float p01, float p11, float& px, float& 
   py = (p01 + p11) - (p00 + p10);
 }
 // momentum step of point q from its PS differences: the new transports un, vn
-DEVI void mom_point(const BtArgs& a, int so, long q, float px, float py, double& un, double& vn) {
-  const long n2 = a.g.n2;
-  double uo = a.ubt[so * n2 + q], vo = a.vbt[so * n2 + q];
-  float uf = mixed::d2f_rn(uo), vf = mixed::d2f_rn(vo), hf = plane(a, A)[q];
-  float d1 = fmaf(hf, vf, fmaf(plane(a, BX)[q], px, plane(a, PX)[q]));
-  float d2 = fmaf(-hf, uf, fmaf(plane(a, BY)[q], py, plane(a, PY)[q]));
-  float t1 = uf + d1, t2 = vf + d2, g1 = plane(a, G1)[q], g2 = plane(a, G2)[q];
+template <bool EARLY>
+struct MomIn {
+  Loaded<EARLY, double> uo, vo;
+  Loaded<EARLY, float> hf, bx, px, by, py, g1, g2;
+  DEVI MomIn(const BtArgs& a, int so, long q)
+      : uo(a.ubt + so * a.g.n2 + q), vo(a.vbt + so * a.g.n2 + q), hf(plane(a, A) + q), bx(plane(a, BX) + q),
+        px(plane(a, PX) + q), by(plane(a, BY) + q), py(plane(a, PY) + q), g1(plane(a, G1) + q), g2(plane(a, G2) + q) {}
+};
+template <bool EARLY>
+DEVI void mom_point(const MomIn<EARLY>& m, float px, float py, double& un, double& vn) {
+  const double uo = m.uo, vo = m.vo;
+  const float uf = mixed::d2f_rn(uo), vf = mixed::d2f_rn(vo), hf = m.hf;
+  float d1 = fmaf(hf, vf, fmaf(m.bx, px, m.px));
+  float d2 = fmaf(-hf, uf, fmaf(m.by, py, m.py));
+  float t1 = uf + d1, t2 = vf + d2, g1 = m.g1, g2 = m.g2;
   un = uo + mixed::f2d(d1 + fmaf(g1, t1, g2 * t2));
   vn = vo + mixed::f2d(d2 + fmaf(g1, t2, -g2 * t1));
 }
 // time sums of the transports of point q, formed where the new transports are
 // (the momentum step; the corrector does not change them)
-DEVI void sum_point(const BtArgs& a, double wgt, long q, double un, double vn) {
-  if (a.stepB) {
-    a.udrho_u[q] = fma(wgt, un, a.udrho_u[q]);
-    a.udrho_v[q] = fma(wgt, vn, a.udrho_v[q]);
-  } else {
-    a.udrho_u[q] += un;
-    a.udrho_v[q] += vn;
-  }
+DEVI void sum_point(const BtArgs& a, double wgt, long q, double un, double vn, double su, double sv) {
+  a.udrho_u[q] = a.stepB ? fma(wgt, un, su) : su + un;
+  a.udrho_v[q] = a.stepB ? fma(wgt, vn, sv) : sv + vn;
 }
 // corrector of point q from its divergence D, with the time sum of eta
 DEVI double corr_point(const BtArgs& a, int so, int sn, long q, float D) {
@@ -187,23 +190,28 @@ DEVI void pred_body(const BtArgs& a, int so, int sn, int reuse, int bx) {
   plane(a, PS)[q0] = ps;
 }
 
+template <bool EARLY>
 DEVI void mom_body(const BtArgs& a, int so, int sn, double wgt, int bx) {
+  if (!EARLY) bt_after_previous();
   const Geo& g = a.g;
   int i, j;
   if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j), n2 = g.n2;
+  const MomIn<EARLY> in(a, so, q);
+  const Loaded<EARLY, double> dyu(a.dyu + q), dxu(a.dxu + q), su(a.udrho_u + q), sv(a.udrho_v + q);
+  if (EARLY) bt_after_previous();
   float px = 0.0f, py = 0.0f;
   if (i <= g.ni && j <= g.nj) {
     const float* ps = plane(a, PS);
     ps_diff(ps[q], ps[q + 1], ps[q + g.nxd], ps[q + g.nxd + 1], px, py);
   }
   double un, vn;
-  mom_point(a, so, q, px, py, un, vn);
+  mom_point(in, px, py, un, vn);
   a.ubt[sn * n2 + q] = un;
   a.vbt[sn * n2 + q] = vn;
-  a.uhb[sn * n2 + q] = un * a.dyu[q];
-  a.vhb[sn * n2 + q] = vn * a.dxu[q];
-  sum_point(a, wgt, q, un, vn);
+  a.uhb[sn * n2 + q] = un * dyu;
+  a.vhb[sn * n2 + q] = vn * dxu;
+  sum_point(a, wgt, q, un, vn, su, sv);
 }
 
 DEVI void corr_body(const BtArgs& a, int so, int sn, int bx) {
@@ -224,20 +232,28 @@ DEVI void corr_body(const BtArgs& a, int so, int sn, int bx) {
 // it is.  The predicted eta is not stored (the next corrector overwrites it
 // unread), nor is the divergence.  Same arithmetic as corr_body then pred_body
 // with reuse, so the same bits.
+template <bool EARLY>
 DEVI void corr_pred_body(const BtArgs& a, int so, int sn, int bx) {
+  if (!EARLY) bt_after_previous();
   const Geo& g = a.g;
   int i, j;
   if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j), n2 = g.n2;
+  const Loaded<EARLY, double> eo(a.eta_bt + so * n2 + q), bar(a.eta_bar + q), e0q(eref(a) + q);
+  const Loaded<EARLY, float> kc(plane(a, KC) + q), sc(plane(a, SC) + q), kg(plane(a, KG) + q), sg(plane(a, SG) + q),
+      rgq(plane(a, RG) + q);
+  if (EARLY) bt_after_previous();
   const float D = div_num(g, a.uhb + sn * n2, a.vhb + sn * n2, i, j);
-  double en = corr_point(a, so, sn, q, D);
+  double en = eo + mixed::f2d(fmaf(kc, D, sc));  // corr_point
+  a.eta_bt[sn * n2 + q] = en;
+  a.eta_bar[q] = bar + en;
   // the next subcycle's predictor at this point (pred_point with reuse)
-  if (a.gamma > 0.0) en += mixed::f2d(fmaf(plane(a, KG)[q], D, plane(a, SG)[q]));
+  if (a.gamma > 0.0) en += mixed::f2d(fmaf(kg, D, sg));
   float* ps = plane(a, PS);
   const float* rg = plane(a, RG);
   const double* e0 = eref(a);
   int ii = i, jj = j;
-  if (!halo_image(g, ii, jj) || (ii == i && jj == j)) ps[q] = rg[q] * mixed::d2f_rn(en - e0[q]);
+  if (!halo_image(g, ii, jj) || (ii == i && jj == j)) ps[q] = rgq * mixed::d2f_rn(en - e0q);
   if (i < 1 || i > g.ni || j < 1 || j > g.nj) return;
   // periodic halo points whose image this compute point is
   int hx[2], nhx = 0, hy[2], nhy = 0;
@@ -306,7 +322,7 @@ DEVI void fused_body(const BtArgs& a, int so, int sn, int reuse, double wgt, int
       ps_diff(ps_s[pe], ps_s[pe + 1], ps_s[pe + PXN], ps_s[pe + PXN + 1], px, py);
     }
     double un, vn;
-    mom_point(a, so, q, px, py, un, vn);
+    mom_point(MomIn<true>(a, so, q), px, py, un, vn);
     const double uh = un * a.dyu[q], vh = vn * a.dxu[q];
     uh_s[e] = uh;
     vh_s[e] = vh;
@@ -315,7 +331,7 @@ DEVI void fused_body(const BtArgs& a, int so, int sn, int reuse, double wgt, int
       a.vbt[sn * n2 + q] = vn;
       a.uhb[sn * n2 + q] = uh;
       a.vhb[sn * n2 + q] = vh;
-      sum_point(a, wgt, q, un, vn);
+      sum_point(a, wgt, q, un, vn, a.udrho_u[q], a.udrho_v[q]);
     }
   }
   __syncthreads();

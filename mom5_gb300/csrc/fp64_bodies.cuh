@@ -539,15 +539,14 @@ DEVI double div_ud(const BtArgs& a, const double* u, const double* v, int i, int
 // B-grid DIV_UD from the stored products uh = u*dyu, vh = v*dxu: the same
 // operations as div_ud on the same values, without recomputing the products.
 template <bool INT = false>
-DEVI double div_ud_bh(const BtArgs& a, const double* uh, const double* vh, int i, int j) {
-  const Geo& g = a.g;
+DEVI double div_ud_bh(const Geo& g, double datr, const double* uh, const double* vh, int i, int j) {
   if (i < 1 || j < 1) return 0.0;
   long q = I2(g, i, j), qw = q - 1, qs = q - g.nxd, qsw = qs - 1;
   double uh_bay = half_exact(uh[q] + uh[qs]);
   double vh_bax = half_exact(vh[q] + vh[qw]);
   double uhim_bay = half_exact(uh[qw] + uh[qsw]);
   double vhjm_bax = half_exact(vh[qs] + vh[qsw]);
-  return bt_mul<INT>(a.datr[q], (uh_bay - uhim_bay) + (vh_bax - vhjm_bax));
+  return bt_mul<INT>(datr, (uh_bay - uhim_bay) + (vh_bax - vhjm_bax));
 }
 
 // image of a halo point under the single-PE full halo update; returns false
@@ -644,7 +643,7 @@ DEVI void bt_pred_body(BtArgs a, int so, int sn, int reuse, int bx) {
   if (dpos(a.gamma)) {
     double dv = reuse ? a.dvs[q]
                       : (a.cgrid ? div_ud(a, a.ubt + so * g.n2, a.vbt + so * g.n2, i, j)
-                                 : div_ud_bh(a, a.uhb + so * g.n2, a.vhb + so * g.n2, i, j));
+                                 : div_ud_bh(g, a.datr[I2(g, i, j)], a.uhb + so * g.n2, a.vhb + so * g.n2, i, j));
     double tm = a.tmask1[q];
     double tmp = is_zero(tm) ? 0.0 : mask_mul(-dv, tm);
     en = eo[q] + a.dtbt_gamma_rho0r * (tmp + a.steady[q]);
@@ -657,46 +656,51 @@ DEVI void bt_pred_body(BtArgs a, int so, int sn, int reuse, int bx) {
 }
 
 // momentum update, B grid (:3466-3485)
-template <bool INT = false>
+template <bool INT = false, bool EARLY = false>
 DEVI void bt_mom_b_body(BtArgs a, int so, int sn, int bx) {
+  if (!EARLY) bt_after_previous();
   const Geo& g = a.g;
   int i, j;
   if (!bt_point(g, bx, i, j)) return;
-  long q = I2(g, i, j);
+  const long q = I2(g, i, j);
+  const Loaded<EARLY, double> um(a.umask1 + q), dxur(a.dxur + q), dyur(a.dyur + q), thick(a.thicku + q);
+  const Loaded<EARLY, double> uo(a.ubt + (so * g.n2 + q)), vo(a.vbt + (so * g.n2 + q));
+  const Loaded<EARLY, double> fu(a.forcing_u + q), fv(a.forcing_v + q), cori1(a.cori1 + q), cori2(a.cori2 + q);
+  const Loaded<EARLY, double> dyu(a.dyu + q), dxu(a.dxu + q);
+  const double hf = half_exact(a.f[q]);  // 0.5*f; -0.5*f is its negation
+  if (EARLY) bt_after_previous();
   double gx = 0.0, gy = 0.0;
   if (i <= g.ni && j <= g.nj) {
     const double* ps = a.ps;
-    double um = a.umask1[q];
     if (!is_zero(um)) {
-      double p00 = ps[q], p10 = ps[I2(g, i + 1, j)], p01 = ps[I2(g, i, j + 1)], p11 = ps[I2(g, i + 1, j + 1)];
+      double p00 = ps[q], p10 = ps[q + 1], p01 = ps[q + g.nxd], p11 = ps[q + g.nxd + 1];
       double p_fay = half_exact(p00 + p01);
       double p_fax = half_exact(p00 + p10);
       double pip_fay = half_exact(p10 + p11);
       double pjp_fax = half_exact(p01 + p11);
-      gx = mask_mul((pip_fay - p_fay) * a.dxur[q], um);
-      gy = mask_mul((pjp_fax - p_fax) * a.dyur[q], um);
+      gx = mask_mul((pip_fay - p_fay) * dxur, um);
+      gy = mask_mul((pjp_fax - p_fax) * dyur, um);
     }
   }
-  double pf1 = -a.thicku[q] * gx;
-  double pf2 = -a.thicku[q] * gy;
-  double uo = a.ubt[so * g.n2 + q], vo = a.vbt[so * g.n2 + q];
-  double hf = half_exact(a.f[q]);  // 0.5*f; -0.5*f is its negation
-  double t1 = uo + bt_mul<INT>(a.dtbt, plus_zero(hf * vo + pf1 + a.forcing_u[q]));
-  double t2 = vo + bt_mul<INT>(a.dtbt, plus_zero((-hf) * uo + pf2 + a.forcing_v[q]));
-  double un = bt_mul<INT>(a.cori2[q], t1 + bt_mul<INT>(a.cori1[q], t2));
-  double vn = bt_mul<INT>(a.cori2[q], t2 - bt_mul<INT>(a.cori1[q], t1));
+  double pf1 = -thick * gx;
+  double pf2 = -thick * gy;
+  double t1 = uo + bt_mul<INT>(a.dtbt, plus_zero(hf * vo + pf1 + fu));
+  double t2 = vo + bt_mul<INT>(a.dtbt, plus_zero((-hf) * uo + pf2 + fv));
+  double un = bt_mul<INT>(cori2, t1 + bt_mul<INT>(cori1, t2));
+  double vn = bt_mul<INT>(cori2, t2 - bt_mul<INT>(cori1, t1));
   a.ubt[sn * g.n2 + q] = un;
   a.vbt[sn * g.n2 + q] = vn;
-  a.uhb[sn * g.n2 + q] = bt_mul<INT>(a.dyu[q], un);
-  a.vhb[sn * g.n2 + q] = bt_mul<INT>(a.dxu[q], vn);
+  a.uhb[sn * g.n2 + q] = bt_mul<INT>(dyu, un);
+  a.vhb[sn * g.n2 + q] = bt_mul<INT>(dxu, vn);
 }
 
 // C grid: Coriolis (compute domain) + gradient + momentum (:3780-3830), and the
 // halo update of the transports: the thread of a halo point with a periodic image
 // forms the image's value.  The transports times their areas over their lengths,
 // which the divergence takes (ocean_operators.F90:507-608), are stored beside them.
-template <bool INT>
+template <bool INT, bool EARLY>
 DEVI void bt_mom_c_body(BtArgs a, int so, int sn, int itime, int bx) {
+  if (!EARLY) bt_after_previous();
   const Geo& g = a.g;
   int i0, j0;
   if (!bt_point(g, bx, i0, j0)) return;
@@ -708,61 +712,68 @@ DEVI void bt_mom_c_body(BtArgs a, int so, int sn, int itime, int bx) {
   const long n2 = g.n2, q0 = I2(g, i0, j0), q = I2(g, i, j);
   const double abm0 = 23.0 / 12.0, abm1 = -16.0 / 12.0, abm2 = 5.0 / 12.0;
   const int m2 = (itime + 0) % 3, m1 = (itime + 1) % 3, m0 = (itime + 2) % 3;
-  double ca0 = 0.0, ca1 = 0.0;
-  if (i >= 1 && i <= g.ni && j >= 1 && j <= g.nj) {
-    double c0, c1;
+  double ca0 = 0.0, ca1 = 0.0, c0 = 0.0, c1 = 0.0;
+  const bool inside = i >= 1 && i <= g.ni && j >= 1 && j <= g.nj;
+  if (inside) {
     bt_coriolis_c<INT>(a, a.ubt + so * n2, a.vbt + so * n2, i, j, c0, c1);
-    if (q == q0) {
-      a.cf[(m0 * 2 + 0) * n2 + q] = c0;
-      a.cf[(m0 * 2 + 1) * n2 + q] = c1;
-    }
     ca0 = bt_mul<INT>(abm0, c0) + bt_mul<INT>(abm1, a.cf[(m1 * 2 + 0) * n2 + q]) + abm2 * a.cf[(m2 * 2 + 0) * n2 + q];
     ca1 = bt_mul<INT>(abm0, c1) + bt_mul<INT>(abm1, a.cf[(m1 * 2 + 1) * n2 + q]) + abm2 * a.cf[(m2 * 2 + 1) * n2 + q];
   }
-  const double te = a.tmen_e[q], tn = a.tmen_n[q];
+  const Loaded<EARLY, double> te(a.tmen_e + q), tn(a.tmen_n + q), dxter(a.dxter + q), dytnr(a.dytnr + q);
+  const Loaded<EARLY, double> the(a.thicken_e + q), thn(a.thicken_n + q), fu(a.forcing_u + q), fv(a.forcing_v + q);
+  const Loaded<EARLY, double> uo(a.ubt + (so * n2 + q)), vo(a.vbt + (so * n2 + q));
+  const Loaded<EARLY, double> dat0(a.dat + q0), dxter0(a.dxter + q0), dytnr0(a.dytnr + q0);
+  if (EARLY) bt_after_previous();
+  if (inside && q == q0) {
+    a.cf[(m0 * 2 + 0) * n2 + q] = c0;
+    a.cf[(m0 * 2 + 1) * n2 + q] = c1;
+  }
   double gx = 0.0, gy = 0.0;
   if (i <= g.ni && j <= g.nj) {
     const double p = a.ps[q];
-    gx = is_zero(te) ? 0.0 : mask_mul((a.ps[q + 1] - p) * a.dxter[q], te);
-    gy = is_zero(tn) ? 0.0 : mask_mul((a.ps[q + g.nxd] - p) * a.dytnr[q], tn);
+    gx = is_zero(te) ? 0.0 : mask_mul((a.ps[q + 1] - p) * dxter, te);
+    gy = is_zero(tn) ? 0.0 : mask_mul((a.ps[q + g.nxd] - p) * dytnr, tn);
   }
-  const double pf1 = bt_mul<INT, true>(-a.thicken_e[q], gx);
-  const double pf2 = bt_mul<INT, true>(-a.thicken_n[q], gy);
+  const double pf1 = bt_mul<INT, true>(-the, gx);
+  const double pf2 = bt_mul<INT, true>(-thn, gy);
   // dtbt*tmasken*(...): nothing is added where the mask is zero
-  const double su = ca0 + pf1 + a.forcing_u[q], sv = ca1 + pf2 + a.forcing_v[q];
+  const double su = ca0 + pf1 + fu, sv = ca1 + pf2 + fv;
   double du = bt_mul<INT>(a.dtbt, su), dv = bt_mul<INT>(a.dtbt, sv);
   rare_lanes(!(is_one(te) || is_zero(te)), [&] { du = a.dtbt * te * su; });
   rare_lanes(!(is_one(tn) || is_zero(tn)), [&] { dv = a.dtbt * tn * sv; });
-  const double un = a.ubt[so * n2 + q] + (is_zero(te) ? 0.0 : du);
-  const double vn = a.vbt[so * n2 + q] + (is_zero(tn) ? 0.0 : dv);
+  const double un = uo + (is_zero(te) ? 0.0 : du);
+  const double vn = vo + (is_zero(tn) ? 0.0 : dv);
   a.ubt[sn * n2 + q0] = un;
   a.vbt[sn * n2 + q0] = vn;
-  a.ca[q0] = bt_mul<INT>(un, a.dat[q0]) * a.dxter[q0];
-  a.ca[n2 + q0] = bt_mul<INT>(vn, a.dat[q0]) * a.dytnr[q0];
+  a.ca[q0] = bt_mul<INT>(un, dat0) * dxter0;
+  a.ca[n2 + q0] = bt_mul<INT>(vn, dat0) * dytnr0;
 }
 
 // C grid: the corrector of subcycle t and the predictor of subcycle t+1, which
 // reads only its own point's corrected eta and divergence (bt_corr_body's and
 // bt_pred_body's operations).
-template <bool INT>
+template <bool INT, bool EARLY>
 DEVI void bt_corr_pred_c_body(BtArgs a, int so, int sn, double wgt, int bx) {
+  if (!EARLY) bt_after_previous();
   const Geo& g = a.g;
   int i, j;
   if (!bt_point(g, bx, i, j)) return;
   const long n2 = g.n2, q = I2(g, i, j);
+  const Loaded<EARLY, double> tm(a.tmask1 + q), steady(a.steady + q), datr(a.datr + q), eo(a.eta_bt + (so * n2 + q));
+  const Loaded<EARLY, double> bar(a.eta_bar + q), su(a.udrho_u + q), sv(a.udrho_v + q), rho_g(a.rho_g + q), patm(a.patm + q);
+  if (EARLY) bt_after_previous();
+  const double un = a.ubt[sn * n2 + q], vn = a.vbt[sn * n2 + q];
   double dv = 0.0;
   if (i >= 1 && j >= 1)
-    dv = bt_mul<INT>(a.datr[q], (a.ca[q] - a.ca[q - 1]) + (a.ca[n2 + q] - a.ca[n2 + q - g.nxd]));
-  const double tm = a.tmask1[q];
-  const double st = (is_zero(tm) ? 0.0 : mask_mul(-dv, tm)) + a.steady[q];
-  const double en = a.eta_bt[so * n2 + q] + bt_mul<INT>(a.dtbt_rho0r, st);
+    dv = bt_mul<INT>(datr, (a.ca[q] - a.ca[q - 1]) + (a.ca[n2 + q] - a.ca[n2 + q - g.nxd]));
+  const double st = (is_zero(tm) ? 0.0 : mask_mul(-dv, tm)) + steady;
+  const double en = eo + bt_mul<INT>(a.dtbt_rho0r, st);
   a.eta_bt[sn * n2 + q] = en;
-  a.eta_bar[q] = a.eta_bar[q] + en;
-  const double un = a.ubt[sn * n2 + q], vn = a.vbt[sn * n2 + q];
-  a.udrho_u[q] = a.udrho_u[q] + (a.stepB ? bt_mul<INT>(wgt, un) : un);
-  a.udrho_v[q] = a.udrho_v[q] + (a.stepB ? bt_mul<INT>(wgt, vn) : vn);
+  a.eta_bar[q] = bar + en;
+  a.udrho_u[q] = su + (a.stepB ? bt_mul<INT>(wgt, un) : un);
+  a.udrho_v[q] = sv + (a.stepB ? bt_mul<INT>(wgt, vn) : vn);
   const double ep = dpos(a.gamma) ? en + a.dtbt_gamma_rho0r * st : en;
-  a.ps[q] = a.rho_g[q] * ep + a.patm[q];
+  a.ps[q] = rho_g * ep + patm;
 }
 
 // corrector + accumulation
@@ -772,7 +783,7 @@ DEVI void bt_corr_body(BtArgs a, int so, int sn, double wgt, int bx) {
   if (!bt_point(g, bx, i, j)) return;
   long q = I2(g, i, j);
   double dv = a.cgrid ? div_ud(a, a.ubt + sn * g.n2, a.vbt + sn * g.n2, i, j)
-                      : div_ud_bh(a, a.uhb + sn * g.n2, a.vhb + sn * g.n2, i, j);
+                      : div_ud_bh(g, a.datr[I2(g, i, j)], a.uhb + sn * g.n2, a.vhb + sn * g.n2, i, j);
   a.dvs[q] = dv;
   double tm = a.tmask1[q];
   double tmp = is_zero(tm) ? 0.0 : mask_mul(-dv, tm);
@@ -797,32 +808,30 @@ DEVI void bt_corr_body(BtArgs a, int so, int sn, double wgt, int bx) {
 // at the periodic halo points whose image it is.  The predicted eta is not
 // stored (the next corrector overwrites it unread), nor is the divergence.  The
 // operations are bt_corr_body's and bt_pred_body's, so the bits are theirs.
-template <bool INT = false>
+template <bool INT = false, bool EARLY = false>
 DEVI void bt_corr_pred_body(BtArgs a, int so, int sn, double wgt, int bx) {
+  if (!EARLY) bt_after_previous();
   const Geo& g = a.g;
   int i, j;
   if (!bt_point(g, bx, i, j)) return;
   const long n2 = g.n2;
   long q = I2(g, i, j);
-  double dv = div_ud_bh<INT>(a, a.uhb + sn * n2, a.vhb + sn * n2, i, j);
-  double tm = a.tmask1[q];
+  const Loaded<EARLY, double> tm(a.tmask1 + q), steady(a.steady + q), datr(a.datr + q), eo(a.eta_bt + (so * n2 + q));
+  const Loaded<EARLY, double> bar(a.eta_bar + q), su(a.udrho_u + q), sv(a.udrho_v + q), rho_g(a.rho_g + q), patm(a.patm + q);
+  if (EARLY) bt_after_previous();
+  const double un = a.ubt[sn * n2 + q], vn = a.vbt[sn * n2 + q];
+  double dv = div_ud_bh<INT>(g, datr, a.uhb + sn * n2, a.vhb + sn * n2, i, j);
   double tmp = is_zero(tm) ? 0.0 : mask_mul(-dv, tm);
-  const double st = tmp + a.steady[q];
-  double en = a.eta_bt[so * n2 + q] + bt_mul<INT>(a.dtbt_rho0r, st);
+  const double st = tmp + steady;
+  double en = eo + bt_mul<INT>(a.dtbt_rho0r, st);
   a.eta_bt[sn * n2 + q] = en;
-  a.eta_bar[q] = a.eta_bar[q] + en;
-  double un = a.ubt[sn * n2 + q], vn = a.vbt[sn * n2 + q];
-  if (a.stepB) {
-    a.udrho_u[q] = a.udrho_u[q] + bt_mul<INT>(wgt, un);
-    a.udrho_v[q] = a.udrho_v[q] + bt_mul<INT>(wgt, vn);
-  } else {
-    a.udrho_u[q] = a.udrho_u[q] + un;
-    a.udrho_v[q] = a.udrho_v[q] + vn;
-  }
+  a.eta_bar[q] = bar + en;
+  a.udrho_u[q] = su + (a.stepB ? bt_mul<INT>(wgt, un) : un);
+  a.udrho_v[q] = sv + (a.stepB ? bt_mul<INT>(wgt, vn) : vn);
   // the next subcycle's predictor (bt_pred_body with reuse)
   const double ep = dpos(a.gamma) ? en + a.dtbt_gamma_rho0r * st : en;
   int ii = i, jj = j;
-  if (!halo_image(g, ii, jj) || (ii == i && jj == j)) a.ps[q] = a.rho_g[q] * ep + a.patm[q];
+  if (!halo_image(g, ii, jj) || (ii == i && jj == j)) a.ps[q] = rho_g * ep + patm;
   if (i < 1 || i > g.ni || j < 1 || j > g.nj) return;
   int hx[2], nhx = 0, hy[2], nhy = 0;  // periodic halo points whose image this is
   if (g.cx) {
@@ -884,7 +893,7 @@ DEVI void bt_fused_body(BtArgs a, int so, int sn, int reuse, double wgt, int bx,
     const long q = I2(g, i, j);
     double en;
     if (dpos(a.gamma)) {
-      double dv = reuse ? dvs_o[q] : div_ud_bh(a, a.uhb + so * n2, a.vhb + so * n2, i, j);
+      double dv = reuse ? dvs_o[q] : div_ud_bh(g, a.datr[I2(g, i, j)], a.uhb + so * n2, a.vhb + so * n2, i, j);
       double tm = a.tmask1[q];
       double tmp = is_zero(tm) ? 0.0 : mask_mul(-dv, tm);
       en = eo[q] + a.dtbt_gamma_rho0r * (tmp + a.steady[q]);

@@ -286,6 +286,25 @@ __device__ __forceinline__ bool bt_point(const Geo& g, int block, int& i, int& j
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The start of a subcycle kernel; with EARLY it stands between the loads of what the
+// launch before does not write and the rest, so that their latency overlaps the end
+// of that launch.  (The launch before waited for the one before it before it allowed
+// this one: pdl_trigger comes after pdl_wait everywhere.)
+__device__ __forceinline__ void bt_after_previous() {
+  pdl_wait();
+  pdl_trigger();
+}
+// A value loaded where it is declared (EARLY) or, to hold no register until then,
+// where it is used.
+template <bool EARLY, class T>
+struct Loaded {
+  const T* p;
+  T v;
+  __device__ __forceinline__ explicit Loaded(const T* q) : p(q) {
+    if (EARLY) v = *q;
+  }
+  __device__ __forceinline__ operator T() const { return EARLY ? v : *p; }
+};
 #endif
 template <typename... P, typename... A>
 cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
@@ -307,6 +326,17 @@ cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, A
 // columns 0.65 and 0.74 ms, 300x260 0.99 and 1.14, 360x300 1.23 and 1.10; C grid, 48
 // subcycles, 361x243 0.68 and 0.60; 60 subcycles, 1440x1080 9.81 and 8.17.
 inline bool bt_int_products(long columns) { return columns >= 85000; }
+// Whether the subcycle kernels load early (bt_after_previous).  With the registers
+// that takes, the waiting blocks of one launch and the running ones of the launch
+// before fit an SM together up to about 92000 columns (90x60 columns, 80 subcycles:
+// 0.65 -> 0.45 ms alone; C grid 361x243 0.62 -> 0.60); past that the waiting ones come to
+// the SMs that end first, which a launch of one round pays for (360x300: 1.12 -> 1.38 ms)
+// and one of several does not (1440x1080, precision form, 60 subcycles: 4.28 -> 3.88).
+inline bool bt_early_loads(long columns) { return columns <= 92000 || columns >= 300000; }
+// the instantiation <INT, EARLY> of a subcycle kernel for so many columns
+#define BT_VARIANT(K, columns)                                                             \
+  (bt_int_products(columns) ? (bt_early_loads(columns) ? K<true, true> : K<true, false>)   \
+                            : (bt_early_loads(columns) ? K<false, true> : K<false, false>))
 // Threads and blocks of a 2-D barotropic launch of one domain: small blocks while
 // they fit the SMs in one round (360x300: 1.10 ms with 64 threads, 1.12 with 128, 1.34
 // with 32, of which an SM holds too few).

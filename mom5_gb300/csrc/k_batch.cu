@@ -32,11 +32,10 @@ __global__ void __launch_bounds__(128) kb_btf_pred(const BtArgs* d, BatchWork w,
   BTF_ENTRY
   btfast::pred_body(a, so, sn, reuse, bx);
 }
+template <bool EARLY>
 __global__ void __launch_bounds__(128) kb_btf_mom(const BtArgs* d, BatchWork w, int so, int sn, double wgt) {
-  pdl_wait();
-  pdl_trigger();
   BTF_ENTRY
-  btfast::mom_body(a, so, sn, wgt, bx);
+  btfast::mom_body<EARLY>(a, so, sn, wgt, bx);
 }
 __global__ void __launch_bounds__(128) kb_btf_corr(const BtArgs* d, BatchWork w, int so, int sn) {
   pdl_wait();
@@ -44,11 +43,10 @@ __global__ void __launch_bounds__(128) kb_btf_corr(const BtArgs* d, BatchWork w,
   BTF_ENTRY
   btfast::corr_body(a, so, sn, bx);
 }
+template <bool EARLY>
 __global__ void __launch_bounds__(128) kb_btf_corr_pred(const BtArgs* d, BatchWork w, int so, int sn) {
-  pdl_wait();
-  pdl_trigger();
   BTF_ENTRY
-  btfast::corr_pred_body(a, so, sn, bx);
+  btfast::corr_pred_body<EARLY>(a, so, sn, bx);
 }
 
 }  // namespace
@@ -65,9 +63,10 @@ int launch_batch_btf_subcycle(const BtArgs* bt, const BatchWork& w, int itime, i
   const int so = itime % 2, sn = (itime + 1) % 2;
   const double wgt = (double)(nts - itime + 1);
   const dim3 g2(w.tb2), b(128);
+  const bool early = bt_early_loads(128L * w.tb2);
   if (itime == 1) launch_pdl(kb_btf_pred, g2, b, s, bt, w, so, sn, 0);
-  launch_pdl(kb_btf_mom, g2, b, s, bt, w, so, sn, wgt);
-  if (itime < nts) launch_pdl(kb_btf_corr_pred, g2, b, s, bt, w, so, sn);
+  launch_pdl(early ? kb_btf_mom<true> : kb_btf_mom<false>, g2, b, s, bt, w, so, sn, wgt);
+  if (itime < nts) launch_pdl(early ? kb_btf_corr_pred<true> : kb_btf_corr_pred<false>, g2, b, s, bt, w, so, sn);
   else launch_pdl(kb_btf_corr, g2, b, s, bt, w, so, sn);
   return itime == 1 ? 3 : 2;
 }

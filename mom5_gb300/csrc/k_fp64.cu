@@ -1306,34 +1306,26 @@ __global__ void k_bt_pred(BtArgs a, int so, int sn, int reuse) {
   pdl_trigger();
   bt_pred_body(a, so, sn, reuse, blockIdx.x);
 }
-template <bool INT>
+template <bool INT, bool EARLY>
 __global__ void k_bt_mom_b(BtArgs a, int so, int sn) {
-  pdl_wait();
-  pdl_trigger();
-  bt_mom_b_body<INT>(a, so, sn, blockIdx.x);
+  bt_mom_b_body<INT, EARLY>(a, so, sn, blockIdx.x);
 }
-template <bool INT>
+template <bool INT, bool EARLY>
 __global__ void k_bt_mom_c(BtArgs a, int so, int sn, int itime) {
-  pdl_wait();
-  pdl_trigger();
-  bt_mom_c_body<INT>(a, so, sn, itime, blockIdx.x);
+  bt_mom_c_body<INT, EARLY>(a, so, sn, itime, blockIdx.x);
 }
-template <bool INT>
+template <bool INT, bool EARLY>
 __global__ void k_bt_corr_pred_c(BtArgs a, int so, int sn, double wgt) {
-  pdl_wait();
-  pdl_trigger();
-  bt_corr_pred_c_body<INT>(a, so, sn, wgt, blockIdx.x);
+  bt_corr_pred_c_body<INT, EARLY>(a, so, sn, wgt, blockIdx.x);
 }
 __global__ void k_bt_corr(BtArgs a, int so, int sn, double wgt) {
   pdl_wait();
   pdl_trigger();
   bt_corr_body(a, so, sn, wgt, blockIdx.x);
 }
-template <bool INT>
+template <bool INT, bool EARLY>
 __global__ void k_bt_corr_pred(BtArgs a, int so, int sn, double wgt) {
-  pdl_wait();
-  pdl_trigger();
-  bt_corr_pred_body<INT>(a, so, sn, wgt, blockIdx.x);
+  bt_corr_pred_body<INT, EARLY>(a, so, sn, wgt, blockIdx.x);
 }
 // 32 x 8 tiles of 352 threads: one point per thread in each phase (the 34 x 10
 // pressure ring is the largest); 64 x 8 tiles of 256 threads, several points
@@ -1661,7 +1653,6 @@ int launch_barotropic(mom5gpu_domain* d, int tau, int taup1) {
                                                           esm, d->opt.initsum_with_bar);
   const int bt = bt_threads(g);
   const dim3 g2 = bt_grid(g, bt);
-  const bool bint = bt_int_products(n2);
   if (a.cgrid) {
     dim3 gc((g.ni + 127) / 128, g.nj);
     k_bt_cgrid_init<<<gc, 128, 0, s>>>(a);
@@ -1686,13 +1677,13 @@ int launch_barotropic(mom5gpu_domain* d, int tau, int taup1) {
       const double wgt = (double)(a.nts - itime + 1);
       if (itime == 1) launch_pdl(k_bt_pred, g2, dim3(bt), st, a, so, sn, 0);
       if (a.cgrid) {
-        launch_pdl(bint ? k_bt_mom_c<true> : k_bt_mom_c<false>, g2, dim3(bt), st, a, so, sn, itime);
-        launch_pdl(bint ? k_bt_corr_pred_c<true> : k_bt_corr_pred_c<false>, g2, dim3(bt), st, a, so, sn, wgt);
+        launch_pdl(BT_VARIANT(k_bt_mom_c, n2), g2, dim3(bt), st, a, so, sn, itime);
+        launch_pdl(BT_VARIANT(k_bt_corr_pred_c, n2), g2, dim3(bt), st, a, so, sn, wgt);
         continue;
       }
-      launch_pdl(bint ? k_bt_mom_b<true> : k_bt_mom_b<false>, g2, dim3(bt), st, a, so, sn);
+      launch_pdl(BT_VARIANT(k_bt_mom_b, n2), g2, dim3(bt), st, a, so, sn);
       if (itime < a.nts)
-        launch_pdl(bint ? k_bt_corr_pred<true> : k_bt_corr_pred<false>, g2, dim3(bt), st, a, so, sn, wgt);
+        launch_pdl(BT_VARIANT(k_bt_corr_pred, n2), g2, dim3(bt), st, a, so, sn, wgt);
       else launch_pdl(k_bt_corr, g2, dim3(bt), st, a, so, sn, wgt);
     }
   };
@@ -1742,7 +1733,7 @@ int launch_barotropic_phase(mom5gpu_domain* d, int tau, int taup1, int phase, in
       count_launches(d, 1);
       break;
     case 2:
-      k_bt_mom_b<false><<<g2, 128, 0, s>>>(a, so, sn);
+      k_bt_mom_b<false, false><<<g2, 128, 0, s>>>(a, so, sn);
       k_bt_corr<<<g2, 128, 0, s>>>(a, so, sn, (double)(a.nts - itime + 1));
       count_launches(d, 2);
       break;

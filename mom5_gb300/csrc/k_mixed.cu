@@ -12,20 +12,18 @@ __global__ void __launch_bounds__(128) k_btf_pred(BtArgs a, int so, int sn, int 
   pdl_trigger();
   btfast::pred_body(a, so, sn, reuse, blockIdx.x);
 }
+template <bool EARLY>
 __global__ void __launch_bounds__(128) k_btf_mom(BtArgs a, int so, int sn, double wgt) {
-  pdl_wait();
-  pdl_trigger();
-  btfast::mom_body(a, so, sn, wgt, blockIdx.x);
+  btfast::mom_body<EARLY>(a, so, sn, wgt, blockIdx.x);
 }
 __global__ void __launch_bounds__(128) k_btf_corr(BtArgs a, int so, int sn) {
   pdl_wait();
   pdl_trigger();
   btfast::corr_body(a, so, sn, blockIdx.x);
 }
+template <bool EARLY>
 __global__ void __launch_bounds__(128) k_btf_corr_pred(BtArgs a, int so, int sn) {
-  pdl_wait();
-  pdl_trigger();
-  btfast::corr_pred_body(a, so, sn, blockIdx.x);
+  btfast::corr_pred_body<EARLY>(a, so, sn, blockIdx.x);
 }
 
 void launch_btf_prep(const BtArgs& a, cudaStream_t s) {
@@ -60,9 +58,10 @@ int launch_btf_subcycle(const BtArgs& a, int itime, int nts, bool fused, cudaStr
     return 1;
   }
   const dim3 b(bt_threads(a.g)), g2 = bt_grid(a.g, b.x);
+  const bool early = bt_early_loads(a.g.n2);
   if (itime == 1) launch_pdl(k_btf_pred, g2, b, s, a, so, sn, 0);
-  launch_pdl(k_btf_mom, g2, b, s, a, so, sn, wgt);
-  if (itime < nts) launch_pdl(k_btf_corr_pred, g2, b, s, a, so, sn);
+  launch_pdl(early ? k_btf_mom<true> : k_btf_mom<false>, g2, b, s, a, so, sn, wgt);
+  if (itime < nts) launch_pdl(early ? k_btf_corr_pred<true> : k_btf_corr_pred<false>, g2, b, s, a, so, sn);
   else launch_pdl(k_btf_corr, g2, b, s, a, so, sn);
   return itime == 1 ? 3 : 2;
 }
