@@ -293,6 +293,15 @@ DEVI double tx_halo(const MdflArgs& a, int n, int i, int j, int k) {
 // would cost a warp of its own, all of a face's FP64 instructions for one lane
 // (360x270x50, 10 tracers: 1.39 -> 1.12 ms).
 constexpr int kTX = 128, kXCells = kTX - 1;
+// Blocks of 128 threads per SM that the x and y passes of more than two tracers keep
+// registers for (48 and 72): the FP64 pipe's latency wants the warps (360x270x50, 10
+// tracers: x 1.19 ms with the compiler's 68 registers, 1.07 with 48; y 2.12 with 74,
+// 2.10 with 72; the z pass, whose columns give 5 blocks per SM, gains nothing, nor do
+// small domains: 37x29x12, 2 tracers 12.7 us a step without, 13.2 with).
+template <int MAXN>
+constexpr int kXBlocks = MAXN > 2 ? 10 : 1;
+template <int MAXN>
+constexpr int kYBlocks = MAXN > 2 ? 7 : 6;
 __host__ __device__ inline int x_blocks(const Geo& g) { return (g.ni + kXCells - 1) / kXCells; }
 
 // x-face i of row (j,k): fluxes of every tracer into sm[n][slot].  Rs[n][r-1..r+1]

@@ -141,7 +141,7 @@ int y_strip_rows(long cols, long nj) {
 }
 
 template <bool ALL, bool SWEBY, int MAXN, bool SPLIT>
-__global__ void __launch_bounds__(kTX) k_mdfl_x(MdflArgs a) {
+__global__ void __launch_bounds__(kTX, kXBlocks<MAXN>) k_mdfl_x(MdflArgs a) {
   pdl_wait();
   pdl_trigger();
   const int nk = a.g.nk;
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kTX) k_mdfl_x(MdflArgs a) {
 }
 
 template <bool ALL, bool SWEBY, int MAXN, bool SPLIT>
-__global__ void __launch_bounds__(128, 6) k_mdfl_y(MdflArgs a, int TJ) {
+__global__ void __launch_bounds__(128, kYBlocks<MAXN>) k_mdfl_y(MdflArgs a, int TJ) {
   pdl_wait();
   pdl_trigger();
   const int nk = a.g.nk;
