@@ -482,8 +482,8 @@ int mom5gpu_batch_step(mom5gpu_batch* b, const int* index, const int* parity, in
  * overwritten.  A summary is written to report (may be NULL). */
 int mom5gpu_batch_autotune(mom5gpu_batch* b, double dtime, char* report, size_t report_len);
 /* Read or set the launch shape directly (e.g. to reuse one autotune result on
- * several batches): rows = precision-form tile height (16 or 24; 32: 16 rows up
- * to 4 tracers, else 20), tj = FP64 y-pass rows per thread (0 = automatic, else
+ * several batches): rows = precision-form tile height (16 or 24; 32: 16, 20 or
+ * 24 by the number of tracers), tj = FP64 y-pass rows per thread (0 = automatic, else
  * 2, 4, 8 or 16), blocks_per_sm = most resident blocks per SM of the precision
  * form's persistent launch (1..4). */
 int mom5gpu_batch_get_tuning(const mom5gpu_batch* b, int* rows, int* tj, int* blocks_per_sm);

@@ -120,7 +120,7 @@ void fill_work(const mom5gpu_batch* b, const std::vector<std::pair<int, int>>& l
   int* pr[6];
   for (int k = 0; k < 6; ++k) pr[k] = ent + c + k * (c + 1);
   // the precision form's tiles are cut into segments of one length, chosen for all of them together
-  const int rows = stream_tile_rows(b->rows, b->ntr);
+  const int rows = stream_tile_rows(b->rows, b->ntr, true);
   long tiles = 0;
   int nk = 1;
   for (auto& it : list) {

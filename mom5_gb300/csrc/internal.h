@@ -396,7 +396,7 @@ void launch_batch_barotropic_post(const BtArgs* bt, const BtExtra* x, const Batc
 // ---- precision-form advection (k_mixed_stream.cu) ----
 // tile height of a tuning value (16, 24, or by the tracer count), a domain's tiles
 // of that height, and the levels per segment for a launch of so many tiles
-int stream_tile_rows(int tuned, int ntr);
+int stream_tile_rows(int tuned, int ntr, bool batch);
 long stream_tiles(const Geo& g, int rows);
 int stream_levels(long tiles, int nk, int ntr, int rows);
 // the tracers of a (at most 10) of one domain, outputs numbered from n0

@@ -16,6 +16,12 @@ namespace {
 // of 20 rows (96 registers) is the largest without spills: 1440x1080x50, 10
 // tracers, 7.10 ms against 7.54 with 16 rows and 8.43 with 24.
 constexpr int stream_rows(int np) { return np <= 2 ? 16 : 20; }
+// The same for the persistent kernel, whose registers hold its work list too: a height
+// that spills there pays for each spill with a trip to L2, as the tiles leave no L1
+// (a step of 8 domains, precision form with 40 subcycles: 4 tracers 1.42 ms with 24
+// rows, 2.00 with 16; 9 tracers 2.06 with 16, 3.03 with 20, 3.21 with 24; 6 tracers 1.65
+// with 20, 1.73 with 16, 1.93 with 24; 2 tracers 1.25 with 16, 1.26 with 24).
+constexpr int stream_batch_rows(int np) { return np == 2 ? 24 : np == 3 ? 20 : 16; }
 constexpr int stream_blocks(int np, int rows) { return np <= 2 && rows == 16 ? 2 : 1; }
 
 template <int NP, int ZR>
@@ -110,8 +116,9 @@ int configure_batch_rows() {
 
 }  // namespace
 
-int stream_tile_rows(int tuned, int ntr) {
-  return tuned == 16 || tuned == 24 ? tuned : stream_rows((ntr + 1) / 2);
+int stream_tile_rows(int tuned, int ntr, bool batch) {
+  const int np = (ntr + 1) / 2;
+  return tuned == 16 || tuned == 24 ? tuned : batch ? stream_batch_rows(np) : stream_rows(np);
 }
 
 long stream_tiles(const Geo& g, int rows) { return tiles_of(g, rows); }
@@ -142,7 +149,7 @@ int stream_levels(long tiles, int nk, int ntr, int rows) {
 }
 
 int launch_mixed_stream(mom5gpu_domain* d, const MixArgs& a, int n0) {
-  const int ntr = a.ntr, rows = stream_tile_rows(d->tune_mixed_rows, ntr);
+  const int ntr = a.ntr, rows = stream_tile_rows(d->tune_mixed_rows, ntr, false);
   return STREAM_DISPATCH(run, d, a, n0);
 }
 
@@ -156,7 +163,7 @@ int prepare_batch_mixed() {
 int launch_batch_mixed(const MixArgs* mix, const BatchWork& w, int ntr, int tuned_rows, int blocks_per_sm, int sms,
                        int* counter, cudaStream_t s) {
   if (w.tm <= 0) return MOM5GPU_OK;
-  const int rows = stream_tile_rows(tuned_rows, ntr);
+  const int rows = stream_tile_rows(tuned_rows, ntr, true);
   return STREAM_DISPATCH(run_batch, mix, w, blocks_per_sm, sms, counter, s);
 }
 
