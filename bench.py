@@ -93,21 +93,20 @@ def adv_bytes(ni, nj, nk, ntr):
 
 
 # DRAM bytes per tracer-cell of the advection launch set from ncu captures: FP64, the
-# 360x270x50 block (4.740 GB for 360*270*50*10 tracer-cells); precision form, the TMA-staged
-# kernel (the launch shape chosen on C2) on the 1440x360x50 band, 10.3 waves (6.099 GB for
-# 1440*360*50*10 tracer-cells).
-TRAFFIC_PER_TRACER_CELL = {"fp64": 4.740e9 / (360 * 270 * 50 * 10), "mixed": 6.099e9 / (1440 * 360 * 50 * 10)}
+# 360x270x50 block (4.012 GB for 360*270*50*10 tracer-cells); precision form, the tile
+# kernel on the 1440x360x50 band (5.865 GB for 1440*360*50*10 tracer-cells).
+TRAFFIC_PER_TRACER_CELL = {"fp64": 4.012e9 / (360 * 270 * 50 * 10), "mixed": 5.865e9 / (1440 * 360 * 50 * 10)}
 TRAFFIC_SOURCE = {"fp64": "ncu DRAM bytes of the advection launch set on a 360x270x50 block, scaled by tracer-cells",
-                  "mixed": "ncu DRAM bytes of the TMA-staged kernel on a 1440x360x50 band, scaled by tracer-cells"}
+                  "mixed": "ncu DRAM bytes of the tile kernel on a 1440x360x50 band, scaled by tracer-cells"}
 
 
-# FP64 thread-instructions per tracer-cell of the exact MDFL passes (z + x + y) and per
-# column of one exact barotropic subcycle (momentum 29.7 + corrector with the next
-# predictor 21.0 in the steady state; 50.8 averaged over a 60-subcycle step with its
-# first predictor and last corrector), counted by ncu on the 360x270x50 block; the
-# FP64 instruction rate of GB300 measured with a probe kernel.
-FP64_OPS_PER_TRACER_CELL = 62.4
-FP64_OPS_PER_COLUMN_SUBCYCLE = 50.8
+# FP64 instructions (per thread of a warp that issues one) per tracer-cell of the exact
+# MDFL passes (z 10.8, x 10.5, y with the explicit update 18.6) and per column of one
+# exact barotropic subcycle (momentum 20.4, corrector with the next predictor 17.9),
+# counted by ncu on the 360x270x50 block and on 360x300 columns; the FP64 instruction
+# rate of GB300 measured with a probe kernel.
+FP64_OPS_PER_TRACER_CELL = 40.0
+FP64_OPS_PER_COLUMN_SUBCYCLE = 38.3
 FP64_PEAK_OPS = 5.05e11
 
 

@@ -1658,7 +1658,7 @@ int launch_barotropic(mom5gpu_domain* d, int tau, int taup1) {
     k_bt_cgrid_init<<<gc, 128, 0, s>>>(a);
   }
   if (a.btf) launch_btf_prep(a, s);
-  // the nts subcycles (3 to 5 launches each, all arguments in a): one CUDA graph,
+  // the nts subcycles (2 launches each, all arguments in a): one CUDA graph,
   // captured on first use and replayed while a is unchanged
   const dim3 gf((g.ni + 2 + kFusedTX - 1) / kFusedTX, (g.nj + 2 + kFusedTY - 1) / kFusedTY);
   auto subcycles = [&](cudaStream_t st) {
