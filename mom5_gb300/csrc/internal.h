@@ -88,7 +88,7 @@ struct mom5gpu_domain {
   size_t mixed_cap = 0;
   double* bt = nullptr;        // barotropic scratch
   int* kmt_d = nullptr;        // device copy of kmt (uploaded on first use)
-  double* psom_scr = nullptr;  // PSOM mass and x/y/z face fluxes, 4 x n3
+  double* psom_scr = nullptr;  // PSOM mass and x/y/z face fluxes, 4 x n3; cells beside the segments
   long itt0 = 0;               // Time%itt0 (orders the PSOM sweeps)
   double* red = nullptr;       // reduction scratch (device)
   double* red_h = nullptr;     // pinned host result

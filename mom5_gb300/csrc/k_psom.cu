@@ -15,6 +15,9 @@
 // moments of the faces it is upstream of in shared memory and, after one
 // barrier, applies the inflows.  The two end threads of a segment run the
 // outflow of the neighbouring cells only to supply the segment's end faces.
+// Those cells belong to the line's other segments, whose blocks update them in
+// place at any time: on a line of several segments their state before the sweep
+// is copied first (k_psom_edges) and read from the copy.
 // A periodic direction is a ring (the halo update makes each halo cell a copy
 // of its image before it is used), and the boundary face of a closed direction
 // carries nothing: its velocity is masked to zero, which makes the halo cell
@@ -60,6 +63,8 @@ struct Args {
   const double *tmask, *dat, *datr, *dxtn, *dyte, *uh, *vh, *w, *rdz, *T;
   double *sm, *s0;
   double* mr[NROLE];  // the moments in role order for this direction
+  double* edge;       // state before the sweep of the cells beside each segment (Edge)
+  int nseg;           // segments per line
   double *fx, *fy, *fz;
   double* th;
 };
@@ -278,10 +283,69 @@ struct Line {
   }
 };
 
-// Both sweeps of one direction for segments of L-2 cells on BI lines; 24 warps per
+// Copy of the state next to the segments of a line: 2*nseg cells per line (2*seg: the
+// one below segment seg, 2*seg + 1: the one above), NEDGE values each (NROLE moments, the
+// mass and s0), along x a line's values together, else those of the lines along i.
+constexpr int NEDGE = NROLE + 2;
+template <int DIR>
+struct Edge {
+  long at;      // first value
+  long stride;  // from one value to the next
+  DEVI Edge(const Geo& g, int nseg, int i, int j, int k, int h) {
+    if (DIR == 1) {
+      at = (((long)k * g.nj + (j - 1)) * (2 * nseg) + h) * NEDGE;
+      stride = 1;
+    } else {
+      stride = (long)g.ni * (DIR == 2 ? g.nk : g.nj);
+      at = (long)h * NEDGE * stride + (long)(DIR == 2 ? k : j - 1) * g.ni + (i - 1);
+    }
+  }
+};
+static size_t edge_values(const Geo& g, int dir, int nseg) {
+  const size_t lines = dir == 1 ? (size_t)g.nj * g.nk : dir == 2 ? (size_t)g.ni * g.nk : (size_t)g.ni * g.nj;
+  return nseg > 1 ? lines * 2 * nseg * NEDGE : 0;
+}
+
+// One thread per copied cell; grid y (x sweep: threads) over the 2*nseg cells of a line.
+template <int DIR, int L>
+__global__ void __launch_bounds__(128) k_psom_edges(Args a) {
+  const Geo& g = a.g;
+  const long id = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  int i = 0, j = 0, k = 0, h;
+  if (DIR == 1) {
+    const long line = id / (2 * a.nseg);
+    h = (int)(id - line * (2 * a.nseg));
+    k = (int)(line / g.nj);
+    j = (int)(line - (long)k * g.nj) + 1;
+    if (k >= g.nk) return;
+  } else {
+    const int o = (int)(id / g.ni);
+    i = (int)(id - (long)o * g.ni) + 1;
+    h = blockIdx.y;
+    if (o >= (DIR == 2 ? g.nk : g.nj)) return;
+    if (DIR == 2) k = o;
+    else j = o + 1;
+  }
+  const Line<DIR> ln(g, i, j, k);
+  const int s0 = (h >> 1) * (L - 2);
+  int s = s0, sc = 0;
+  if (h & 1) s = s0 + L - 1 < ln.N + 1 ? s0 + L - 1 : ln.N + 1;
+  if (!ln.cell(s, sc)) return;  // beyond a closed edge: no state, and none is read
+  const long p = ln.index(sc);
+  const Edge<DIR> e(g, a.nseg, i, j, k, h);
+#pragma unroll
+  for (int r = 0; r < NROLE; ++r) a.edge[e.at + r * e.stride] = a.mr[r][p];
+  if (!a.first) {
+    a.edge[e.at + NROLE * e.stride] = a.sm[p];
+    a.edge[e.at + (NROLE + 1) * e.stride] = a.s0[p];
+  }
+}
+
+// Both sweeps of one direction for segments of L-2 cells on BI lines (SEG: more than
+// one per line, whose neighbouring cells come from the copy); 24 warps per
 // SM (80 registers) in blocks of 128 threads (121x30x30: 290 us a step alone against 310
 // with the compiler's 88 to 96 registers, 322 in blocks of 512).
-template <int DIR, int BI, int L>
+template <int DIR, int BI, int L, bool SEG>
 __global__ void __launch_bounds__(BI* L, 768 / (BI * L)) k_psom_dir(Args a) {
   __shared__ double slot[NF][L - 1][BI];
   const Geo& g = a.g;
@@ -309,13 +373,20 @@ __global__ void __launch_bounds__(BI* L, 768 / (BI * L)) k_psom_dir(Args a) {
       long q = DIR == 1 ? I2(g, sc, j) : DIR == 2 ? I2(g, i, sc) : I2(g, i, j);
       c.sm = a.rdz[p] * a.dat[q];
       c.s0 = a.T[p] * c.sm * a.tmask[p];
-    } else {
-      c.sm = a.sm[p];
-      c.s0 = a.s0[p];
     }
-    c.a = a.mr[RA][p], c.aa = a.mr[RAA][p], c.b1 = a.mr[RB1][p], c.b2 = a.mr[RB2][p];
-    c.c1 = a.mr[RC1][p], c.c2 = a.mr[RC2][p], c.bb1 = a.mr[RBB1][p], c.bb2 = a.mr[RBB2][p];
-    c.bc = a.mr[RBC][p];
+    if (SEG && (t < 1 || t > L - 2 || s > ln.N)) {  // not this segment's cell
+      const Edge<DIR> e(g, a.nseg, i, j, k, 2 * seg + (t < 1 ? 0 : 1));
+      auto at = [&](int v) { return a.edge[e.at + v * e.stride]; };
+      if (!a.first) c.sm = at(NROLE), c.s0 = at(NROLE + 1);
+      c.a = at(RA), c.aa = at(RAA), c.b1 = at(RB1), c.b2 = at(RB2);
+      c.c1 = at(RC1), c.c2 = at(RC2), c.bb1 = at(RBB1), c.bb2 = at(RBB2);
+      c.bc = at(RBC);
+    } else {
+      if (!a.first) c.sm = a.sm[p], c.s0 = a.s0[p];
+      c.a = a.mr[RA][p], c.aa = a.mr[RAA][p], c.b1 = a.mr[RB1][p], c.b2 = a.mr[RB2][p];
+      c.c1 = a.mr[RC1][p], c.c2 = a.mr[RC2][p], c.bb1 = a.mr[RBB1][p], c.bb2 = a.mr[RBB2][p];
+      c.bc = a.mr[RBC][p];
+    }
     if (a.limit) ln.limit(a, sc, p, c);
   }
   int fwc = 0, fec = 0;
@@ -379,6 +450,27 @@ __global__ void __launch_bounds__(128) k_psom_tendency(Args a) {
   a.th[p] = a.th[p] + (-advect);
 }
 
+// Cells of a line that a segment of each direction updates: L - 2 of its L positions.
+constexpr int LX = 128, LYZ = 32, BI = 4;
+static int segments(const Geo& g, int dir) {
+  const int n = dir == 1 ? g.ni : dir == 2 ? g.nj : g.nk, cells = (dir == 1 ? LX : LYZ) - 2;
+  return (n + cells - 1) / cells;
+}
+
+// The copy of the cells beside the segments, where a line has several, and the sweeps.
+template <int DIR, int B, int L>
+static void sweep(const Args& a, dim3 grid, cudaStream_t s) {
+  const Geo& g = a.g;
+  const dim3 block = DIR == 1 ? dim3(1, L) : dim3(B, L);
+  if (a.nseg == 1) {
+    k_psom_dir<DIR, B, L, false><<<grid, block, 0, s>>>(a);
+    return;
+  }
+  const long n = DIR == 1 ? (long)g.nj * g.nk * 2 * a.nseg : (long)g.ni * (DIR == 2 ? g.nk : g.nj);
+  k_psom_edges<DIR, L><<<dim3((unsigned)((n + 127) / 128), DIR == 1 ? 1 : 2 * a.nseg), 128, 0, s>>>(a);
+  k_psom_dir<DIR, B, L, true><<<grid, block, 0, s>>>(a);
+}
+
 }  // namespace psom
 
 using namespace psom;
@@ -387,10 +479,16 @@ int launch_psom(mom5gpu_domain* d, int n, int taum1, double dtime) {
   const Geo& g = d->geo;
   size_t n3 = (size_t)g.n3;
   if (!d->psom_scr) {
-    cudaError_t e = cudaMalloc(&d->psom_scr, sizeof(double) * 4 * n3);
+    size_t edges = 0;  // the directions' sweeps use them one after another
+    for (int dir = 1; dir <= 3; ++dir) {
+      const size_t v = edge_values(g, dir, segments(g, dir));
+      edges = v > edges ? v : edges;
+    }
+    const size_t bytes = sizeof(double) * (4 * n3 + edges);
+    cudaError_t e = cudaMalloc(&d->psom_scr, bytes);
     if (e != cudaSuccess) return fail(d, MOM5GPU_ENOMEM, "psom scratch: %s", cudaGetErrorString(e));
-    d->bytes += sizeof(double) * 4 * n3;
-    cudaMemsetAsync(d->psom_scr, 0, sizeof(double) * 4 * n3, d->stream);
+    d->bytes += bytes;
+    cudaMemsetAsync(d->psom_scr, 0, bytes, d->stream);
   }
   Args a;
   a.g = g;
@@ -413,6 +511,7 @@ int launch_psom(mom5gpu_domain* d, int n, int taum1, double dtime) {
   a.fx = d->psom_scr + n3;
   a.fy = d->psom_scr + 2 * n3;
   a.fz = d->psom_scr + 3 * n3;
+  a.edge = d->psom_scr + 4 * n3;
   a.s0 = fptr(d, MOM5GPU_PSOM_S0, n, 0);
   double* m[NMOM];
   for (int q = 0; q < NMOM; ++q) m[q] = fptr(d, MOM5GPU_PSOM_SX + q, n, 0);
@@ -431,25 +530,20 @@ int launch_psom(mom5gpu_domain* d, int n, int taum1, double dtime) {
   ClockScope clk(d, SEC_MDFL);
   cudaStream_t s = d->stream;
   const int* o = order[d->itt0 % 6];
-  constexpr int LX = 128, BI = 4, LYZ = 32;
   for (int st = 0; st < 3; ++st) {
     int dir = o[st];
     a.first = st == 0;
+    a.nseg = segments(g, dir);
     for (int r = 0; r < NROLE; ++r) a.mr[r] = m[roles[dir - 1][r]];
-    if (dir == 1) {
-      dim3 grid((g.ni + LX - 3) / (LX - 2), g.nj, g.nk);
-      k_psom_dir<1, 1, LX><<<grid, dim3(1, LX), 0, s>>>(a);
-    } else if (dir == 2) {
-      dim3 grid((g.ni + BI - 1) / BI, (g.nj + LYZ - 3) / (LYZ - 2), g.nk);
-      k_psom_dir<2, BI, LYZ><<<grid, dim3(BI, LYZ), 0, s>>>(a);
-    } else {
-      dim3 grid((g.ni + BI - 1) / BI, g.nj, (g.nk + LYZ - 3) / (LYZ - 2));
-      k_psom_dir<3, BI, LYZ><<<grid, dim3(BI, LYZ), 0, s>>>(a);
-    }
+    const unsigned nb = (g.ni + BI - 1) / BI;
+    if (dir == 1) sweep<1, 1, LX>(a, dim3(a.nseg, g.nj, g.nk), s);
+    else if (dir == 2) sweep<2, BI, LYZ>(a, dim3(nb, a.nseg, g.nk), s);
+    else sweep<3, BI, LYZ>(a, dim3(nb, g.nj, a.nseg), s);
+    count_launches(d, a.nseg > 1 ? 2 : 1);
   }
   dim3 gt((g.ni + 127) / 128, g.nj, g.nk);
   k_psom_tendency<<<gt, 128, 0, s>>>(a);
-  count_launches(d, 4);
+  count_launches(d, 1);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MOM5GPU_OK : cuda_fail(d, e, "psom");
 }
