@@ -57,13 +57,17 @@ DEVI void rare_lanes(bool rare, F&& f) {
 // of 2^-24, and at most two more too large for the bits cut from B) less four
 // units, hence below 2^24 2^52/B by at most 2^-20.4 of it, and a digit is below
 // 2^19.  Every remainder is then in [0, 2B), so arithmetic modulo 2^64 is
-// exact, and the last one says whether one more belongs to Q.  A quotient of two 53-bit significands is never the
-// midpoint of two doubles, so Q's bits below the result's last one round it
-// correctly without a sticky bit.
+// exact, and the last one says whether one more belongs to Q.  The reciprocal is held
+// to [1/2, 1 - 2^-24], where the true one lies too (but for B = 2^52, whose 1 loses
+// one unit): outside it the 24 bits would not start at the same place, and next to
+// both ends the error of rcp.approx reaches outside.  A quotient of two 53-bit
+// significands is never the midpoint of two doubles, so Q's bits below the result's
+// last one round it correctly without a sticky bit.
 //
-// Operands of an exponent within 2^-510 .. 2^512 take this path, and a zero
-// dividend with such a divisor; any other lane takes the division instruction, so
-// every function returns exactly the IEEE result.
+// Dividends of an exponent within 2^-509 .. 2^512 over divisors within
+// 2^-511 .. 2^512 take this path, and a zero dividend with such a divisor; any other
+// lane takes the division instruction, so every function returns exactly the IEEE
+// result.
 //
 // Shifts are written as products where that lets the multiply-add pipe do them:
 // with the products of the schemes on the integer pipe too, the adder and logic
@@ -71,15 +75,19 @@ DEVI void rare_lanes(bool rare, F&& f) {
 struct Divisor {
   unsigned ex, nlo, nhi, y;  // sign and exponent of b (its high word less the significand's); -B modulo 2^64; 24-bit reciprocal
 };
-DEVI Divisor divisor_of(double b) {
+// The divisor b given rcp.approx of its 24 leading bits.
+DEVI Divisor divisor_with(double b, float y) {
   const unsigned hi = (unsigned)__double2hiint(b), lo = (unsigned)__double2loint(b);
   const unsigned m = (hi & 0xfffffu) | 0x100000u;
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffffu) | 0x3f800000u)));
-  unsigned yb = __float_as_uint(y);
-  yb = yb < 0x3f7fffffu ? yb : 0x3f7fffffu;  // rcp(1) = 1 would lose its leading bit
+  const unsigned yb = min(max(__float_as_uint(y), 0x3f000000u), 0x3f7fffffu);
   const unsigned long long nb = 0ULL - (((unsigned long long)m << 32) | lo);
   return {hi - m, (unsigned)nb, (unsigned)(nb >> 32), ((yb & 0x7fffffu) | 0x800000u) - 4u};
+}
+DEVI Divisor divisor_of(double b) {
+  const unsigned hi = (unsigned)__double2hiint(b), lo = (unsigned)__double2loint(b);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffffu) | 0x3f800000u)));
+  return divisor_with(b, y);
 }
 // The next 18-bit digit of r / B; r becomes the remainder.
 DEVI unsigned div_digit(unsigned long long& r, const Divisor& d) {

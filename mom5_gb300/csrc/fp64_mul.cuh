@@ -14,11 +14,11 @@ namespace fp64 {
 // a * b, the IEEE result.  Significands A, B in [2^52, 2^53): the top 85 of the 117
 // bits of A * (B 2^11) are formed, 52 or 53 of them above bit 32, and rounded with
 // the 32 below.  A remainder of exactly half (a tie, or the rare product with more
-// bits below those), operands of an exponent outside 2^-511 .. 2^510, Inf and NaN
-// take the multiplication instruction.  So do zeros, unless ZA or ZB says that a or
-// b is zero often enough to be given its own path.  Shifts are written as products,
-// which the multiply-add pipe does; the sum of the high words less the
-// significands carries both the sign and the exponent.
+// bits below those), an a of an exponent outside 2^-511 .. 2^510, a b of one outside
+// 2^-511 .. 2^512, Inf and NaN take the multiplication instruction.  So do zeros,
+// unless ZA or ZB says that a or b is zero often enough to be given its own path.
+// Shifts are written as products, which the multiply-add pipe does; the sum of the
+// high words less the significands carries both the sign and the exponent.
 template <bool ZA = false, bool ZB = false>
 DEVI double mul_int(double a, double b) {
   const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
