@@ -607,12 +607,16 @@ DEVI double quarter_exact(double x) {
   return r;
 }
 // C grid: the Coriolis acceleration of the transports u, v at (i, j) (:3707-3715)
-template <bool INT>
+template <bool INT, bool EARLY>
 DEVI void bt_coriolis_c(const BtArgs& a, const double* u, const double* v, int i, int j, double& c0, double& c1) {
   const Geo& g = a.g;
   const long q = I2(g, i, j), s = q - g.nxd, w = q - 1;
-  c0 = quarter_exact(bt_mul<INT>(a.f[q], v[q] + v[q + 1]) + bt_mul<INT>(a.f[s], v[s] + v[s + 1]));
-  c1 = neg_if(quarter_exact(bt_mul<INT>(a.f[q], u[q] + u[q + g.nxd]) + bt_mul<INT>(a.f[w], u[w] + u[w + g.nxd])), true);
+  auto at = [](const double* p) { return load_early<EARLY>(p); };
+  const double fq = at(a.f + q);
+  c0 = quarter_exact(bt_mul<INT>(fq, at(v + q) + at(v + q + 1)) + bt_mul<INT>(at(a.f + s), at(v + s) + at(v + s + 1)));
+  c1 = neg_if(quarter_exact(bt_mul<INT>(fq, at(u + q) + at(u + q + g.nxd)) +
+                            bt_mul<INT>(at(a.f + w), at(u + w) + at(u + w + g.nxd))),
+              true);
 }
 
 // C-grid: initial Adams-Bashforth Coriolis history (:3707-3730)
@@ -623,7 +627,7 @@ DEVI void bt_cgrid_init_body(BtArgs a, int bx, int by) {
   if (i > g.ni) return;
   const long n2 = g.n2, q = I2(g, i, j);
   double c0, c1;
-  bt_coriolis_c<false>(a, a.ubt + n2, a.vbt + n2, i, j, c0, c1);
+  bt_coriolis_c<false, false>(a, a.ubt + n2, a.vbt + n2, i, j, c0, c1);
   for (int m = 0; m < 3; ++m) {
     a.cf[(m * 2 + 0) * n2 + q] = c0;
     a.cf[(m * 2 + 1) * n2 + q] = c1;
@@ -676,7 +680,7 @@ DEVI void bt_mom_b_body(BtArgs a, int so, int sn, int bx) {
   const Loaded<EARLY, double> uo(a.ubt + (so * g.n2 + q)), vo(a.vbt + (so * g.n2 + q));
   const Loaded<EARLY, double> fu(a.forcing_u + q), fv(a.forcing_v + q), cori1(a.cori1 + q), cori2(a.cori2 + q);
   const Loaded<EARLY, double> dyu(a.dyu + q), dxu(a.dxu + q);
-  const double hf = half_exact(a.f[q]);  // 0.5*f; -0.5*f is its negation
+  const double hf = half_exact(load_early<EARLY>(a.f + q));  // 0.5*f; -0.5*f is its negation
   if (EARLY) bt_after_previous();
   double gx = 0.0, gy = 0.0;
   if (i <= g.ni && j <= g.nj) {
@@ -724,9 +728,10 @@ DEVI void bt_mom_c_body(BtArgs a, int so, int sn, int itime, int bx) {
   double ca0 = 0.0, ca1 = 0.0, c0 = 0.0, c1 = 0.0;
   const bool inside = i >= 1 && i <= g.ni && j >= 1 && j <= g.nj;
   if (inside) {
-    bt_coriolis_c<INT>(a, a.ubt + so * n2, a.vbt + so * n2, i, j, c0, c1);
-    ca0 = bt_mul<INT>(abm0, c0) + bt_mul<INT>(abm1, a.cf[(m1 * 2 + 0) * n2 + q]) + abm2 * a.cf[(m2 * 2 + 0) * n2 + q];
-    ca1 = bt_mul<INT>(abm0, c1) + bt_mul<INT>(abm1, a.cf[(m1 * 2 + 1) * n2 + q]) + abm2 * a.cf[(m2 * 2 + 1) * n2 + q];
+    bt_coriolis_c<INT, EARLY>(a, a.ubt + so * n2, a.vbt + so * n2, i, j, c0, c1);
+    auto cf = [&](int m, int c) { return load_early<EARLY>(a.cf + ((m * 2 + c) * n2 + q)); };
+    ca0 = bt_mul<INT>(abm0, c0) + bt_mul<INT>(abm1, cf(m1, 0)) + abm2 * cf(m2, 0);
+    ca1 = bt_mul<INT>(abm0, c1) + bt_mul<INT>(abm1, cf(m1, 1)) + abm2 * cf(m2, 1);
   }
   const Loaded<EARLY, double> te(a.tmen_e + q), tn(a.tmen_n + q), dxter(a.dxter + q), dytnr(a.dytnr + q);
   const Loaded<EARLY, double> the(a.thicken_e + q), thn(a.thicken_n + q), fu(a.forcing_u + q), fv(a.forcing_v + q);

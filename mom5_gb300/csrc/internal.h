@@ -288,11 +288,22 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // The start of a subcycle kernel; with EARLY it stands between the loads of what the
 // launch before does not write and the rest, so that their latency overlaps the end
-// of that launch.  (The launch before waited for the one before it before it allowed
-// this one: pdl_trigger comes after pdl_wait everywhere.)
+// of that launch.  Such a load may read what the launch before that one wrote, with no
+// wait of its own.  Two things make it see those writes:
+//   * pdl_trigger comes after pdl_wait everywhere, so the launch before allowed this
+//     one only when each of its blocks had waited for the launch before it, that is for
+//     its completion and for its writes to be performed and visible;
+//   * the load goes to L2, where those writes are (load_early): a line that this SM's L1
+//     kept from an earlier subcycle cannot answer it, whatever the launch of a
+//     dependent does with that cache.  The manual promises visibility to a launch that
+//     has waited; it says nothing of one that has not.
 __device__ __forceinline__ void bt_after_previous() {
   pdl_wait();
   pdl_trigger();
+}
+template <bool EARLY, class T>
+__device__ __forceinline__ T load_early(const T* p) {
+  return EARLY ? __ldcg(p) : *p;
 }
 // A value loaded where it is declared (EARLY) or, to hold no register until then,
 // where it is used.
@@ -301,7 +312,7 @@ struct Loaded {
   const T* p;
   T v;
   __device__ __forceinline__ explicit Loaded(const T* q) : p(q) {
-    if (EARLY) v = *q;
+    if (EARLY) v = load_early<EARLY>(q);
   }
   __device__ __forceinline__ operator T() const { return EARLY ? v : *p; }
 };
