@@ -36,6 +36,7 @@ struct mom5gpu_batch {
   int* d_counter = nullptr;  // items of the precision form taken so far
   // tuning
   int rows = 32, tj = 0, blocks_per_sm = 2, sms = 152;
+  BtResident resident;  // of the precision form's barotropic subcycles
   bool any_cyclic = false;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   double last_ms = 0.0;
@@ -141,6 +142,7 @@ void fill_work(const mom5gpu_batch* b, const std::vector<std::pair<int, int>>& l
   w.tx = pr[1][c];
   w.ty = pr[2][c];
   w.tb2 = pr[3][c];
+  w.early = b->resident.loads_early(128L * w.tb2);
   w.tb1 = pr[4][c];
   w.tm = pr[5][c];
 }
@@ -319,6 +321,7 @@ int mom5gpu_batch_create(mom5gpu_domain* const* domains, int n, mom5gpu_batch** 
   int dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev);
+  if (b->prec == MOM5GPU_PRECISION_MIXED) b->resident = batch_btf_resident();
   cudaError_t e = cudaStreamCreateWithFlags(&b->own, cudaStreamNonBlocking);
   b->stream = b->own;
   if (e == cudaSuccess) e = cudaEventCreate(&b->e0);

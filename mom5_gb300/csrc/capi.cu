@@ -748,6 +748,8 @@ int mom5gpu_barotropic_init(mom5gpu_domain* d, double dtuv, double dtbt) {
     cudaMemsetAsync(d->bt, 0, bytes, d->stream);
     d->bytes += bytes;
   }
+  if (d->dims.horz_grid == MOM5GPU_CGRID) d->bt_early = true;
+  else d->bt_early = (o.precision == MOM5GPU_PRECISION_MIXED ? btf_resident() : bt_resident()).loads_early(g.n2);
   d->nts = nts;
   d->dtuv = dtuv;
   d->dtbt = dtbt;

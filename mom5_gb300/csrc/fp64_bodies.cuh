@@ -513,7 +513,7 @@ DEVI void mdfl_y_body(MdflArgs a, int TJ, int bx, int by, int bz) {
 // Products of the exact B-grid subcycle: with INT those by dtbt, cori1, cori2, the
 // transports' lengths, datr, dtbt/rho0 and the time weight run on the integer pipe
 // (mul_int), 10 of 20 beside 28 sums (1440x1080, 60 subcycles: 9.8 -> 8.2 ms; with
-// all 20, 8.9); bt_int_products says where.
+// all 20, 8.9), on as many columns as bt_int_products says.
 template <bool INT, bool ZA = false>
 DEVI double bt_mul(double a, double b) {
   if constexpr (INT) return mul_int<ZA, true>(a, b);
@@ -711,9 +711,9 @@ DEVI void bt_mom_b_body(BtArgs a, int so, int sn, int bx) {
 // halo update of the transports: the thread of a halo point with a periodic image
 // forms the image's value.  The transports times their areas over their lengths,
 // which the divergence takes (ocean_operators.F90:507-608), are stored beside them.
-template <bool INT, bool EARLY>
+template <bool INT>
 DEVI void bt_mom_c_body(BtArgs a, int so, int sn, int itime, int bx) {
-  if (!EARLY) bt_after_previous();
+  constexpr bool EARLY = true;
   const Geo& g = a.g;
   int i0, j0;
   if (!bt_point(g, bx, i0, j0)) return;
@@ -737,7 +737,7 @@ DEVI void bt_mom_c_body(BtArgs a, int so, int sn, int itime, int bx) {
   const Loaded<EARLY, double> the(a.thicken_e + q), thn(a.thicken_n + q), fu(a.forcing_u + q), fv(a.forcing_v + q);
   const Loaded<EARLY, double> uo(a.ubt + (so * n2 + q)), vo(a.vbt + (so * n2 + q));
   const Loaded<EARLY, double> dat0(a.dat + q0), dxter0(a.dxter + q0), dytnr0(a.dytnr + q0);
-  if (EARLY) bt_after_previous();
+  bt_after_previous();
   if (inside && q == q0) {
     a.cf[(m0 * 2 + 0) * n2 + q] = c0;
     a.cf[(m0 * 2 + 1) * n2 + q] = c1;
@@ -766,16 +766,16 @@ DEVI void bt_mom_c_body(BtArgs a, int so, int sn, int itime, int bx) {
 // C grid: the corrector of subcycle t and the predictor of subcycle t+1, which
 // reads only its own point's corrected eta and divergence (bt_corr_body's and
 // bt_pred_body's operations).
-template <bool INT, bool EARLY>
+template <bool INT>
 DEVI void bt_corr_pred_c_body(BtArgs a, int so, int sn, double wgt, int bx) {
-  if (!EARLY) bt_after_previous();
+  constexpr bool EARLY = true;
   const Geo& g = a.g;
   int i, j;
   if (!bt_point(g, bx, i, j)) return;
   const long n2 = g.n2, q = I2(g, i, j);
   const Loaded<EARLY, double> tm(a.tmask1 + q), steady(a.steady + q), datr(a.datr + q), eo(a.eta_bt + (so * n2 + q));
   const Loaded<EARLY, double> bar(a.eta_bar + q), su(a.udrho_u + q), sv(a.udrho_v + q), rho_g(a.rho_g + q), patm(a.patm + q);
-  if (EARLY) bt_after_previous();
+  bt_after_previous();
   const double un = a.ubt[sn * n2 + q], vn = a.vbt[sn * n2 + q];
   double dv = 0.0;
   if (i >= 1 && j >= 1)

@@ -110,6 +110,7 @@ struct mom5gpu_domain {
   int* wait_err = nullptr;   // set when a bounded device wait gave up: bit 1 a grid barrier
   unsigned* bt_sync = nullptr;  // arrival counter of the cooperative barotropic subcycle's grid barriers
   int tune_y_tj = 0;         // FP64 y-pass rows per thread
+  bool bt_early = true;      // the barotropic subcycles load early (BtResident), set by barotropic_init
   int bt_fused = 0;          // exact B-grid subcycles: 0 three launches each, 1 one launch each,
                              // 2 all in one cooperative launch
   int coop_blocks = 0;       // resident blocks per SM of the cooperative subcycle kernel (0: not queried, -1: none)
@@ -188,6 +189,7 @@ constexpr int kMdflChunk = 10;
 struct BtArgs {
   Geo g;
   int cgrid, nts, stepB;
+  int early;  // one-domain subcycles load early (BtResident)
   double dtbt, dtbt_gamma_rho0r, dtbt_rho0r, gamma;
   const double *tmask1, *umask1, *f, *dxu, *dyu, *dxur, *dyur, *dat, *datr, *dxter, *dytnr, *tmen_e, *tmen_n;
   const double *dte, *dtw, *dus, *dun, *daur;
@@ -336,22 +338,43 @@ cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, A
 // pipe (bt_mul).  On the FP64 pipe and on the integer pipe, 80 subcycles: 120x100
 // columns 0.65 and 0.74 ms, 300x260 0.99 and 1.14, 360x300 1.23 and 1.10; C grid, 48
 // subcycles, 361x243 0.68 and 0.60; 60 subcycles, 1440x1080 9.81 and 8.17.
-inline bool bt_int_products(long columns) { return columns >= 85000; }
-// Whether the subcycle kernels load early (bt_after_previous).  With the registers
-// that takes, the waiting blocks of one launch and the running ones of the launch
-// before fit an SM together up to about 92000 columns (90x60 columns, 80 subcycles:
-// 0.65 -> 0.45 ms alone; C grid 361x243 0.62 -> 0.60); past that the waiting ones come to
-// the SMs that end first, which a launch of one round pays for (360x300: 1.12 -> 1.38 ms)
-// and one of several does not (1440x1080, precision form, 60 subcycles: 4.28 -> 3.88).
-inline bool bt_early_loads(long columns) { return columns <= 92000 || columns >= 300000; }
-// the instantiation <INT, EARLY> of a subcycle kernel for so many columns
-#define BT_VARIANT(K, columns)                                                             \
-  (bt_int_products(columns) ? (bt_early_loads(columns) ? K<true, true> : K<true, false>)   \
-                            : (bt_early_loads(columns) ? K<false, true> : K<false, false>))
-// Threads and blocks of a 2-D barotropic launch of one domain: small blocks while
-// they fit the SMs in one round (360x300: 1.10 ms with 64 threads, 1.12 with 128, 1.34
-// with 32, of which an SM holds too few).
-inline int bt_threads(const Geo& g) { return g.n2 < 152L * 2048 ? 64 : 128; }
+inline bool bt_int_products(bool, long columns) { return columns >= 85000; }
+// Columns over which both a running launch of kernel a and a waiting one of kernel b, in
+// blocks of so many threads, are resident.
+long bt_resident_columns(const void* a, const void* b, int threads);
+// Whether the subcycle kernels load early (bt_after_previous).  A launch's blocks come
+// to the SMs as soon as the one before has started all of its own, and wait there.
+// Where both launches fit the SMs together, the start of each is hidden behind the end
+// of the other and early loads win.  They take registers, so this holds up to fewer
+// columns for the kernels that load early (`early`) than for those that load late
+// (`late`); between the two late loads win.  Past both, the waiting blocks come as the
+// running ones end in either form, and early loads win again.
+// 60 subcycles, us a step, early and late.  B grid, blocks of 64 (48 + 64 and 40 + 40
+// registers, 9 and 12 pairs of blocks an SM): 659 and 739 at 86955 columns, 1021 and 764
+// at 91134, 1024 and 843 at 111360, 1036 and 1386 at 119110, 1382 and 1465 at 226524.
+// Precision form, blocks of 128 (40 + 40 and 32 + 32: 6 and 8 pairs): 455 and 495 at
+// 111360, 675 and 533 at 119110, 686 and 595 at 151140, 696 and 933 at 166600, 874 and
+// 972 at 286812.  The C grid's kernels lose at most 2% by early loads (785 and 773 at 95914
+// columns, 767 and 771 at 91134, 882 and 911 at 127167, 904 and 1514 at 137200) and
+// always load early, and so do the exact form's batches, whose two forms fit up to the
+// same 4 pairs of blocks of 128 (600 and 668 at 67584 columns, 952 and 1102 at 88192, 2038 and 2213 at 323968).
+struct BtResident {
+  long early = 0, late = 0;
+  bool loads_early(long columns) const { return columns <= early || columns > late; }
+};
+BtResident bt_resident();           // B grid, exact form (k_fp64.cu)
+BtResident btf_resident();          // B grid, precision form (k_mixed.cu)
+BtResident batch_btf_resident();    // batches, precision form (k_batch.cu)
+// the instantiation <INT, EARLY> of an exact B-grid subcycle kernel; FP64 products only on few
+// columns, where the loads are early
+#define BT_VARIANT(K, columns, early) \
+  (!bt_int_products(false, columns) ? K<false, true> : (early) ? K<true, true> : K<true, false>)
+// Threads per block of a one-domain 2-D launch.  Exact form: 64 (60 subcycles against
+// blocks of 128: 513 and 567 us a step at 52750 columns, 1132 and 1143 at 166600, 5056 and 5119 at 1003230).
+// Precision form, whose kernels are half as long: 128 from 30000 columns on (338 us against
+// 409 with 64 at 52750, 446 against 585 at 102960), 64 below (307 and 313 at 22444).
+constexpr int kBtThreads = 64;
+inline int btf_threads(const Geo& g) { return g.n2 < 30000 ? 64 : 128; }
 inline dim3 bt_grid(const Geo& g, int threads) { return dim3((unsigned)((g.n2 + threads - 1) / threads)); }
 // precision-form barotropic subcycle (k_mixed.cu, k_batch.cu)
 void launch_btf_prep(const BtArgs& a, cudaStream_t s);
@@ -385,6 +408,7 @@ struct BatchWork {
   int count;
   int tz, tx, ty, tb2, tb1, tm;      // total blocks of each pass
   int seg;                           // levels per item of the precision form
+  bool early;                        // the precision form's subcycles load early (BtResident)
 };
 // blocks of one domain in each pass, for the work-list prefix sums; m: the
 // precision form's items, tiles of tile_rows rows by segments of seg levels

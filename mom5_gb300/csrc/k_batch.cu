@@ -58,12 +58,17 @@ void launch_batch_btf_prep(const BtArgs* bt, const BatchWork& w, cudaStream_t s)
 // subcycle itime of nts, as the one-domain form 0: the predictor launched only in
 // the first subcycle, the corrector forming the next subcycle's predictor in all
 // but the last; returns the launches
+BtResident batch_btf_resident() {
+  auto pair = [](auto* mom, auto* corr) { return bt_resident_columns((const void*)mom, (const void*)corr, 128); };
+  return {pair(kb_btf_mom<true>, kb_btf_corr_pred<true>), pair(kb_btf_mom<false>, kb_btf_corr_pred<false>)};
+}
+
 int launch_batch_btf_subcycle(const BtArgs* bt, const BatchWork& w, int itime, int nts, cudaStream_t s) {
   if (w.tb2 <= 0) return 0;
   const int so = itime % 2, sn = (itime + 1) % 2;
   const double wgt = (double)(nts - itime + 1);
   const dim3 g2(w.tb2), b(128);
-  const bool early = bt_early_loads(128L * w.tb2);
+  const bool early = w.early;
   if (itime == 1) launch_pdl(kb_btf_pred, g2, b, s, bt, w, so, sn, 0);
   launch_pdl(early ? kb_btf_mom<true> : kb_btf_mom<false>, g2, b, s, bt, w, so, sn, wgt);
   if (itime < nts) launch_pdl(early ? kb_btf_corr_pred<true> : kb_btf_corr_pred<false>, g2, b, s, bt, w, so, sn);

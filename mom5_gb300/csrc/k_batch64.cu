@@ -71,10 +71,10 @@ __global__ void __launch_bounds__(128) kb_bt_pred(const BtArgs* d, BatchWork w, 
   BT2D_ENTRY
   bt_pred_body(a, so, sn, reuse, bx);
 }
-template <bool INT, bool EARLY>
+template <bool INT>
 __global__ void __launch_bounds__(128) kb_bt_mom_b(const BtArgs* d, BatchWork w, int so, int sn) {
   BT2D_ENTRY
-  bt_mom_b_body<INT, EARLY>(a, so, sn, bx);
+  bt_mom_b_body<INT, true>(a, so, sn, bx);
 }
 __global__ void __launch_bounds__(128) kb_bt_corr(const BtArgs* d, BatchWork w, int so, int sn, double wgt) {
   pdl_wait();
@@ -82,10 +82,10 @@ __global__ void __launch_bounds__(128) kb_bt_corr(const BtArgs* d, BatchWork w, 
   BT2D_ENTRY
   bt_corr_body(a, so, sn, wgt, bx);
 }
-template <bool INT, bool EARLY>
+template <bool INT>
 __global__ void __launch_bounds__(128) kb_bt_corr_pred(const BtArgs* d, BatchWork w, int so, int sn, double wgt) {
   BT2D_ENTRY
-  bt_corr_pred_body<INT, EARLY>(a, so, sn, wgt, bx);
+  bt_corr_pred_body<INT, true>(a, so, sn, wgt, bx);
 }
 __global__ void __launch_bounds__(256) kb_bt_post1(const BtArgs* d, BatchWork w, double rntsp1, double rnts) {
   int e = find_entry(w.pb1, w.count, blockIdx.x);
@@ -157,9 +157,9 @@ void launch_batch_barotropic_loop(const BtArgs* bt, const BtExtra* x, const Batc
     const dim3 g2(w.tb2), b(128);
     const double wgt = (double)(nts - itime + 1);
     if (itime == 1) launch_pdl(kb_bt_pred, g2, b, s, bt, w, so, sn, 0);
-    const long cols = 128L * w.tb2;
-    launch_pdl(BT_VARIANT(kb_bt_mom_b, cols), g2, b, s, bt, w, so, sn);
-    if (itime < nts) launch_pdl(BT_VARIANT(kb_bt_corr_pred, cols), g2, b, s, bt, w, so, sn, wgt);
+    const bool in = bt_int_products(false, 128L * w.tb2);
+    launch_pdl(in ? kb_bt_mom_b<true> : kb_bt_mom_b<false>, g2, b, s, bt, w, so, sn);
+    if (itime < nts) launch_pdl(in ? kb_bt_corr_pred<true> : kb_bt_corr_pred<false>, g2, b, s, bt, w, so, sn, wgt);
     else launch_pdl(kb_bt_corr, g2, b, s, bt, w, so, sn, wgt);
   }
   (void)stepB;

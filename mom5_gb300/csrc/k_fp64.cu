@@ -1310,13 +1310,13 @@ template <bool INT, bool EARLY>
 __global__ void k_bt_mom_b(BtArgs a, int so, int sn) {
   bt_mom_b_body<INT, EARLY>(a, so, sn, blockIdx.x);
 }
-template <bool INT, bool EARLY>
+template <bool INT>
 __global__ void k_bt_mom_c(BtArgs a, int so, int sn, int itime) {
-  bt_mom_c_body<INT, EARLY>(a, so, sn, itime, blockIdx.x);
+  bt_mom_c_body<INT>(a, so, sn, itime, blockIdx.x);
 }
-template <bool INT, bool EARLY>
+template <bool INT>
 __global__ void k_bt_corr_pred_c(BtArgs a, int so, int sn, double wgt) {
-  bt_corr_pred_c_body<INT, EARLY>(a, so, sn, wgt, blockIdx.x);
+  bt_corr_pred_c_body<INT>(a, so, sn, wgt, blockIdx.x);
 }
 __global__ void k_bt_corr(BtArgs a, int so, int sn, double wgt) {
   pdl_wait();
@@ -1508,6 +1508,30 @@ int grid_barrier_selftest(mom5gpu_domain* d, int rounds, int unreachable) {
 __global__ void k_bt_post2(BtArgs a, double* conv, double* eta_u, double* ps_out) { bt_post2_body(a, conv, eta_u, ps_out, blockIdx.x); }
 __global__ void k_bt_post3(BtArgs a, const double* ps, double* gxo, double* gyo) { bt_post3_body(a, ps, gxo, gyo, blockIdx.x); }
 
+long bt_resident_columns(const void* a, const void* b, int threads) {
+  cudaFuncAttributes fa, fb;
+  int dev = 0, sms = 0, regs = 0, warps = 0, blocks = 0;
+  cudaGetDevice(&dev);
+  if (cudaFuncGetAttributes(&fa, a) != cudaSuccess || cudaFuncGetAttributes(&fb, b) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&regs, cudaDevAttrMaxRegistersPerMultiprocessor, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&warps, cudaDevAttrMaxThreadsPerMultiProcessor, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&blocks, cudaDevAttrMaxBlocksPerMultiprocessor, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;  // both limits 0: early loads
+  }
+  auto rounded = [](int r) { return (r + 7) / 8 * 8; };  // registers are given to a warp in groups of 8 a thread
+  int pairs = regs / ((rounded(fa.numRegs) + rounded(fb.numRegs)) * threads);
+  if (pairs > warps / (2 * threads)) pairs = warps / (2 * threads);
+  if (pairs > blocks / 2) pairs = blocks / 2;
+  return (long)pairs * sms * threads;
+}
+BtResident bt_resident() {
+  auto pair = [](auto* mom, auto* corr) { return bt_resident_columns((const void*)mom, (const void*)corr, kBtThreads); };
+  return {pair(k_bt_mom_b<true, true>, k_bt_corr_pred<true, true>),
+          pair(k_bt_mom_b<true, false>, k_bt_corr_pred<true, false>)};
+}
+
 int make_bt_args(mom5gpu_domain* d, int tau, int taup1, BtArgs* ap, BtExtra* xp) {
   const Geo& g = d->geo;
   if (!d->baro_ready) return fail(d, MOM5GPU_ESTATE, "update_ocean_barotropic before mom5gpu_barotropic_init");
@@ -1516,6 +1540,7 @@ int make_bt_args(mom5gpu_domain* d, int tau, int taup1, BtArgs* ap, BtExtra* xp)
   memset(&a, 0, sizeof(BtArgs));  // padding too: the bytes key the subcycle graph
   a.g = g;
   a.cgrid = d->dims.horz_grid == MOM5GPU_CGRID;
+  a.early = d->bt_early;
   a.nts = d->nts;
   a.stepB = d->opt.barotropic_time_stepping_B;
   a.dtbt = d->dtbt;
@@ -1651,7 +1676,7 @@ int launch_barotropic(mom5gpu_domain* d, int tau, int taup1) {
   count_launches(d, 1 + (a.cgrid ? 1 : 0) + (a.btf ? 1 : 0) + sub_launches + 4 + 5 * halo);
   k_bt_init<<<(unsigned)((n2 + 255) / 256), 256, 0, s>>>(a, eta_bar_tau, eta_tau, ud_tau, vd_tau, pme, river, src,
                                                           esm, d->opt.initsum_with_bar);
-  const int bt = bt_threads(g);
+  const int bt = kBtThreads;
   const dim3 g2 = bt_grid(g, bt);
   if (a.cgrid) {
     dim3 gc((g.ni + 127) / 128, g.nj);
@@ -1677,13 +1702,14 @@ int launch_barotropic(mom5gpu_domain* d, int tau, int taup1) {
       const double wgt = (double)(a.nts - itime + 1);
       if (itime == 1) launch_pdl(k_bt_pred, g2, dim3(bt), st, a, so, sn, 0);
       if (a.cgrid) {
-        launch_pdl(BT_VARIANT(k_bt_mom_c, n2), g2, dim3(bt), st, a, so, sn, itime);
-        launch_pdl(BT_VARIANT(k_bt_corr_pred_c, n2), g2, dim3(bt), st, a, so, sn, wgt);
+        const bool in = bt_int_products(true, n2);
+        launch_pdl(in ? k_bt_mom_c<true> : k_bt_mom_c<false>, g2, dim3(bt), st, a, so, sn, itime);
+        launch_pdl(in ? k_bt_corr_pred_c<true> : k_bt_corr_pred_c<false>, g2, dim3(bt), st, a, so, sn, wgt);
         continue;
       }
-      launch_pdl(BT_VARIANT(k_bt_mom_b, n2), g2, dim3(bt), st, a, so, sn);
+      launch_pdl(BT_VARIANT(k_bt_mom_b, n2, a.early), g2, dim3(bt), st, a, so, sn);
       if (itime < a.nts)
-        launch_pdl(BT_VARIANT(k_bt_corr_pred, n2), g2, dim3(bt), st, a, so, sn, wgt);
+        launch_pdl(BT_VARIANT(k_bt_corr_pred, n2, a.early), g2, dim3(bt), st, a, so, sn, wgt);
       else launch_pdl(k_bt_corr, g2, dim3(bt), st, a, so, sn, wgt);
     }
   };

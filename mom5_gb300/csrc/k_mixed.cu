@@ -49,6 +49,11 @@ __global__ void __launch_bounds__(kBtfThreads) k_btf_fused(BtArgs a, int so, int
 // first subcycle), the momentum step, and the corrector, which in every
 // subcycle but the last also forms the next subcycle's predictor; 1 + 2*nts
 // launches per step.  Form 1: one launch per subcycle.  Returns the launches.
+BtResident btf_resident() {
+  auto pair = [](auto* mom, auto* corr) { return bt_resident_columns((const void*)mom, (const void*)corr, 128); };
+  return {pair(k_btf_mom<true>, k_btf_corr_pred<true>), pair(k_btf_mom<false>, k_btf_corr_pred<false>)};
+}
+
 int launch_btf_subcycle(const BtArgs& a, int itime, int nts, bool fused, cudaStream_t s) {
   const int so = itime % 2, sn = (itime + 1) % 2;
   const double wgt = (double)(nts - itime + 1);
@@ -57,8 +62,8 @@ int launch_btf_subcycle(const BtArgs& a, int itime, int nts, bool fused, cudaStr
     launch_pdl(k_btf_fused, gf, dim3(kBtfThreads), s, a, so, sn, (int)(itime > 1), wgt);
     return 1;
   }
-  const dim3 b(bt_threads(a.g)), g2 = bt_grid(a.g, b.x);
-  const bool early = bt_early_loads(a.g.n2);
+  const dim3 b(btf_threads(a.g)), g2 = bt_grid(a.g, b.x);
+  const bool early = a.early;
   if (itime == 1) launch_pdl(k_btf_pred, g2, b, s, a, so, sn, 0);
   launch_pdl(early ? k_btf_mom<true> : k_btf_mom<false>, g2, b, s, a, so, sn, wgt);
   if (itime < nts) launch_pdl(early ? k_btf_corr_pred<true> : k_btf_corr_pred<false>, g2, b, s, a, so, sn);

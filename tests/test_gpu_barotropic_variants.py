@@ -24,8 +24,8 @@ def domain(ni, nj, cx, cy, ntr=0, nk=1, seed=0):
     return sp, grid.make_domain(sp)
 
 
-# columns of the data domain: 5538 (FP64 products, early loads), 88935, 111325 (late loads), 316713 (128 threads)
-SIZES = [(69, 76), (361, 243), (363, 303), (577, 545)]
+# columns of the data domain: 5538, 88935, 111325, 125139, 316713
+SIZES = [(69, 76), (361, 243), (363, 303), (411, 301), (577, 545)]
 
 
 @pytest.mark.parametrize("cgrid", [False, True])
