@@ -335,10 +335,12 @@ cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, A
 }
 
 // Whether a launch over so many columns takes the subcycle's products on the integer
-// pipe (bt_mul).  On the FP64 pipe and on the integer pipe, 80 subcycles: 120x100
-// columns 0.65 and 0.74 ms, 300x260 0.99 and 1.14, 360x300 1.23 and 1.10; C grid, 48
-// subcycles, 361x243 0.68 and 0.60; 60 subcycles, 1440x1080 9.81 and 8.17.
-inline bool bt_int_products(bool, long columns) { return columns >= 85000; }
+// pipe (bt_mul).  Small launches are chains of latency, which its longer sequence
+// adds to; larger ones are bound by the FP64 pipe.  On the FP64 and on the integer pipe,
+// 60 subcycles, us a step: B grid 394 and 406 at 28566 columns, 490 and 438 at 34748;
+// batches 349 and 360 at 12928, 424 and 412 at 21376, 440 and 430 at 38144; C grid
+// 494 and 552 at 52750, 588 and 567 at 58968, 684 and 644 at 71052.
+inline bool bt_int_products(bool cgrid, long columns) { return columns >= (cgrid ? 60000 : 30000); }
 // Columns over which both a running launch of kernel a and a waiting one of kernel b, in
 // blocks of so many threads, are resident.
 long bt_resident_columns(const void* a, const void* b, int threads);
