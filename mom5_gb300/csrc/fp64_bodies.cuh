@@ -43,27 +43,35 @@ DEVI double plus_zero(double x) { return bits_of(x) == (long long)0x800000000000
 DEVI double neg_if(double x, bool flip) {
   return double_of(bits_of(x) ^ (flip ? (long long)0x8000000000000000ULL : 0LL));
 }
-// 0.5*x: for a normal x whose exponent field is at least 2 the product is the
-// exponent lowered by one; +-0 is unchanged.  Subnormals, the smallest normals,
-// Inf and NaN take the multiply.
+// x*m for a mask m of 0.0 or 1.0 (tmask: tracer_advect_init refuses others), without the
+// vote and the branch of a fallback, which the row and level marches of the flux-form
+// schemes wait for on small domains (with half_exact as below: 2nd order, 12 tracers on
+// 169x17x8 cells 291 -> 212 us a step, upwind, 8 tracers on 69x21x17 256 -> 212).
+DEVI double mask_sel(double x, double m) {
+  const unsigned hi = (unsigned)__double2hiint(x), mh = (unsigned)__double2hiint(m);
+  const bool inf = (hi & 0x7ff00000u) == 0x7ff00000u;  // Inf*0 and NaN*0: NaN
+  const double z = __hiloint2double((int)(inf ? 0x7fffffffu : (hi ^ mh) & 0x80000000u), inf ? -1 : 0);
+  return is_zero(m) ? z : x;
+}
+// 0.5*x: the exponent lowered by one, Inf and NaN unchanged; at exponent fields 0 and 1
+// the bits of the magnitude count in units of 2^-1074, and their half is rounded to even.
 DEVI double half_exact(double x) {
-  long long b = bits_of(x);
-  unsigned e = (unsigned)((unsigned long long)b >> 52) & 0x7ffu;
-  bool normal = e - 2u < 0x7fdu;  // 2 <= e <= 0x7fe
-  double r = double_of(normal ? b - (1LL << 52) : b);
-  rare_lanes(!(normal || (b << 1) == 0), [&] { r = 0.5 * x; });
-  return r;
+  const long long b = bits_of(x);
+  const unsigned mh = (unsigned)((unsigned long long)b >> 32) & 0x7fffffffu;
+  const unsigned long long mag = (unsigned long long)b & 0x7fffffffffffffffULL;
+  const long long small = (long long)((mag >> 1) + ((b & 3) == 3 ? 1 : 0)) | (b & (long long)0x8000000000000000ULL);
+  long long r = b - (mh < 0x7ff00000u ? 1LL << 52 : 0LL);
+  return double_of(mh < 0x00200000u ? small : r);
 }
 
-// 2*x: the exponent raised by one where both are normal; +-0 is unchanged, the rest
-// take the multiply.
+// 2*x: the exponent raised by one, Inf and NaN unchanged; a magnitude of exponent field 0
+// is shifted, and one of the largest field gives Inf.
 DEVI double twice(double x) {
-  const long long b = bits_of(x);
-  const unsigned e = (unsigned)((unsigned long long)b >> 52) & 0x7ffu;
-  const bool normal = e - 1u < 0x7fdu;  // 1 <= e <= 0x7fd
-  double r = double_of(normal ? b + (1LL << 52) : b);
-  rare_lanes(!(normal || (b << 1) == 0), [&] { r = 2.0 * x; });
-  return r;
+  const long long b = bits_of(x), s = b & (long long)0x8000000000000000ULL;
+  const unsigned mh = (unsigned)((unsigned long long)b >> 32) & 0x7fffffffu;
+  long long r = b + (mh < 0x7ff00000u ? 1LL << 52 : 0LL);
+  if (mh >= 0x7fe00000u && mh < 0x7ff00000u) r = s | 0x7ff0000000000000LL;
+  return double_of(mh < 0x00100000u ? (b << 1) | s : r);
 }
 
 // Arithmetic of an MDFL pass: sums on the FP64 pipe, the products whose bit is set

@@ -338,7 +338,7 @@ DEVI void horz_faces_once(const Geo& g, const double* tmask, const double* datr,
     if (cell) {
       double fn = fy(i, j, k);
       long p = I3(g, i, j, k);
-      double rr = mask_mul(sfx[t + 1] - sfx[t] + fn - fs, tmask[p]) * datr[I2(g, i, j)];
+      double rr = mask_sel(sfx[t + 1] - sfx[t] + fn - fs, tmask[p]) * datr[I2(g, i, j)];
       th[p] = th[p] + (-rr);
       fs = fn;
     }
@@ -354,7 +354,7 @@ DEVI void vert_segment(const Geo& g, const double* tmask, double* th, FZ fz) {
   for (int k = k0; k < k1; ++k) {
     double ft2 = fz(i, j, k);
     long p = I3(g, i, j, k);
-    double r = mask_mul(ft1 - ft2, tmask[p]);
+    double r = mask_sel(ft1 - ft2, tmask[p]);
     th[p] = th[p] + (-r);
     ft1 = ft2;
   }
@@ -378,7 +378,7 @@ DEVI double upw_fe(const UpwArgs& a, int i, int j, int k) {
   double uneg = velocity - fabs(velocity);
   double f = a.dyte[I2(g, i, j)] * (upos * a.T[I3(g, i, j, k)] + uneg * a.T[I3(g, i + 1, j, k)]);
   double m0 = a.tmask[I3(g, i, j, k)], m1 = a.tmask[I3(g, i + 1, j, k)];
-  return (!is_zero(m0) && !is_zero(m1)) ? mask_mul(mask_mul(f, m0), m1) : 0.0;
+  return (!is_zero(m0) && !is_zero(m1)) ? f : 0.0;
 }
 DEVI double upw_fn(const UpwArgs& a, int i, int j, int k) {
   const Geo& g = a.g;
@@ -387,7 +387,7 @@ DEVI double upw_fn(const UpwArgs& a, int i, int j, int k) {
   double uneg = velocity - fabs(velocity);
   double f = a.dxtn[I2(g, i, j)] * (upos * a.T[I3(g, i, j, k)] + uneg * a.T[I3(g, i, j + 1, k)]);
   double m0 = a.tmask[I3(g, i, j, k)], m1 = a.tmask[I3(g, i, j + 1, k)];
-  return (!is_zero(m0) && !is_zero(m1)) ? mask_mul(mask_mul(f, m0), m1) : 0.0;
+  return (!is_zero(m0) && !is_zero(m1)) ? f : 0.0;
 }
 
 __global__ void __launch_bounds__(HB) k_upwind_horz(UpwArgs a) {
@@ -405,7 +405,7 @@ DEVI double upw_fz(const UpwArgs& a, int i, int j, int k) {
   double wpos = velocity + fabs(velocity);
   double wneg = velocity - fabs(velocity);
   double ft2 = (wneg * a.T[p] + wpos * a.T[pp]);
-  return (!is_zero(a.tmask[p]) && !is_zero(a.tmask[pp])) ? mask_mul(mask_mul(ft2, a.tmask[p]), a.tmask[pp]) : 0.0;
+  return (!is_zero(a.tmask[p]) && !is_zero(a.tmask[pp])) ? ft2 : 0.0;
 }
 
 __global__ void k_upwind_vert(UpwArgs a) {
@@ -491,7 +491,7 @@ DEVI double quk_fx(const QukArgs& a, int i, int j, int k) {
     double upos = half_exact(vel + fabs(vel));
     double uneg = half_exact(vel - fabs(vel));
     double f = a.dyte[q] * (upos * a.Tm1[I3(g, i, j, k)] + uneg * a.Tm1[I3(g, i + 1, j, k)]);
-    return mask_mul(mask_mul(f, a.tmask[I3(g, i, j, k)]), a.tmask[I3(g, i + 1, j, k)]);
+    return mask_sel(mask_sel(f, a.tmask[I3(g, i, j, k)]), a.tmask[I3(g, i + 1, j, k)]);
   }
   double vel = a.dyte[q] * a.uh[I3(g, i, j, k)];
   double upos = half_exact(vel + fabs(vel));
@@ -516,7 +516,7 @@ DEVI double quk_fy(const QukArgs& a, int i, int j, int k) {
     double upos = half_exact(vel + fabs(vel));
     double uneg = half_exact(vel - fabs(vel));
     double f = a.dxtn[q] * (upos * a.Tm1[I3(g, i, j, k)] + uneg * a.Tm1[I3(g, i, j + 1, k)]);
-    return mask_mul(mask_mul(f, a.tmask[I3(g, i, j, k)]), a.tmask[I3(g, i, j + 1, k)]);
+    return mask_sel(mask_sel(f, a.tmask[I3(g, i, j, k)]), a.tmask[I3(g, i, j + 1, k)]);
   }
   double vel = a.dxtn[q] * a.vh[I3(g, i, j, k)];
   double upos = half_exact(vel + fabs(vel));
@@ -551,7 +551,7 @@ DEVI double quk_fz(const QukArgs& a, int i, int j, int k) {
   double uneg = half_exact(vel - fabs(vel));
   const double* Tm = a.Tm1;
   if (is_one(a.tmask_limit[p]))
-    return mask_mul(mask_mul(uneg * Tm[p] + upos * Tm[I3(g, i, j, kp1)], a.tmask[p]), a.tmask[I3(g, i, j, kp1)]);
+    return mask_sel(mask_sel(uneg * Tm[p] + upos * Tm[I3(g, i, j, kp1)], a.tmask[p]), a.tmask[I3(g, i, j, kp1)]);
   // kp2 = nint(tmask(p2)*p2 + (1-tmask(p2))*kp1): p2 when level p2 is wet, else kp1
   int kp2 = !is_zero(a.tmask[I3(g, i, j, p2)]) ? p2 : kp1;
   bool upmsk = !is_zero(a.tmask[p]) && is_zero(a.tmask[I3(g, i, j, km1)]);
@@ -577,12 +577,12 @@ DEVI double qm3_fx(const QukArgs& a, int i, int j, int k) {
     double upos = half_exact(vel + fabs(vel));
     double uneg = half_exact(vel - fabs(vel));
     double f = a.dyte[q] * (upos * a.Tm1[I3(g, i, j, k)] + uneg * a.Tm1[I3(g, i + 1, j, k)]);
-    return mask_mul(mask_mul(f, a.tmask[I3(g, i, j, k)]), a.tmask[I3(g, i + 1, j, k)]);
+    return mask_sel(mask_sel(f, a.tmask[I3(g, i, j, k)]), a.tmask[I3(g, i + 1, j, k)]);
   }
   auto mq = [&](int ii) { return a.mask2[IM(g, ii, j, k)] ? 1.0 : 0.0; };
   double vel = a.dyte[q] * a.uh[I3(g, i, j, k)];
-  double upos = mask_mul(mask_mul(mask_mul(half_exact(vel + fabs(vel)), mq(i - 1)), mq(i)), mq(i + 1));
-  double uneg = mask_mul(mask_mul(mask_mul(half_exact(vel - fabs(vel)), mq(i + 2)), mq(i + 1)), mq(i));
+  double upos = mask_sel(mask_sel(mask_sel(half_exact(vel + fabs(vel)), mq(i - 1)), mq(i)), mq(i + 1));
+  double uneg = mask_sel(mask_sel(mask_sel(half_exact(vel - fabs(vel)), mq(i + 2)), mq(i + 1)), mq(i));
   double tqm = tq(g, a.Tm1, i - 1, j, k), tq0 = tq(g, a.Tm1, i, j, k);
   double tq1 = tq(g, a.Tm1, i + 1, j, k), tq2 = tq(g, a.Tm1, i + 2, j, k);
   return vel * (a.q.quick_x[q] * a.T0[I3(g, i, j, k)] + a.q.quick_x[n2 + q] * a.T0[I3(g, i + 1, j, k)]) -
@@ -599,13 +599,13 @@ DEVI double qm3_fy(const QukArgs& a, int i, int j, int k) {
     double upos = half_exact(vel + fabs(vel));
     double uneg = half_exact(vel - fabs(vel));
     double f = a.dxtn[q] * (upos * a.Tm1[I3(g, i, j, k)] + uneg * a.Tm1[I3(g, i, j + 1, k)]);
-    return mask_mul(mask_mul(f, a.tmask[I3(g, i, j, k)]), a.tmask[I3(g, i, j + 1, k)]);
+    return mask_sel(mask_sel(f, a.tmask[I3(g, i, j, k)]), a.tmask[I3(g, i, j + 1, k)]);
   }
   const int jp2 = j + 2 < g.nj ? j + 2 : g.nj;  // min(j+2, jec)
   auto mq = [&](int jj) { return a.mask2[IM(g, i, jj, k)] ? 1.0 : 0.0; };
   double vel = a.dxtn[q] * a.vh[I3(g, i, j, k)];
-  double upos = mask_mul(mask_mul(mask_mul(half_exact(vel + fabs(vel)), mq(j - 1)), mq(j)), mq(j + 1));
-  double uneg = mask_mul(mask_mul(mask_mul(half_exact(vel - fabs(vel)), mq(jp2)), mq(j + 1)), mq(j));
+  double upos = mask_sel(mask_sel(mask_sel(half_exact(vel + fabs(vel)), mq(j - 1)), mq(j)), mq(j + 1));
+  double uneg = mask_sel(mask_sel(mask_sel(half_exact(vel - fabs(vel)), mq(jp2)), mq(j + 1)), mq(j));
   double tqm = tq(g, a.Tm1, i, j - 1, k), tq0 = tq(g, a.Tm1, i, j, k);
   double tq1 = tq(g, a.Tm1, i, j + 1, k), tq2 = tq(g, a.Tm1, i, jp2, k);
   return vel * (a.q.quick_y[q] * a.T0[I3(g, i, j, k)] + a.q.quick_y[n2 + q] * a.T0[I3(g, i, j + 1, k)]) -
