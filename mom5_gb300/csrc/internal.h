@@ -226,6 +226,7 @@ struct MixArgs {
   const double* T;                    // tracer 0 at taum1 (tracer n at + n*g.n3)
   double* out;                        // fused: T(taup1); else th_tendency (tracer n at + n*g.n3)
   int fused;
+  float one = 1.0f;                   // a factor that the compiler cannot see to be 1 (mixed_stream.cuh)
 };
 
 // Arguments of the FP64 explicit update.

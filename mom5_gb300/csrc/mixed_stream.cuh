@@ -61,9 +61,8 @@ DEVI f2 sub2(f2 a, f2 b) { return fma2(b, 0xbf800000bf800000ULL, a); }
 // The sum of a product m and b.  The assembler contracts mul.rn.f32x2 followed by
 // add.rn.f32x2 (or by an fma with the constant factor 1) into one fused
 // multiply-add, also under -fmad=false (measured: the fused result's bits).  With
-// a factor 1 that it cannot see -- blockDim.y, 1 in every launch -- the sum stays
+// a factor 1 that it cannot see -- one, from the kernel's arguments -- the sum stays
 // a rounding of its own: the product by 1 is exact.
-DEVI f2 opaque_one() { return dup(__uint_as_float(0x3f800000u * blockDim.y)); }
 DEVI f2 addm2(f2 m, f2 b, f2 one) { return fma2(m, one, b); }
 DEVI f2 sel2(bool p, f2 a, f2 b) { return p ? a : b; }
 
@@ -194,7 +193,7 @@ DEVI void stream_tile(const MixArgs& a, int n0, int tile_x, int tile_y, int k0, 
     else ftp[q] = 0ULL;
   }
   float wk_prev = 0.f;
-  const f2 one = opaque_one();
+  const f2 one = dup(a.one);
 
   for (int k = ks; k < k1; ++k) {
     const int kp3 = k + 3 < g.nk ? k + 3 : nkm1;
