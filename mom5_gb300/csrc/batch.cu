@@ -352,7 +352,7 @@ int mom5gpu_batch_create(mom5gpu_domain* const* domains, int n, mom5gpu_batch** 
       }
     }
   } else {
-    int rc = prepare_batch_mixed();
+    int rc = prepare_mixed(b->ntr, true);
     if (rc) {
       mom5gpu_batch_destroy(b);
       return fail(nullptr, rc, "batch_create: kernel attributes");

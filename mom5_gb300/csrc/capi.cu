@@ -679,6 +679,8 @@ int mom5gpu_tracer_advect_init(mom5gpu_domain* d) {
     rc = quicker_init(d, dxt, dyt);
     if (rc) return rc;
   }
+  if (d->opt.precision == MOM5GPU_PRECISION_MIXED && prepare_mixed(d->dims.num_prog_tracers, false) != MOM5GPU_OK)
+    return cuda_fail(d, cudaGetLastError(), "precision form: kernel attributes");
   d->advect_ready = true;
   return MOM5GPU_OK;
 }

@@ -439,10 +439,13 @@ long stream_tiles(const Geo& g, int rows);
 int stream_levels(long tiles, int nk, int ntr, int rows);
 // the tracers of a (at most 10) of one domain, outputs numbered from n0
 int launch_mixed_stream(mom5gpu_domain* d, const MixArgs& a, int n0);
-// persistent kernel over a batch's items; the attributes are set before any graph capture
+// persistent kernel over a batch's items
 int launch_batch_mixed(const MixArgs* mix, const BatchWork& w, int ntr, int tuned_rows, int blocks_per_sm, int sms,
                        int* counter, cudaStream_t s);
-int prepare_batch_mixed();
+// Attributes of the kernels that up to ntr tracers may take, one domain or batched: they
+// belong to the device, so every precision-form domain (tracer_advect_init) and batch
+// sets them for its own, before any launch or capture.
+int prepare_mixed(int ntr, bool batch);
 
 // ---- precision form (k_mixed.cu) ----
 int launch_mdfl_mixed(mom5gpu_domain* d, int n_first, int ntr, int taum1, int tau, int taup1, double dtime,

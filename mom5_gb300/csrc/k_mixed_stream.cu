@@ -70,12 +70,6 @@ template <int NP, int ZR>
 int run(mom5gpu_domain* d, const MixArgs& a, int n0) {
   const Geo& g = d->geo;
   constexpr size_t smem = sizeof(StreamSmem<NP, ZR>);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(k_mdfl_stream<NP, ZR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_fail(d, e, "mixed kernel attribute");
-    configured = true;
-  }
   const int L = stream_levels(tiles_of(g, ZR), g.nk, a.ntr, ZR);
   dim3 grid((g.ni + TI - 1) / TI, (g.nj + ZR - 5) / (ZR - 4), (g.nk + L - 1) / L);
   k_mdfl_stream<NP, ZR><<<grid, 32 * ZR, smem, d->stream>>>(a, n0, L);
@@ -91,17 +85,17 @@ int run_batch(const MixArgs* m, const BatchWork& w, int bps, int sms, int* count
   return MOM5GPU_OK;
 }
 
+// The dynamic shared memory of every tile height of NP pairs, on the current device.
 template <int NP, int ZR>
-int configure_batch() {
-  return cudaFuncSetAttribute(kb_mdfl_stream<NP, ZR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sizeof(StreamSmem<NP, ZR>)) == cudaSuccess
-             ? 0
-             : 1;
+bool configure(bool batch) {
+  const void* k = batch ? (const void*)kb_mdfl_stream<NP, ZR> : (const void*)k_mdfl_stream<NP, ZR>;
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StreamSmem<NP, ZR>)) ==
+         cudaSuccess;
 }
 
 template <int NP>
-int configure_batch_rows() {
-  return configure_batch<NP, 16>() | configure_batch<NP, stream_rows(NP)>() | configure_batch<NP, 24>();
+bool configure_rows(bool batch) {
+  return configure<NP, 16>(batch) && configure<NP, stream_rows(NP)>(batch) && configure<NP, 24>(batch);
 }
 
 // f<NP, ZR>() for ntr tracers (1..10) and a tile height of stream_tile_rows
@@ -153,11 +147,13 @@ int launch_mixed_stream(mom5gpu_domain* d, const MixArgs& a, int n0) {
   return STREAM_DISPATCH(run, d, a, n0);
 }
 
-int prepare_batch_mixed() {
-  return configure_batch_rows<1>() | configure_batch_rows<2>() | configure_batch_rows<3>() |
-                 configure_batch_rows<4>() | configure_batch_rows<5>()
-             ? MOM5GPU_ECUDA
-             : MOM5GPU_OK;
+int prepare_mixed(int ntr, bool batch) {
+  const int np = ntr < 10 ? (ntr + 1) / 2 : 5;
+  return (np < 1 || configure_rows<1>(batch)) && (np < 2 || configure_rows<2>(batch)) &&
+                 (np < 3 || configure_rows<3>(batch)) && (np < 4 || configure_rows<4>(batch)) &&
+                 (np < 5 || configure_rows<5>(batch))
+             ? MOM5GPU_OK
+             : MOM5GPU_ECUDA;
 }
 
 int launch_batch_mixed(const MixArgs* mix, const BatchWork& w, int ntr, int tuned_rows, int blocks_per_sm, int sms,
