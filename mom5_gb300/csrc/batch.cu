@@ -472,10 +472,12 @@ int mom5gpu_batch_autotune(mom5gpu_batch* b, double dtime, char* report, size_t 
   struct Cand {
     int rows, tj, bps;
   };
-  static const Cand kMixed[] = {{32, 0, 2}, {16, 0, 2}, {24, 0, 2}};
-  static const Cand kFp64[] = {{32, 2, 2}, {32, 4, 2}, {32, 8, 2}, {32, 16, 2}};
-  std::vector<Cand> cands = b->prec == MOM5GPU_PRECISION_MIXED ? std::vector<Cand>(kMixed, kMixed + 3)
-                                                                 : std::vector<Cand>(kFp64, kFp64 + 4);
+  std::vector<Cand> cands = {{32, 2, 2}, {32, 4, 2}, {32, 8, 2}, {32, 16, 2}};
+  if (b->prec == MOM5GPU_PRECISION_MIXED) {  // tile heights, each once (32: by the tracer count)
+    cands = {{32, 0, 2}};
+    for (int rows : {16, 24})
+      if (stream_tile_rows(rows, b->ntr, true) != stream_tile_rows(32, b->ntr, true)) cands.push_back({rows, 0, 2});
+  }
   std::vector<int> idx(b->doms.size()), par(b->doms.size(), 0);
   for (size_t i = 0; i < idx.size(); ++i) idx[i] = (int)i;
   std::string rep;

@@ -937,10 +937,16 @@ int mom5gpu_autotune(mom5gpu_domain* d, double dtime, char* report, size_t repor
   if (!d) return MOM5GPU_EINVAL;
   if (!d->advect_ready) return fail(d, MOM5GPU_ESTATE, "autotune before mom5gpu_tracer_advect_init");
   bool mixed = d->opt.precision == MOM5GPU_PRECISION_MIXED;
-  // candidate launch shapes: precision-form tile height (32: by the tracer count); FP64 y-pass rows per thread
-  const int kRows[] = {32, 16, 24};
-  const int kTj[] = {2, 4, 8, 16};
-  int ncand = mixed ? 3 : 4;
+  // candidate launch shapes: precision-form tile height (32: by the tracer count; the others
+  // where that is not their height); FP64 y-pass rows per thread
+  std::vector<int> cands = {2, 4, 8, 16};
+  if (mixed) {
+    const int ntr = d->dims.num_prog_tracers < 10 ? d->dims.num_prog_tracers : 10;
+    cands = {32};
+    for (int rows : {16, 24})
+      if (stream_tile_rows(rows, ntr, false) != stream_tile_rows(32, ntr, false)) cands.push_back(rows);
+  }
+  const int ncand = (int)cands.size();
   cudaEvent_t t0, t1;
   if (cudaEventCreate(&t0) != cudaSuccess) return fail(d, MOM5GPU_ECUDA, "autotune events");
   if (cudaEventCreate(&t1) != cudaSuccess) {
@@ -952,10 +958,10 @@ int mom5gpu_autotune(mom5gpu_domain* d, double dtime, char* report, size_t repor
   int bestc = 0, rc = MOM5GPU_OK;
   for (int c = 0; c < ncand && rc == MOM5GPU_OK; ++c) {
     if (mixed) {
-      d->tune_mixed_rows = kRows[c];
+      d->tune_mixed_rows = cands[c];
       d->tune_mixed_pf = 0;
     } else {
-      d->tune_y_tj = kTj[c];
+      d->tune_y_tj = cands[c];
     }
     rc = mom5gpu_tracer_advection_step(d, 1, 1, 2, dtime);  // warm-up
     cudaEventRecord(t0, d->stream);
@@ -972,8 +978,8 @@ int mom5gpu_autotune(mom5gpu_domain* d, double dtime, char* report, size_t repor
     ms /= 3.f;
     char line[96];
     if (mixed)
-      snprintf(line, sizeof(line), "rows=%d: %.3f ms; ", kRows[c], ms);
-    else snprintf(line, sizeof(line), "tj=%d: %.3f ms; ", kTj[c], ms);
+      snprintf(line, sizeof(line), "rows=%d: %.3f ms; ", cands[c], ms);
+    else snprintf(line, sizeof(line), "tj=%d: %.3f ms; ", cands[c], ms);
     rep += line;
     if (ms < best) {
       best = ms;
@@ -983,15 +989,15 @@ int mom5gpu_autotune(mom5gpu_domain* d, double dtime, char* report, size_t repor
   cudaEventDestroy(t0);
   cudaEventDestroy(t1);
   if (mixed) {
-    d->tune_mixed_rows = kRows[bestc];
+    d->tune_mixed_rows = cands[bestc];
   } else {
-    d->tune_y_tj = kTj[bestc];
+    d->tune_y_tj = cands[bestc];
   }
   if (rc) return rc;
   char line[64];
   if (mixed)
-    snprintf(line, sizeof(line), "chosen rows=%d", kRows[bestc]);
-  else snprintf(line, sizeof(line), "chosen tj=%d", kTj[bestc]);
+    snprintf(line, sizeof(line), "chosen rows=%d", cands[bestc]);
+  else snprintf(line, sizeof(line), "chosen tj=%d", cands[bestc]);
   rep += line;
   if (report && report_len) {
     strncpy(report, rep.c_str(), report_len - 1);
