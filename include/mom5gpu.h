@@ -450,7 +450,10 @@ int mom5gpu_check_finite(mom5gpu_domain* d, int n, int level, int* out);
 int mom5gpu_enable_timing(mom5gpu_domain* d, int on);
 /* Total device milliseconds and number of calls of a named section since
  * timing was enabled; synchronises the stream.  Sections: "mdfl", "mdfl_mixed",
- * "tracer_update", "barotropic", "upwind", "quicker". */
+ * "tracer_update", "barotropic", "upwind", "quicker", "batch".  The update of a
+ * whole MDFL step (mom5gpu_tracer_advection_step with every tracer on that scheme)
+ * runs inside the advection kernels: FP64 steps count as calls of "tracer_update",
+ * but their time is in "mdfl"; the precision form has it all in "mdfl_mixed". */
 int mom5gpu_timing_query(mom5gpu_domain* d, const char* section, double* total_ms, long* calls);
 /* Number of kernels this domain has launched since creation. */
 long mom5gpu_launch_count(const mom5gpu_domain* d);
