@@ -74,36 +74,22 @@ DEVI double twice(double x) {
   return double_of(mh < 0x00100000u ? (b << 1) | s : r);
 }
 
-// Arithmetic of an MDFL pass: sums on the FP64 pipe, the products whose bit is set
-// in MASK on the integer pipe.  The four of a face (d1*theta, c*theta, psi*Rj, the
-// mass flux) go there; with one more of the update's the passes took 0 to 3%
-// longer, with none 17 to 41% (z 1.71 -> 1.21 ms, x 1.67 -> 1.39, y 2.08 -> 1.77 for
-// 10 tracers on 360x270x50): by then the FP64 pipe is 65 to 76% busy, the adder and
-// logic pipe 50 to 57%, and the rest is latency at 20 to 31 warps per SM.
-template <unsigned MASK>
-struct Arith {
-  static DEVI double add(double a, double b) { return a + b; }
-  static DEVI double sub(double a, double b) { return a - b; }
-  static DEVI double mul(double a, double b) { return a * b; }
-  // product B of a face: theta, psi and Rj are often zero
-  template <int B>
-  static DEVI double face_mul(double a, double b) {
-    if constexpr ((MASK >> B) & 1) return mul_int<B == 2, B <= 2>(a, b);
-    return a * b;
-  }
-};
-using FaceArith = Arith<15>;
+// Products of an MDFL face, on the integer pipe: d1*theta, c*theta, psi*Rj and the mass
+// flux.  With one more, of the update's, the passes took 0 to 3% longer, with none 17 to
+// 41% (z 1.71 -> 1.21 ms, x 1.67 -> 1.39, y 2.08 -> 1.77 for 10 tracers on 360x270x50): by
+// then the FP64 pipe is 65 to 76% busy, the adder and logic pipe 50 to 57%, and the rest
+// is latency at 20 to 31 warps per SM.  theta, psi and Rj are often zero.
 
 // Sweby limiter psi (ocean_tracer_advect.F90:3868-3878).  With the limiter on
 // the reference forms psi*(1-1) + max(...)*1, with it off psi*1 + max(...)*0;
 // for finite psi both reduce to the selected term exactly.
-template <bool SWEBY, class Ar>
+template <bool SWEBY>
 DEVI double limiter(double theta, double d0, double d1, double c) {
-  double lin = Ar::add(d0, Ar::template face_mul<0>(d1, theta));
+  double lin = d0 + mul_int<false, true>(d1, theta);
   if (!SWEBY) return lin;
   // max(0, min(1, lin, c*theta)) on the bit patterns as integers: they order
   // non-negative values, and whichever of two negative ones is taken, 0 results
-  long long m = bits_of(lin), ct = bits_of(Ar::template face_mul<1>(c, theta));
+  long long m = bits_of(lin), ct = bits_of(mul_int<false, true>(c, theta));
   m = m < ct ? m : ct;
   m = m < 0x3ff0000000000000LL ? m : 0x3ff0000000000000LL;
   return double_of(m > 0 ? m : 0);
@@ -117,16 +103,16 @@ DEVI double limiter(double theta, double d0, double d1, double c) {
 // the division once, not once per branch; Tdn - p is computed as Tdn + (-p),
 // which IEEE defines to be the same operation, with -p formed on the integer
 // pipe.
-template <bool SWEBY, class Ar>
+template <bool SWEBY>
 DEVI double face_flux(double mf, double Rjm, double Rj, double Rjp, double Tp, double Tm, double d0, double d1,
                       double c) {
   long long b = bits_of(mf);
   bool pos = b > 0;                                                 // mf > 0
   bool neg = b < 0 && b != (long long)0x8000000000000000ULL;        // mf < 0
   double theta = div_seeded(pos ? Rjm : Rjp, add_1em30(Rj));
-  double psi = limiter<SWEBY, Ar>(theta, d0, d1, c);
-  double p = Ar::template face_mul<2>(psi, Rj);
-  double r = Ar::template face_mul<3>(mf, Ar::add(pos ? Tp : Tm, neg_if(p, !pos)));
+  double psi = limiter<SWEBY>(theta, d0, d1, c);
+  double p = mul_int<true, true>(psi, Rj);
+  double r = mul_int(mf, (pos ? Tp : Tm) + neg_if(p, !pos));
   return (pos || neg) ? r : 0.0;
 }
 
@@ -153,10 +139,9 @@ DEVI ZFace z_face(const MdflArgs& a, const Geo& g, int i, int j, int k, double d
 }
 // R(m) = (m(m) && m(m1)) ? T(m) - T(m1) : 0 with m1 = min(m+1, nk-1): the masked
 // vertical difference that the column march forms once per level
-template <class Ar>
 DEVI double z_rdiff(const MdflArgs& a, const Geo& g, const double* T, int i, int j, int m) {
   const int m1 = m + 1 < g.nk ? m + 1 : g.nk - 1;
-  return (a.mask2[IM(g, i, j, m)] && a.mask2[IM(g, i, j, m1)]) ? Ar::sub(T[I3(g, i, j, m)], T[I3(g, i, j, m1)])
+  return (a.mask2[IM(g, i, j, m)] && a.mask2[IM(g, i, j, m1)]) ? T[I3(g, i, j, m)] - T[I3(g, i, j, m1)]
                                                                  : 0.0;
 }
 
@@ -167,7 +152,6 @@ DEVI double z_rdiff(const MdflArgs& a, const Geo& g, const double* T, int i, int
 // operations, so every segment length gives the same bits.
 template <bool ALL, bool SWEBY, int MAXN, bool SEG = false>
 DEVI void mdfl_z_body(MdflArgs a, int bx, int by, int k0 = 0, int k1 = -1) {
-  using Ar = FaceArith;
   // ftp: flux through the top face; Rp, Rc: the masked differences R(k-1), R(k),
   // R(k) = (m(k) && m(k1)) ? T(k) - T(k1) : 0 with k1 = min(k+1, nk-1).  The
   // reference's Rjp at level k is R(k-1) (+0 at k = 0) and its Rjm is R(k+1), so
@@ -189,7 +173,7 @@ DEVI void mdfl_z_body(MdflArgs a, int bx, int by, int k0 = 0, int k1 = -1) {
       const double* T = a.T + n * a.tstride;
       ftp[n][t] = 0.0;
       Rp[n][t] = 0.0;
-      Rc[n][t] = (m0 && m1) ? Ar::sub(T[I3(g, i, j, 0)], T[I3(g, i, j, k1s)]) : 0.0;
+      Rc[n][t] = (m0 && m1) ? T[I3(g, i, j, 0)] - T[I3(g, i, j, k1s)] : 0.0;
     }
   } else {
     // the bottom face of level kq = k0-1, as the march forms it there
@@ -199,10 +183,10 @@ DEVI void mdfl_z_body(MdflArgs a, int bx, int by, int k0 = 0, int k1 = -1) {
 #pragma unroll 1
     for (int n = 0; n < a.ntr; ++n) {
       const double* T = a.T + n * a.tstride;
-      const double Rjp = kq > 0 ? z_rdiff<Ar>(a, g, T, i, j, kq - 1) : 0.0;
-      const double Rj = z_rdiff<Ar>(a, g, T, i, j, kq);
-      const double Rjm = z_rdiff<Ar>(a, g, T, i, j, k0);
-      ftp[n][t] = fm ? face_flux<SWEBY, Ar>(f.massflux, Rjm, Rj, Rjp, T[I3(g, i, j, k0)], T[I3(g, i, j, kq)], f.d0,
+      const double Rjp = kq > 0 ? z_rdiff(a, g, T, i, j, kq - 1) : 0.0;
+      const double Rj = z_rdiff(a, g, T, i, j, kq);
+      const double Rjm = z_rdiff(a, g, T, i, j, k0);
+      ftp[n][t] = fm ? face_flux<SWEBY>(f.massflux, Rjm, Rj, Rjp, T[I3(g, i, j, k0)], T[I3(g, i, j, kq)], f.d0,
                                              f.d1, f.c)
                      : 0.0;
       Rp[n][t] = Rj;
@@ -237,16 +221,16 @@ DEVI void mdfl_z_body(MdflArgs a, int bx, int by, int k0 = 0, int k1 = -1) {
       double Tkp1 = T[I3(g, i, j, kp1)], Tkp2 = T[I3(g, i, j, kp2)];
       double Rjp = Rp[n][t];
       double Rj = Rc[n][t];
-      double Rjm = (mkp1 && mkp2) ? Ar::sub(Tkp1, Tkp2) : 0.0;
+      double Rjm = (mkp1 && mkp2) ? Tkp1 - Tkp2 : 0.0;
       Rp[n][t] = Rj;
       Rc[n][t] = Rjm;
-      double fbt = fm ? face_flux<SWEBY, Ar>(massflux, Rjm, Rj, Rjp, Tkp1, Tk, d0, d1, c) : 0.0;
-      double div = Ar::add(Ar::mul(datr, Ar::sub(fbt, ftp[n][t])), Ar::mul(Tk, wdiff));
+      double fbt = fm ? face_flux<SWEBY>(massflux, Rjm, Rj, Rjp, Tkp1, Tk, d0, d1, c) : 0.0;
+      double div = datr * (fbt - ftp[n][t]) + Tk * wdiff;
       double tm;
       if (!ALL) {
-        tm = Ar::add(Tk, Ar::mul(dtr, div));
+        tm = Tk + dtr * div;
       } else {
-        tm = Ar::add(Tk, div_seeded(Ar::mul(div, a.dtime), rdz));
+        tm = Tk + div_seeded(div * a.dtime, rdz);
       }
       a.tz[n * g.n3 + p] = tm;
       ftp[n][t] = fbt;
@@ -315,7 +299,7 @@ __host__ __device__ inline int x_blocks(const Geo& g) { return (g.ni + kXCells -
 // x-face i of row (j,k): fluxes of every tracer into sm[n][slot].  Rs[n][r-1..r+1]
 // hold the masked differences R of faces i-1, i, i+1 (the reference's Rjm, Rj,
 // Rjp), each formed once per block.
-template <bool SWEBY, int MAXN, class Ar>
+template <bool SWEBY, int MAXN>
 DEVI void x_face(const MdflArgs& a, int i, int j, int k, double (*sm)[kTX], int slot, const double (*Rs)[kTX + 2],
                  int r) {
   const Geo& g = a.g;
@@ -330,13 +314,12 @@ DEVI void x_face(const MdflArgs& a, int i, int j, int k, double (*sm)[kTX], int 
 #pragma unroll 1
   for (int n = 0; n < a.ntr; ++n) {
     double tB = tz_halo(a, n, i, j, k), tC = tz_halo(a, n, i + 1, j, k);
-    sm[n][slot] = fm ? face_flux<SWEBY, Ar>(massflux, Rs[n][r - 1], Rs[n][r], Rs[n][r + 1], tB, tC, d0, d1, c) : 0.0;
+    sm[n][slot] = fm ? face_flux<SWEBY>(massflux, Rs[n][r - 1], Rs[n][r], Rs[n][r + 1], tB, tC, d0, d1, c) : 0.0;
   }
 }
 
 template <bool ALL, bool SWEBY, int MAXN>
 DEVI void mdfl_x_body(MdflArgs a, int bx, int by, int bz) {
-  using Ar = FaceArith;
   __shared__ double sm[MAXN][kTX], Rs[MAXN][kTX + 2];
   const Geo& g = a.g;
   int i0 = bx * kXCells + 1;
@@ -351,11 +334,11 @@ DEVI void mdfl_x_body(MdflArgs a, int bx, int by, int bz) {
     bool ma = a.mask2[IM(g, f, j, k)], mb = a.mask2[IM(g, f + 1, j, k)];
 #pragma unroll 1
     for (int n = 0; n < a.ntr; ++n) {
-      Rs[n][sl] = (mb && ma) ? Ar::sub(tz_halo(a, n, f + 1, j, k), tz_halo(a, n, f, j, k)) : 0.0;
+      Rs[n][sl] = (mb && ma) ? tz_halo(a, n, f + 1, j, k) - tz_halo(a, n, f, j, k) : 0.0;
     }
   }
   __syncthreads();
-  if (i <= g.ni) x_face<SWEBY, MAXN, Ar>(a, i, j, k, sm, t, Rs, t + 1);
+  if (i <= g.ni) x_face<SWEBY, MAXN>(a, i, j, k, sm, t, Rs, t + 1);
   __syncthreads();
   if (t == 0 || i > g.ni) return;
   bool mk = a.mask2[IM(g, i, j, k)];
@@ -369,12 +352,12 @@ DEVI void mdfl_x_body(MdflArgs a, int bx, int by, int bz) {
   for (int n = 0; n < a.ntr; ++n) {
     double Tk = a.T[n * a.tstride + p];
     double tm = a.tz[n * g.n3 + p];
-    double s = Ar::add(Ar::sub(sm[n][t - 1], sm[n][t]), Ar::mul(Tk, divx));
+    double s = sm[n][t - 1] - sm[n][t] + Tk * divx;
     if (!ALL) {
-      tm = Ar::add(tm, Ar::mul(coef, s));
+      tm = tm + coef * s;
     } else {
-      double w1 = mk ? Ar::mul(datr, s) : 0.0;
-      tm = Ar::add(tm, div_seeded(Ar::mul(w1, a.dtime), rdz));
+      double w1 = mk ? datr * s : 0.0;
+      tm = tm + div_seeded(w1 * a.dtime, rdz);
     }
     a.tx[n * g.n3 + p] = tm;
   }
@@ -408,16 +391,16 @@ DEVI YFace y_geom(const MdflArgs& a, int i, int j, int k, bool& m0, bool& m1) {
   return f;
 }
 // Flux of tracer n through face j, carrying Ra/Rb; tB returns tx at row j.
-template <bool SWEBY, class Ar>
+template <bool SWEBY>
 DEVI double y_flux(const MdflArgs& a, const YFace& f, int i, int j, int k, int n, int t, double (*Ra)[kMdflThreads],
                    double (*Rb)[kMdflThreads], double& tB) {
   tB = tx_halo(a, n, i, j, k);
   double tC = tx_halo(a, n, i, j + 1, k), tD = tx_halo(a, n, i, j + 2, k);
   double Rjm = Ra[n][t], Rj = Rb[n][t];
-  double Rjp = (f.m3 && f.m2) ? Ar::sub(tD, tC) : 0.0;
+  double Rjp = (f.m3 && f.m2) ? tD - tC : 0.0;
   Ra[n][t] = Rj;
   Rb[n][t] = Rjp;
-  return f.fm ? face_flux<SWEBY, Ar>(f.massflux, Rjm, Rj, Rjp, tB, tC, f.d0, f.d1, f.c) : 0.0;
+  return f.fm ? face_flux<SWEBY>(f.massflux, Rjm, Rj, Rjp, tB, tC, f.d0, f.d1, f.c) : 0.0;
 }
 
 // What a whole step leaves outside the compute domain, by the threads of its outer
@@ -444,7 +427,6 @@ static __device__ __noinline__ void step_edges(double* T1, double* th, double tn
 // and Rb only.
 template <bool ALL, bool SWEBY, int MAXN>
 DEVI void mdfl_y_body(MdflArgs a, int TJ, int bx, int by, int bz) {
-  using Ar = FaceArith;
   __shared__ double fprev[MAXN][kMdflThreads];
   __shared__ double Ra[MAXN][kMdflThreads], Rb[MAXN][kMdflThreads];
   const Geo& g = a.g;
@@ -465,10 +447,10 @@ DEVI void mdfl_y_body(MdflArgs a, int TJ, int bx, int by, int bz) {
     for (int n = 0; n < a.ntr; ++n) {
       double tA = tx_halo(a, n, i, j0 - 2, k), tB = tx_halo(a, n, i, j0 - 1, k);
       double tC = tx_halo(a, n, i, j0, k);
-      Ra[n][t] = (m1 && m0) ? Ar::sub(tB, tA) : 0.0;
-      Rb[n][t] = (f.m2 && m1) ? Ar::sub(tC, tB) : 0.0;
+      Ra[n][t] = (m1 && m0) ? tB - tA : 0.0;
+      Rb[n][t] = (f.m2 && m1) ? tC - tB : 0.0;
       double tb;
-      fprev[n][t] = y_flux<SWEBY, Ar>(a, f, i, j0 - 1, k, n, t, Ra, Rb, tb);
+      fprev[n][t] = y_flux<SWEBY>(a, f, i, j0 - 1, k, n, t, Ra, Rb, tb);
     }
   }
   for (int j = j0; j <= j1; ++j) {
@@ -490,24 +472,24 @@ DEVI void mdfl_y_body(MdflArgs a, int TJ, int bx, int by, int bz) {
 #pragma unroll 1
     for (int n = 0; n < a.ntr; ++n) {
       double tm;  // tracer_mdfl after the x pass at (i, j, k)
-      double fc = y_flux<SWEBY, Ar>(a, f, i, j, k, n, t, Ra, Rb, tm);
+      double fc = y_flux<SWEBY>(a, f, i, j, k, n, t, Ra, Rb, tm);
       double Tk = a.T[n * a.tstride + p];
       double fp = fprev[n][t];
       double out;
       if (!ALL) {
-        tm = Ar::add(tm, Ar::mul(coef, Ar::sub(fp, fc)));
-        tm = Ar::add(tm, Ar::mul(div_pair(Ar::mul(a.dtime, Tk), rdz, rr_h, rr_l), corr));
+        tm = tm + coef * (fp - fc);
+        tm = tm + div_pair(a.dtime * Tk, rdz, rr_h, rr_l) * corr;
       } else {
-        double w1 = Ar::add(mk ? Ar::mul(datr, Ar::sub(fp, fc)) : 0.0, Ar::mul(Tk, corr));
-        tm = Ar::add(tm, div_pair(Ar::mul(w1, a.dtime), rdz, rr_h, rr_l));
+        double w1 = (mk ? datr * (fp - fc) : 0.0) + Tk * corr;
+        tm = tm + div_pair(w1 * a.dtime, rdz, rr_h, rr_l);
       }
-      out = mk ? div_pair(Ar::mul(rdz, Ar::sub(tm, Tk)), a.dtime, rdt_h, rdt_l) : 0.0;
+      out = mk ? div_pair(rdz * (tm - Tk), a.dtime, rdt_h, rdt_l) : 0.0;
       double* th = a.th + n * g.n3;
-      out = a.th_fresh ? plus_zero(out) : Ar::add(th[p], out);  // +0 + out == plus_zero(out)
+      out = a.th_fresh ? plus_zero(out) : th[p] + out;  // +0 + out == plus_zero(out)
       th[p] = out;
       if (a.Tp1) {  // the explicit update (ocean_tracer.F90:2341-2350)
         double* T1 = a.Tp1 + n * a.tstride;
-        const double tn = Ar::mul(Ar::add(mul_int<false, true>(rm1, Tk), a.dtime * out), rdzr);
+        const double tn = (mul_int<false, true>(rm1, Tk) + a.dtime * out) * rdzr;
         T1[p] = tn;
         if (edge) step_edges(T1 + (p - I2(g, i, j)), th + (p - I2(g, i, j)), tn, i, j, g.ni, g.nj, g.cx, g.cy);
       }

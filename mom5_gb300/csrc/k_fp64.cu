@@ -133,7 +133,7 @@ static int z_segment_levels(const Geo& g) {
 // Rows per thread of the y pass for cols = columns*levels threads and nj rows: each
 // strip forms one face more than it has rows, so as long as the strips give every
 // SM 12 warps, longer ones are cheaper (120x80x30, 2 tracers: 104 us a step with 4
-// rows, 112 with 2, 121 with 8; 37x29x12: 25, 32 and 44 with 2, 4 and 8, 28 with 1).
+// rows, 110 with 2, 117 with 8; 37x29x12: 25, 31 and 44 with 2, 4 and 8, 28 with 1).
 int y_strip_rows(long cols, long nj) {
   int TJ = 16;
   while (TJ > 2 && cols * ((nj + TJ - 1) / TJ) < 152L * 32 * 12) TJ /= 2;
@@ -165,8 +165,8 @@ static void run_mdfl(const MdflArgs& a, int pass, cudaStream_t s) {
   const Geo& g = a.g;
   const unsigned nx = (g.ni + 127) / 128, nt = SPLIT ? a.ntr : 1;
   // programmatic dependents hide a launch each, which domains of a few blocks per SM feel
-  // (37x29x12, 2 tracers: with SPLIT 24.6 us a step against 43.5); on larger ones the waiting
-  // blocks cost more than that (120x80x30 and 360x270x50: 3%)
+  // (37x29x12, 2 tracers: with SPLIT 24.7 us a step against 31.8); on larger ones the waiting
+  // blocks cost more than that (120x80x30, 2 tracers: 103 and 114; 360x270x50, 10 tracers: 4%)
   const bool dep = (long)nx * g.nj * g.nk < 152L * 8;
   auto launch = [&](auto k, dim3 grid, int threads, auto... args) {
     if (dep) launch_pdl(k, grid, dim3(threads), s, args...);
@@ -187,8 +187,9 @@ static void run_mdfl(const MdflArgs& a, int pass, cudaStream_t s) {
 
 // Below 16 warps of cells per SM the passes are chains of latency on an idle chip,
 // and the terms a face's tracers share are cheaper formed again: each tracer gets
-// blocks of its own (37x29x12 cells, 2 tracers, with programmatic dependents: 24.6 us a
-// step against 43.5).
+// blocks of its own (37x29x12 cells, 2 tracers, with programmatic dependents: 24.7 us a
+// step against 35.3; 60x40x20: 34.7 and 43.9; 60x50x25, 4 tracers, just above the line: 85.5
+// and 77.2).
 template <bool ALL, bool SWEBY>
 static void run_mdfl_n(const MdflArgs& a, int pass, cudaStream_t s) {
   const Geo& g = a.g;

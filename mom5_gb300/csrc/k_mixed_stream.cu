@@ -13,8 +13,9 @@ namespace {
 // pairs, two blocks of 16 rows (64 registers) overlap each other's barriers:
 // 720x540x50 cells, 4 tracers, 895 us against 978 to 1033 with 12, 20, 24 or 32 rows; 2
 // tracers 674 against 734 to 871.  Three pairs and more do not fit twice; one block
-// of 20 rows (96 registers) is the largest without spills: 1440x1080x50, 10
-// tracers, 7.10 ms against 7.54 with 16 rows and 8.43 with 24.
+// of 20 rows (96 registers) is the largest that spills next to nothing (8 bytes with five
+// pairs, against 52 with 24 rows): 1440x1080x50, 10 tracers, 7.10 ms against 7.54 with
+// 16 rows and 8.43 with 24.
 constexpr int stream_rows(int np) { return np <= 2 ? 16 : 20; }
 // The same for the persistent kernel, whose registers hold its work list too: a height
 // that spills there pays for each spill with a trip to L2, as the tiles leave no L1
@@ -123,9 +124,10 @@ long stream_tiles(const Geo& g, int rows) { return tiles_of(g, rows); }
 // prologue and the z pass of the level above).  Of all cuts the cheapest by this
 // model, in level times of a block alone on its SM: each SM works through its
 // share of the blocks one after another, two that share the SM taking 1.55 of one
-// (measured).  255x181x40, 4 tracers: 131 us with segments of 14 levels against 174
-// for whole columns; 300x200x35: 120 (9 levels) against 173; 37x29x12, 2 tracers:
-// 12 (2 levels) against 34.
+// (measured).  Its choice, whole columns and the best of all lengths, us a step:
+// 255x181x40, 4 tracers 127 (8 levels), 174, 124; 300x200x35, 4 tracers 122 (12 levels),
+// 172, 120; 330x210x30, 10 tracers 267 (10 levels), 365, 255; 500x300x40, 4 tracers 292 (20
+// levels), 308, 292; 37x29x12, 2 tracers 12.3 (2 levels), 34.8, 12.3.
 int stream_levels(long tiles, int nk, int ntr, int rows) {
   const bool two = stream_blocks((ntr + 1) / 2, rows) == 2;
   int best = nk;
