@@ -509,6 +509,23 @@ DEVI double bt_mul(double a, double b) {
   if constexpr (INT) return mul_int<ZA, true>(a, b);
   return a * b;
 }
+// 0.5*x in the subcycle.  LOOP: the multiplication in a loop over the lanes that need it
+// (rare_lanes), which the kernels of the default form keep: half_exact's longer
+// sequence makes those that load early take 46 and 56 registers instead of 48 and 64
+// (batches 56 and 56 instead of 62 and 64), and more of their blocks land on one SM
+// while others have none (60 subcycles, us a step: B grid 669 -> 752 at 82950 columns, 1044
+// -> 1082 at 127167, batches 413 -> 495 at 29440, 952 -> 989 at 88192; above 160000 columns
+// 1 to 5% less).
+template <bool LOOP>
+DEVI double bt_half(double x) {
+  if constexpr (!LOOP) return half_exact(x);
+  const long long b = bits_of(x);
+  const unsigned e = (unsigned)((unsigned long long)b >> 52) & 0x7ffu;
+  const bool normal = e - 2u < 0x7fdu;  // 2 <= e <= 0x7fe: the exponent lowered by one
+  double r = double_of(normal ? b - (1LL << 52) : b);
+  rare_lanes(!(normal || (b << 1) == 0), [&] { r = 0.5 * x; });
+  return r;
+}
 // DIV_UD at (i,j) (ocean_operators.F90:507-608), halo_in = halo_out = 1.
 DEVI double div_ud(const BtArgs& a, const double* u, const double* v, int i, int j) {
   const Geo& g = a.g;
@@ -537,14 +554,14 @@ DEVI double div_ud(const BtArgs& a, const double* u, const double* v, int i, int
 
 // B-grid DIV_UD from the stored products uh = u*dyu, vh = v*dxu: the same
 // operations as div_ud on the same values, without recomputing the products.
-template <bool INT = false>
+template <bool INT = false, bool LOOP = false>
 DEVI double div_ud_bh(const Geo& g, double datr, const double* uh, const double* vh, int i, int j) {
   if (i < 1 || j < 1) return 0.0;
   long q = I2(g, i, j), qw = q - 1, qs = q - g.nxd, qsw = qs - 1;
-  double uh_bay = half_exact(uh[q] + uh[qs]);
-  double vh_bax = half_exact(vh[q] + vh[qw]);
-  double uhim_bay = half_exact(uh[qw] + uh[qsw]);
-  double vhjm_bax = half_exact(vh[qs] + vh[qsw]);
+  double uh_bay = bt_half<LOOP>(uh[q] + uh[qs]);
+  double vh_bax = bt_half<LOOP>(vh[q] + vh[qw]);
+  double uhim_bay = bt_half<LOOP>(uh[qw] + uh[qsw]);
+  double vhjm_bax = bt_half<LOOP>(vh[qs] + vh[qsw]);
   return bt_mul<INT>(datr, (uh_bay - uhim_bay) + (vh_bax - vhjm_bax));
 }
 
@@ -670,17 +687,18 @@ DEVI void bt_mom_b_body(BtArgs a, int so, int sn, int bx) {
   const Loaded<EARLY, double> uo(a.ubt + (so * g.n2 + q)), vo(a.vbt + (so * g.n2 + q));
   const Loaded<EARLY, double> fu(a.forcing_u + q), fv(a.forcing_v + q), cori1(a.cori1 + q), cori2(a.cori2 + q);
   const Loaded<EARLY, double> dyu(a.dyu + q), dxu(a.dxu + q);
-  const double hf = half_exact(load_early<EARLY>(a.f + q));  // 0.5*f; -0.5*f is its negation
+  constexpr bool LOOP = INT || EARLY;  // the default form's kernels
+  const double hf = bt_half<LOOP>(load_early<EARLY>(a.f + q));  // 0.5*f; -0.5*f is its negation
   if (EARLY) bt_after_previous();
   double gx = 0.0, gy = 0.0;
   if (i <= g.ni && j <= g.nj) {
     const double* ps = a.ps;
     if (!is_zero(um)) {
       double p00 = ps[q], p10 = ps[q + 1], p01 = ps[q + g.nxd], p11 = ps[q + g.nxd + 1];
-      double p_fay = half_exact(p00 + p01);
-      double p_fax = half_exact(p00 + p10);
-      double pip_fay = half_exact(p10 + p11);
-      double pjp_fax = half_exact(p01 + p11);
+      double p_fay = bt_half<LOOP>(p00 + p01);
+      double p_fax = bt_half<LOOP>(p00 + p10);
+      double pip_fay = bt_half<LOOP>(p10 + p11);
+      double pjp_fax = bt_half<LOOP>(p01 + p11);
       gx = mask_mul((pip_fay - p_fay) * dxur, um);
       gy = mask_mul((pjp_fax - p_fax) * dyur, um);
     }
@@ -824,7 +842,7 @@ DEVI void bt_corr_pred_body(BtArgs a, int so, int sn, double wgt, int bx) {
   const Loaded<EARLY, double> bar(a.eta_bar + q), su(a.udrho_u + q), sv(a.udrho_v + q), rho_g(a.rho_g + q), patm(a.patm + q);
   if (EARLY) bt_after_previous();
   const double un = a.ubt[sn * n2 + q], vn = a.vbt[sn * n2 + q];
-  double dv = div_ud_bh<INT>(g, datr, a.uhb + sn * n2, a.vhb + sn * n2, i, j);
+  double dv = div_ud_bh<INT, true>(g, datr, a.uhb + sn * n2, a.vhb + sn * n2, i, j);
   double tmp = is_zero(tm) ? 0.0 : mask_mul(-dv, tm);
   const double st = tmp + steady;
   double en = eo + bt_mul<INT>(a.dtbt_rho0r, st);
