@@ -111,7 +111,7 @@ struct mom5gpu_domain {
   unsigned* bt_sync = nullptr;  // arrival counter of the cooperative barotropic subcycle's grid barriers
   int tune_y_tj = 0;         // FP64 y-pass rows per thread
   bool bt_early = true;      // the barotropic subcycles load early (BtResident), set by barotropic_init
-  int bt_fused = 0;          // exact B-grid subcycles: 0 three launches each, 1 one launch each,
+  int bt_fused = 0;          // exact B-grid subcycles: 0 two launches each, 1 one launch each,
                              // 2 all in one cooperative launch
   int coop_blocks = 0;       // resident blocks per SM of the cooperative subcycle kernel (0: not queried, -1: none)
   int coop_sms = 0;          // SMs of the device

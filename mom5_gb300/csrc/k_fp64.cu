@@ -1437,16 +1437,21 @@ static int coop_resident(mom5gpu_domain* d, const void* kernel) {
 }
 
 // Every SM gets the same number of blocks, no more than the walk has blocks of
-// work for and no more than can be resident.
+// work for, than can be resident, and than kCoopBlocks: with more, each grid barrier
+// waits for more arrivals and the last round of the walk is emptier (a step of 40
+// subcycles, us, with 5, 7 and 12 blocks: 500x404 columns 1483, 1525, 1741; 700x500 2019,
+// 2168, 2635; 1440x1080 9113, 8086, 8202).
+constexpr int kCoopBlocks = 7;
 static int launch_bt_coop(mom5gpu_domain* d, const BtArgs& a, cudaStream_t s) {
   int rc = ensure_wait_words(d);
   if (rc) return rc;
   if (!d->coop_blocks) d->coop_blocks = coop_resident(d, (const void*)k_bt_coop);
   if (d->coop_blocks < 0) return MOM5GPU_EUNSUPPORTED;
   const Geo& g = a.g;
-  const int nvb = ((g.ni + 2 + 127) / 128) * (g.nj + 2);
+  const int nvb = (int)((g.n2 + 127) / 128);  // k_bt_coop's
   int bps = (nvb + d->coop_sms - 1) / d->coop_sms;
   if (bps > d->coop_blocks) bps = d->coop_blocks;
+  if (bps > kCoopBlocks) bps = kCoopBlocks;
   cudaMemsetAsync(d->bt_sync, 0, sizeof(unsigned), s);
   BtArgs av = a;
   unsigned* ctr = d->bt_sync;
@@ -1456,15 +1461,14 @@ static int launch_bt_coop(mom5gpu_domain* d, const BtArgs& a, cudaStream_t s) {
   return e == cudaSuccess ? MOM5GPU_OK : cuda_fail(d, e, "barotropic subcycles (cooperative launch)");
 }
 
-// Form of the exact B-grid subcycles: 0 three launches each (replayed from a
+// Form of the exact B-grid subcycles: 0 two launches each (replayed from a
 // CUDA graph; the default), 1 one launch each (k_bt_fused, the ring
 // recomputed), 2 all of a step in one cooperative launch (k_bt_coop).  Measured
-// on GB300 both alternatives are slower on every domain tried: the one-launch
-// form adds about 11% FP64 work for its ring to a loop bound by the FP64 pipe;
-// the cooperative launch holds 7 blocks of 72 registers per SM (28 warps)
-// against the three kernels' 16 blocks of 30-32 registers (64 warps), which
-// hide the FP64 latency better, and a grid barrier across about a thousand
-// blocks costs as much as a launch gap of the graph replay.
+// on GB300 both alternatives are slower on every domain tried (360x300, 80
+// subcycles: 1.08, 1.68 and 1.89 ms a step): the one-launch form adds about 11% FP64
+// work for its ring to a loop bound by the FP64 pipe; the cooperative launch keeps
+// every product on that pipe and the predictor a phase of its own, and each of its
+// three grid barriers a subcycle costs as much as a launch gap of the graph replay.
 static int bt_form(const mom5gpu_domain* d, const BtArgs& a) {
   if (a.cgrid) return 0;
   if (a.btf) return d->bt_fused == 1 ? 1 : 0;  // the precision form has no cooperative form

@@ -77,6 +77,27 @@ def test_precision_form(gpu_lib, oracle_lib, ni, nj, cx, cy, step_b):
     d.close()
 
 
+@pytest.mark.parametrize("fusion", [1, 2])
+@pytest.mark.parametrize("ni,nj", [(69, 76), (411, 301), (577, 545)])
+def test_one_launch_forms(gpu_lib, ni, nj, fusion):
+    """One launch per subcycle, and one for all of them, whose blocks walk the columns
+    in one round on 411x301 and in three on 577x545: the bits of the default form."""
+    capi = gpu_lib
+    from mom5_gb300 import harness
+    _, dom = domain(ni, nj, True, False)
+    out = {}
+    for form in (0, fusion):
+        d = harness.load(dom, options=capi.default_options(barotropic_time_stepping_B=1))
+        d.barotropic_init(dtuv=7 * DTBT / 2, dtbt=DTBT)
+        d.set_barotropic_fusion(form)
+        d.update_ocean_barotropic(1, 2)
+        d.synchronize()
+        out[form] = [d.get(getattr(capi.F, k.upper()), level=2) for k in LEVEL_FIELDS]
+        d.close()
+    for k, x, y in zip(LEVEL_FIELDS, out[0], out[fusion]):
+        assert np.array_equal(x, y), k
+
+
 # columns of the lists, each domain rounded up to blocks of 128: about 89000, 119000 and 346000
 LISTS = [[(200, 150), (180, 160), (170, 165)], [(200, 150), (180, 160), (170, 165), (251, 117)],
          [(577, 545), (200, 150)]]
