@@ -102,11 +102,11 @@ TRAFFIC_SOURCE = {"fp64": "ncu DRAM bytes of the advection launch set on a 360x2
 
 # FP64 instructions (per thread of a warp that issues one) per tracer-cell of the exact
 # MDFL passes (z 10.8, x 10.5, y with the explicit update 18.6) and per column of one
-# exact barotropic subcycle (momentum 20.4, corrector with the next predictor 17.9),
-# counted by ncu on the 360x270x50 block and on 360x300 columns; the FP64 instruction
+# exact barotropic subcycle (momentum 21.6, corrector with the next predictor 18.2),
+# counted by ncu on the 360x270x50 block and the 1440x360x50 band; the FP64 instruction
 # rate of GB300 measured with a probe kernel.
 FP64_OPS_PER_TRACER_CELL = 40.0
-FP64_OPS_PER_COLUMN_SUBCYCLE = 38.3
+FP64_OPS_PER_COLUMN_SUBCYCLE = 39.8
 FP64_PEAK_OPS = 5.05e11
 
 
@@ -334,8 +334,8 @@ def _fp64_roofline(prec, sec, steps, cells, ntr, ni, nj, nts):
                      "ops_per_tracer_cell": FP64_OPS_PER_TRACER_CELL},
             "barotropic": {"achieved": round(b, -6), "frac": round(b / FP64_PEAK_OPS, 3),
                            "ops_per_column_subcycle": FP64_OPS_PER_COLUMN_SUBCYCLE},
-            "source": "FP64 instruction counts per tracer-cell and per column-subcycle from ncu on a "
-                      "360x270x50 block"}
+            "source": "FP64 warp instructions, 32 to each, per tracer-cell and per column-subcycle from ncu on a "
+                      "360x270x50 block and a 1440x360x50 band"}
 
 
 def max_over_ranks(ms: float, device) -> float:

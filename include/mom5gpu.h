@@ -332,8 +332,8 @@ int mom5gpu_tracer_advection_step(mom5gpu_domain* d, int taum1, int tau, int tau
 int mom5gpu_autotune(mom5gpu_domain* d, double dtime, char* report, size_t report_len);
 /* The launch shape autotune chose, or one to pin: precision-form tile height
  * (16 or 24 rows incl. halo; 32 or 64: 16 rows up to 4 tracers, else 20);
- * prefetch 0, 1, 2 or 3, kept and reported (with 1 and 3 the height is 16,
- * with 2 it is 16 or 24), the tiles are staged alike with all; FP64 y-pass rows
+ * prefetch 0, 1, 2 or 3, kept and reported (1 and 3 take rows 16, 2 takes 16 or 24)
+ * though it selects nothing: the tiles are staged alike with all; FP64 y-pass rows
  * per thread (0 = built-in choice, 2, 4, 8, 16).  Every shape gives the same
  * results bit for bit. */
 int mom5gpu_set_tuning(mom5gpu_domain* d, int rows, int prefetch, int tj);
@@ -348,9 +348,8 @@ int mom5gpu_set_tuning(mom5gpu_domain* d, int rows, int prefetch, int tj);
  * a stream capture form 0 is used).  Forms 1 and 2 were slower
  * than 0 on every measured domain.  Every form gives the same results bit for
  * bit.  A domain in the precision form (MOM5GPU_PRECISION_MIXED) has forms 0
- * and 1 of its own subcycle (mode 2 runs form 0): form 1 was faster on a
- * 360x300 domain, where the launches set the time, and slower on 1440x1080;
- * both give the same bits. */
+ * and 1 of its own subcycle (mode 2 runs form 0): form 1 was slower on every
+ * measured domain too; both give the same bits. */
 int mom5gpu_set_barotropic_fusion(mom5gpu_domain* d, int mode);
 /* Self-test of the grid barrier of the cooperative subcycle launch: `rounds`
  * (1..100000) barriers over a full resident grid, after each of which every

@@ -348,7 +348,7 @@ class Domain:
         self.check(lib().mom5gpu_set_tuning(self.h, rows, int(prefetch), tj))
 
     def set_barotropic_fusion(self, mode: int):
-        """Exact B-grid subcycles: 0 (default) three launches each, 1 one
+        """Exact B-grid subcycles: 0 (default) two launches each, 1 one
         launch each, 2 all in one cooperative launch."""
         self.check(lib().mom5gpu_set_barotropic_fusion(self.h, int(mode)))
 

@@ -890,8 +890,7 @@ DEVI void bt_corr_pred_body(BtArgs a, int so, int sn, double wgt, int bx) {
 // bt_corr_body, in the same order, so the results are the same bits.  The
 // divergence the predictor reuses comes from plane `so` of a.dvs and the
 // corrector writes plane `sn` (two planes: a neighbouring tile may still be
-// reading the previous one).  For domains where three launches per subcycle
-// cost more than the ring recompute.
+// reading the previous one).
 template <int TX, int TY>
 DEVI void bt_fused_body(BtArgs a, int so, int sn, int reuse, double wgt, int bx, int by) {
   constexpr int PX = TX + 2, PY = TY + 2;  // pressure: points x0-1 .. x0+TX, y0-1 .. y0+TY

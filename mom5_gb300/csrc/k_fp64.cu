@@ -1332,7 +1332,7 @@ __global__ void k_bt_corr_pred(BtArgs a, int so, int sn, double wgt) {
 }
 // 32 x 8 tiles of 352 threads: one point per thread in each phase (the 34 x 10
 // pressure ring is the largest); 64 x 8 tiles of 256 threads, several points
-// per thread, took 1.80 ms per step on 360x300 against 1.41 ms
+// per thread, took a quarter longer on 360x300
 constexpr int kFusedTX = 32, kFusedTY = 8, kFusedThreads = 352;
 __global__ void __launch_bounds__(kFusedThreads) k_bt_fused(BtArgs a, int so, int sn, int reuse, double wgt) {
   pdl_wait();
@@ -1343,8 +1343,8 @@ __global__ void __launch_bounds__(kFusedThreads) k_bt_fused(BtArgs a, int so, in
 //
 // A persistent grid of 128-thread blocks, all resident (cooperative launch),
 // walks the blocks of the predictor, momentum and corrector launches (virtual
-// block vb) with the same bodies, and a grid barrier stands where a launch boundary stood, so the
-// results are those of the three launches bit for bit.  A barrier is an
+// block vb) with the same bodies, and a grid barrier stands where a launch boundary
+// would, so the results are those of the launches bit for bit.  A barrier is an
 // arrival counter: thread 0 of each block publishes the block's writes (fence),
 // adds one and waits until the counter reaches the barrier's target.  The wait
 // is bounded (kGridWaitCycles of the SM clock, about a second) and watches the
