@@ -35,7 +35,7 @@ struct mom5gpu_batch {
   long g_launches[2] = {0, 0};  // kernels per replay of each graph
   int* d_counter = nullptr;  // items of the precision form taken so far
   // tuning
-  int rows = 32, tj = 0, blocks_per_sm = 2, sms = 152;
+  int rows = 32, tj = 0, blocks_per_sm = 2, sms = kSms;
   BtResident resident;  // of the precision form's barotropic subcycles
   bool any_cyclic = false;
   cudaEvent_t e0 = nullptr, e1 = nullptr;

@@ -257,6 +257,7 @@ int launch_mdfl(mom5gpu_domain* d, bool all, int n_first, int ntr, int taum1, in
                 double sweby_limiter);
 // the whole step of every tracer: th_tendency = its advection, T(taup1) by the explicit update
 int launch_mdfl_step(mom5gpu_domain* d, bool all, int taum1, int tau, int taup1, double dtime);
+constexpr int kSms = 152;  // SMs of the GB300, by which the launch rules share work
 int y_strip_rows(long cols, long nj);
 int add_step_args(mom5gpu_domain* d, int n_first, int taum1, int taup1, MdflArgs* a);
 int launch_upwind_horz(mom5gpu_domain* d, int n, int taum1);

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(128) k_mdfl_z_seg(MdflArgs a, int L) {
 // nk / L for one extra face per segment.  Aim at about four blocks per SM.
 static int z_segment_levels(const Geo& g) {
   const long blocks = (long)((g.ni + 127) / 128) * g.nj;
-  const long want = 4L * 152;
+  const long want = 4L * kSms;
   if (blocks >= want || g.nk < 4) return g.nk;
   int nseg = (int)((want + blocks - 1) / blocks);
   if (nseg > g.nk / 2) nseg = g.nk / 2;  // segments of at least two levels
@@ -136,7 +136,7 @@ static int z_segment_levels(const Geo& g) {
 // rows, 110 with 2, 117 with 8; 37x29x12: 25, 31 and 44 with 2, 4 and 8, 28 with 1).
 int y_strip_rows(long cols, long nj) {
   int TJ = 16;
-  while (TJ > 2 && cols * ((nj + TJ - 1) / TJ) < 152L * 32 * 12) TJ /= 2;
+  while (TJ > 2 && cols * ((nj + TJ - 1) / TJ) < 32L * 12 * kSms) TJ /= 2;
   return TJ;
 }
 
@@ -167,7 +167,7 @@ static void run_mdfl(const MdflArgs& a, int pass, cudaStream_t s) {
   // programmatic dependents hide a launch each, which domains of a few blocks per SM feel
   // (37x29x12, 2 tracers: with SPLIT 24.7 us a step against 31.8); on larger ones the waiting
   // blocks cost more than that (120x80x30, 2 tracers: 103 and 114; 360x270x50, 10 tracers: 4%)
-  const bool dep = (long)nx * g.nj * g.nk < 152L * 8;
+  const bool dep = (long)nx * g.nj * g.nk < 8L * kSms;
   auto launch = [&](auto k, dim3 grid, int threads, auto... args) {
     if (dep) launch_pdl(k, grid, dim3(threads), s, args...);
     else k<<<grid, threads, 0, s>>>(args...);
@@ -194,7 +194,7 @@ template <bool ALL, bool SWEBY>
 static void run_mdfl_n(const MdflArgs& a, int pass, cudaStream_t s) {
   const Geo& g = a.g;
   if (a.ntr <= 1) run_mdfl<ALL, SWEBY, 1, false>(a, pass, s);
-  else if ((long)((g.ni + 31) / 32) * g.nj * g.nk < 16L * 152) run_mdfl<ALL, SWEBY, 1, true>(a, pass, s);
+  else if ((long)((g.ni + 31) / 32) * g.nj * g.nk < 16L * kSms) run_mdfl<ALL, SWEBY, 1, true>(a, pass, s);
   else if (a.ntr <= 2) run_mdfl<ALL, SWEBY, 2, false>(a, pass, s);
   else if (a.ntr <= 4) run_mdfl<ALL, SWEBY, 4, false>(a, pass, s);
   else run_mdfl<ALL, SWEBY, kMdflChunk, false>(a, pass, s);

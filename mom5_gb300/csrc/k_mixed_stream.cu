@@ -134,7 +134,7 @@ int stream_levels(long tiles, int nk, int ntr, int rows) {
   double cost = 0.0;
   for (int want = 1; want == 1 || want <= nk / 2; ++want) {
     const int L = (nk + want - 1) / want, n = (nk + L - 1) / L;
-    const long b = (tiles * n + 151) / 152;
+    const long b = (tiles * n + kSms - 1) / kSms;
     const double c = (two ? 1.55 * (b / 2) + b % 2 : (double)b) * (L + (n > 1 ? 2.0 : 1.0));
     if (want == 1 || c < cost) {
       cost = c;
