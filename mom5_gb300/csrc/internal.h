@@ -358,10 +358,11 @@ long bt_resident_columns(const void* a, const void* b, int threads);
 // at 91134, 1024 and 843 at 111360, 1036 and 1386 at 119110, 1382 and 1465 at 226524.
 // Precision form, blocks of 128 (40 + 40 and 32 + 32: 6 and 8 pairs): 455 and 495 at
 // 111360, 675 and 533 at 119110, 686 and 595 at 151140, 696 and 933 at 166600, 874 and
-// 972 at 286812.  The C grid's kernels lose at most 2% by early loads (785 and 773 at 95914
-// columns, 767 and 771 at 91134, 882 and 911 at 127167, 904 and 1514 at 137200) and
+// 972 at 286812.  The C grid's kernels lose at most 3% by early loads (785 and 769 at 95914
+// columns, 834 and 808 at 111360, 882 and 911 at 127167, 904 and 1514 at 137200) and
 // always load early, and so do the exact form's batches, whose two forms fit up to the
-// same 4 pairs of blocks of 128 (600 and 668 at 67584 columns, 952 and 1102 at 88192, 2038 and 2213 at 323968).
+// same 4 pairs of blocks of 128 (600 and 668 at 67584 columns, 952 and 1102 at 88192,
+// 2038 and 2213 at 323968).
 struct BtResident {
   long early = 0, late = 0;
   bool loads_early(long columns) const { return columns <= early || columns > late; }
